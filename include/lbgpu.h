@@ -158,14 +158,11 @@ double lbgpu_build_cylinder(int lx, int ly, int obst_x, int obst_y, int obst_r, 
                             double re, int wall_kind, int outlet_kind, uint8_t *tag,
                             double *bc, uint8_t *zgb_row, double *f);
 
-/* Steps per sweep of the pull scheme: 1 (default) or 2.  With 2, lbgpu_step advances pairs of
- * steps in one kernel that keeps the intermediate state on chip (in registers, shifted across
- * lanes by warp shuffles, for FP64/FP32; in shared memory for 16-bit storage), the GPU form of
- * the reference's collide_tight two-steps-per-sweep idea (lb.c:442-572): one read and one write
- * of the lattice per two steps.  Results are identical to single steps; on B200 it runs at 0.85
- * of one step per sweep, which already streams at the copy bandwidth.
- * Lattices with an extrapolated outlet (a pass between every two steps) and the first step of
- * a fresh lattice still run single steps.  LB_ERR_STATE for the AA scheme. */
+/* Steps per sweep of the pull scheme: 1 (default) or 2.  Both run alike: lbgpu_step advances a run
+ * of pull steps several at a time on tiles in shared memory wherever that is the faster way (two
+ * to eight steps by lattice size and storage type; the GPU form of the reference's collide_tight
+ * two-steps-per-sweep idea, lb.c:442-572), with results identical to single steps.  LB_ERR_STATE for
+ * two steps with the AA scheme. */
 int lbgpu_set_sweep_steps(lbgpu_lattice *lat, int steps);
 
 /* Advance `nsteps` time steps; asynchronous on the lattice's stream. */

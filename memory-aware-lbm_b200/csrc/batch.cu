@@ -86,6 +86,8 @@ BatchInst describe(const Lattice &L)
     b.buf[0] = L.d.buf[0];
     b.buf[1] = L.d.buf[1];
     b.side = L.d.side;
+    b.side_slot[0] = L.d.side_slot[0];
+    b.side_slot[1] = L.d.side_slot[1];
     b.tag = L.d.tag;
     b.bc = L.d.bc;
     b.omega = L.d.omega;

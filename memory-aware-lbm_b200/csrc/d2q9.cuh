@@ -120,6 +120,52 @@ __device__ __forceinline__ void bgk(T f[9], T omega)
     relax_one<8>(f, omega, om1, rho, ux, uy, usqr);
 }
 
+// The relaxation of a pair of opposite directions I, J in FP64: cu and -cu share every product, and
+// every operation keeps the operands and the order of relax_one, so the results are its bits.
+template <int I, int J>
+__device__ __forceinline__ void relax_pair(double f[9], double omega, double om1, double rt, double cu, double u15)
+{
+    using O = Ar<double>;
+    const double c3 = O::M(3.0, cu), q = O::M(O::M(4.5, cu), cu);
+    const double ei = O::M(rt, O::S(O::A(O::A(1.0, c3), q), u15));
+    const double ej = O::M(rt, O::S(O::A(O::S(1.0, c3), q), u15));
+    f[I] = O::A(O::M(f[I], om1), O::M(omega, ei));
+    f[J] = O::A(O::M(f[J], om1), O::M(omega, ej));
+}
+
+static __device__ __noinline__ void bgk_nonfinite(double f[9], double omega)
+{
+    bgk<double>(f, omega);
+}
+
+// BGK in exact FP64 with fewer operations: 1 cu_x + 0 cu_y is cu_x for every finite velocity (a zero's
+// sign is lost in 1 + 3 cu and in cu cu), and the four pairs of opposite directions share their
+// products.  About 115 FP64 operations a node against 155.  An infinite or NaN velocity (0 times
+// it is NaN) takes the general form, out of line.
+__device__ __forceinline__ void bgk_exact(double f[9], double omega)
+{
+    using O = Ar<double>;
+    double rho, ux, uy;
+    macros(f, rho, ux, uy);
+    const double usqr = O::A(O::M(ux, ux), O::M(uy, uy));
+    if (!(usqr < __longlong_as_double(0x7ff0000000000000LL))) {
+        double h[9];
+#pragma unroll
+        for (int i = 0; i < 9; ++i) h[i] = f[i];
+        bgk_nonfinite(h, omega);
+#pragma unroll
+        for (int i = 0; i < 9; ++i) f[i] = h[i];
+        return;
+    }
+    const double om1 = O::S(1.0, omega), u15 = O::M(1.5, usqr);
+    const double rt1 = O::M(rho, wgt(1)), rt5 = O::M(rho, wgt(5));
+    f[0] = O::A(O::M(f[0], om1), O::M(omega, O::M(O::M(rho, wgt(0)), O::S(1.0, u15))));
+    relax_pair<1, 3>(f, omega, om1, rt1, ux, u15);
+    relax_pair<2, 4>(f, omega, om1, rt1, uy, u15);
+    relax_pair<5, 7>(f, omega, om1, rt5, O::A(ux, uy), u15);
+    relax_pair<6, 8>(f, omega, om1, rt5, O::S(uy, ux), u15);
+}
+
 // Throughput form of BGK in FP32: one reciprocal of rho, equilibrium factored as
 // w rho (1 - 1.5u^2) + w rho cu (3 + 4.5 cu), relaxation as f + omega (feq - f).
 template <>
@@ -281,6 +327,75 @@ __device__ __forceinline__ void regularize(T f[9], int side, T rho, T ux, T uy)
     reg_one<8>(f, fe, pxx, pyy, pxy);
 }
 
+// The same in exact FP64 with fewer operations (about 110 against 250), bit for bit: opposite
+// directions share their equilibrium's products (relax_pair) and their stress term, whose products
+// with 0 are left out.  Velocities or stresses that are not finite (0 times them is NaN) take the
+// general form.
+static __device__ __noinline__ void regularize_nonfinite(double f[9], int side, double rho, double ux, double uy)
+{
+    regularize<double>(f, side, rho, ux, uy);
+}
+
+template <int I, int J>
+__device__ __forceinline__ void feq_pair(double fe[9], double rt, double cu, double u15)
+{
+    using O = Ar<double>;
+    const double c3 = O::M(3.0, cu), q = O::M(O::M(4.5, cu), cu);
+    fe[I] = O::M(rt, O::S(O::A(O::A(1.0, c3), q), u15));
+    fe[J] = O::M(rt, O::S(O::A(O::S(1.0, c3), q), u15));
+}
+
+__device__ __forceinline__ void regularize_exact(double f[9], int side, double rho, double ux, double uy)
+{
+    using O = Ar<double>;
+    double fe[9], n[9];
+    const double usqr = O::A(O::M(ux, ux), O::M(uy, uy)), u15 = O::M(1.5, usqr);
+    const double rt1 = O::M(rho, wgt(1)), rt5 = O::M(rho, wgt(5));
+    fe[0] = O::M(O::M(rho, wgt(0)), O::S(1.0, u15));
+    feq_pair<1, 3>(fe, rt1, ux, u15);
+    feq_pair<2, 4>(fe, rt1, uy, u15);
+    feq_pair<5, 7>(fe, rt5, O::A(ux, uy), u15);
+    feq_pair<6, 8>(fe, rt5, O::S(uy, ux), u15);
+#pragma unroll
+    for (int i = 1; i < 9; ++i) n[i] = O::S(f[i], fe[i]);
+    // the known populations along the wall (w1, w3) and its corners (p, m)
+    const bool tb = side <= SIDE_LOWER;
+    const double w1 = tb ? n[1] : n[2], w3 = tb ? n[3] : n[4];
+    // corners in the order the sums take them: pxx of a horizontal wall and pyy of a vertical one
+    // add (p, m); the other adds its three terms as written there
+    const double p = side == SIDE_UPPER || side == SIDE_RIGHT ? n[5] : (side == SIDE_LOWER ? n[7] : n[6]);
+    const double m = side == SIDE_UPPER ? n[6] : (side == SIDE_LEFT ? n[7] : n[8]);
+    const double par = O::A(O::A(w1, w3), O::M(2.0, O::A(p, m)));
+    double nor;
+    if (side == SIDE_UPPER) nor = O::A(O::A(n[6], n[2]), n[5]);
+    else if (side == SIDE_LOWER) nor = O::A(O::A(n[4], n[7]), n[8]);
+    else if (side == SIDE_RIGHT) nor = O::A(O::A(n[1], n[5]), n[8]);
+    else nor = O::A(O::A(n[3], n[6]), n[7]);
+    nor = O::M(2.0, nor);
+    const double pxx = tb ? par : nor, pyy = tb ? nor : par;
+    const double pxy = O::M(2.0, side == SIDE_LEFT ? O::S(n[7], n[6]) : O::S(p, m));
+    if (!(O::M(O::A(O::A(pxx, pyy), O::A(pxy, usqr)), 0.0) == 0.0)) {
+        double h[9];
+#pragma unroll
+        for (int i = 0; i < 9; ++i) h[i] = f[i];
+        regularize_nonfinite(h, side, rho, ux, uy);
+#pragma unroll
+        for (int i = 0; i < 9; ++i) f[i] = h[i];
+        return;
+    }
+    constexpr double third = 1. / 3., two3 = 1.0 - third;
+    const double a = O::M(two3, pxx), b = O::M(-third, pxx), c = O::M(two3, pyy), d = O::M(-third, pyy);
+    const double e = O::M(2.0, pxy);
+    const double s0 = O::A(b, d), sx = O::A(a, d), sy = O::A(b, c), sd = O::A(a, c);
+    const double t0 = O::M(4.5 * wgt(0), s0), t1 = O::M(4.5 * wgt(1), sx), t2 = O::M(4.5 * wgt(1), sy);
+    const double t5 = O::M(4.5 * wgt(5), O::A(sd, e)), t6 = O::M(4.5 * wgt(5), O::S(sd, e));
+    f[0] = O::A(fe[0], t0);
+    f[1] = O::A(fe[1], t1); f[3] = O::A(fe[3], t1);
+    f[2] = O::A(fe[2], t2); f[4] = O::A(fe[4], t2);
+    f[5] = O::A(fe[5], t5); f[7] = O::A(fe[7], t5);
+    f[6] = O::A(fe[6], t6); f[8] = O::A(fe[8], t6);
+}
+
 // Any non-BGK rule; (p0, p1) are the node's table entry: (ux, uy) or (rho, uPar).
 // Boundary rules chain to bulk BGK like every function of boundaries.c:171-414.
 template <class T>
@@ -301,8 +416,10 @@ static __device__ __noinline__ void collide_boundary(int t, T f[9], T omega, T p
         uy = tb ? u : p1;
     }
     if (t < TAG_REG_FIRST) zouhe_complete(f, side, ux, uy, rho);
+    else if constexpr (sizeof(T) == 8) regularize_exact(f, side, rho, ux, uy);
     else regularize(f, side, rho, ux, uy);
-    bgk(f, omega);
+    if constexpr (sizeof(T) == 8) bgk_exact(f, omega);
+    else bgk(f, omega);
 }
 
 // The boundary rules run out of line on a private copy, so the bulk path's populations stay
@@ -311,7 +428,8 @@ template <class T>
 __device__ __forceinline__ void collide(int t, T f[9], T omega, T p0, T p1)
 {
     if (t == TAG_BGK) {
-        bgk(f, omega);
+        if constexpr (sizeof(T) == 8) bgk_exact(f, omega);
+        else bgk(f, omega);
     } else {
         T g[9];
 #pragma unroll

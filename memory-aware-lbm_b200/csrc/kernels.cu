@@ -17,318 +17,14 @@
 //
 // Memory system: the step kernels stream the lattice once per step from HBM; one thread a block
 // prefetches into L2 the rows a block a few rows further down will read
-// (cp.async.bulk.prefetch.L2, distances measured per kernel); the two-step sweep moves its next
-// row into shared memory with cp.async while it computes.
-#include <algorithm>
-#include "codec.cuh"
+// (cp.async.bulk.prefetch.L2, distances measured per kernel).  Runs of pull steps advance several
+// steps a launch in shared memory instead (tile.cu).
 #include "kernels.h"
-#include "lbgpu.h"
+#include "node.cuh"
 
 namespace lbgpu {
 
 namespace {
-
-constexpr int BX = 128;  // threads along x per block (coalesced axis)
-
-template <class S>
-__device__ __forceinline__ const S *plane(const S *b, const Geo &g, int i)
-{
-    return b + (size_t)i * (size_t)g.plane;
-}
-template <class S>
-__device__ __forceinline__ S *plane(S *b, const Geo &g, int i)
-{
-    return b + (size_t)i * (size_t)g.plane;
-}
-
-// Table entry (p0, p1) of a boundary node: (ux, uy) or (rho, uPar).
-__device__ __forceinline__ void node_params(const double *__restrict__ bc, int nb, int t, int X, int Y,
-                                            double &p0, double &p1)
-{
-    p0 = 0.0; p1 = 0.0;
-    if (t >= TAG_ZOUHE_FIRST && t < TAG_COUNT) {
-        const int tb = tag_table(t);
-        const int coord = (tag_side(t) <= SIDE_LOWER) ? X : Y;
-        p0 = bc[(tb * 2 + 0) * nb + coord];
-        p1 = bc[(tb * 2 + 1) * nb + coord];
-    }
-}
-
-__device__ __forceinline__ void node_params(const double *__restrict__ bc, const Geo &g, int t,
-                                            int X, int Y, double &p0, double &p1)
-{
-    node_params(bc, g.nb, t, X, Y, p0, p1);
-}
-
-template <class S>
-__device__ __forceinline__ void collide_node(const double *__restrict__ bc, const Geo &g, int t,
-                                             int X, int Y, typename Codec<S>::R f[9], double omega)
-{
-    using R = typename Codec<S>::R;
-    double p0, p1;
-    node_params(bc, g, t, X, Y, p0, p1);
-    rules::collide<R>(t, f, (R)omega, (R)p0, (R)p1);
-}
-
-template <class S>
-__device__ __forceinline__ typename Codec<S>::R dec_row(const Geo &g, S v, int i, float inv, int Y);
-
-// Post-stream value of slot i at node (X, Y), any node of the lattice including the ghost
-// ring, under each view (kernels.h).  Ghost slots that no interior node streams into keep the
-// content of the buffer the state lives in, as in the reference: for the pull scheme `other`
-// is the second buffer; for the AA scheme's swapped view (an odd step count, which the
-// reference leaves in its second buffer) `other` is that buffer's saved ghost ring
-// [9][nghost].
-template <class S>
-__device__ __forceinline__ typename Codec<S>::R logical(const Geo &g, int view, const S *__restrict__ cur,
-                                                        const S *__restrict__ other,
-                                                        const S *__restrict__ side, int X, int Y,
-                                                        int i, float inv)
-{
-    using C = Codec<S>;
-    const int sx = X - cx(i), sy = Y - cy(i);
-    switch (view) {
-    case VIEW_PULL_PENDING:
-        if (g.interior(sx, sy)) return dec_row<S>(g, plane(cur, g, i)[g.idx(sx, sy)], i, inv, Y);
-        if (g.interior(X, Y)) return dec_row<S>(g, side[(size_t)i * g.nper + g.pidx(X, Y)], i, inv, Y);
-        return dec_row<S>(g, plane(other, g, i)[g.idx(X, Y)], i, inv, Y);
-    case VIEW_AA_NATURAL:
-        if (g.interior(X, Y) && !g.interior(sx, sy))
-            return dec_row<S>(g, side[(size_t)i * g.nper + g.pidx(X, Y)], i, inv, Y);
-        return dec_row<S>(g, plane(cur, g, i)[g.idx(X, Y)], i, inv, Y);
-    case VIEW_AA_SWAPPED:
-        if (g.interior(sx, sy)) return dec_row<S>(g, plane(cur, g, opp(i))[g.idx(sx, sy)], i, inv, Y);
-        if (g.interior(X, Y)) return dec_row<S>(g, side[(size_t)i * g.nper + g.pidx(X, Y)], i, inv, Y);
-        return dec_row<S>(g, other[(size_t)i * g.nghost() + g.gidx(X, Y)], i, inv, Y);
-    default:
-        return dec_row<S>(g, plane(cur, g, i)[g.idx(X, Y)], i, inv, Y);
-    }
-}
-
-// ---- 16-bit storage, four nodes per thread ------------------------------------------------
-//
-// Stored value D_i = (f_i - w_i) 2^s.  With sum(w) = 1 and sum(c w) = 0 the BGK step works on
-// D directly: rho = 1 + 2^-s sum(D), j = 2^-s sum(c D), and
-//   D_i' = D_i + omega (E_i - D_i),  E_i = 2^s w_i (rho (1 + 3 cu + 4.5 cu^2 - 1.5 u^2) - 1),
-// so there is no per-population decode or encode arithmetic, only the conversions (two per
-// instruction when packing).  Boundary rules decode to f and use the generic path.
-
-template <class S> struct Half2Ops;
-template <> struct Half2Ops<__half> {
-    static __device__ __forceinline__ float lo(unsigned w) { return __half2float(__ushort_as_half((unsigned short)(w & 0xffffu))); }
-    static __device__ __forceinline__ float hi(unsigned w) { return __half2float(__ushort_as_half((unsigned short)(w >> 16))); }
-    static __device__ __forceinline__ unsigned pack(float a, float b)
-    {
-        const __half2 h = __floats2half2_rn(a, b);
-        return *reinterpret_cast<const unsigned *>(&h);
-    }
-};
-template <> struct Half2Ops<__nv_bfloat16> {
-    static __device__ __forceinline__ float lo(unsigned w) { return __uint_as_float(w << 16); }
-    static __device__ __forceinline__ float hi(unsigned w) { return __uint_as_float(w & 0xffff0000u); }
-    static __device__ __forceinline__ unsigned pack(float a, float b)
-    {
-        const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-        return *reinterpret_cast<const unsigned *>(&h);
-    }
-};
-
-// BGK on scaled offsets D[9] of one node (sc = 2^s, inv = 2^-s).  With d = rho - 1 =
-// inv sum(D) and j = rho u = inv sum(c D), rho c.u = c.j and rho u^2 = j.u give
-//   E_i = sc w_i (A + 3 c.j + 4.5 (c.u)(c.j)),  A = d - 1.5 j.u,
-// and the relaxation is D_i' = (1 - omega) D_i + omega E_i.  Opposite directions i, opp(i)
-// share c.u and c.j up to sign: omega E_i, omega E_opp = a +- b with
-// a = k (A + 4.5 (c.u)(c.j)), b = 3 k c.j, k = omega sc w.
-// With a row shift (SHIFT, offsets relative to S_i = f_eq_i(1, (us, 0)) instead of w_i):
-// j = (us, 0) + inv J, E_i = sc (f_eq_i(rho, u) - S_i), so A gains -1.5 us (ux - us) and a gains
-// 4.5 k (c.us)(c.u - c.us); b is unchanged.  Without it the arithmetic is exactly the unshifted one.
-// 1/rho uses the hardware reciprocal (the 16-bit path is held to a tolerance, not bit-exact).
-template <bool SHIFT>
-__device__ __forceinline__ void bgk_offsets(float D[9], float omega, float sc, float inv, float us)
-{
-    // J = 2^s (j - us): scaled sums; u = J inv / rho (+ us / rho), inv folded into constants
-    const float sum = ((D[0] + D[1]) + (D[2] + D[3])) + ((D[4] + D[5]) + (D[6] + D[7])) + D[8];
-    const float d = inv * sum;
-    const float Jx = (D[1] - D[3]) + (D[5] - D[6]) + (D[8] - D[7]);
-    const float Jy = (D[2] - D[4]) + (D[5] - D[8]) + (D[6] - D[7]);
-    const float ir = __fdividef(1.0f, 1.0f + d);
-    const float q = inv * ir;
-    const float ux = SHIFT ? fmaf(Jx, q, __fmul_rn(us, ir)) : Jx * q, uy = Jy * q;
-    float A = fmaf(-1.5f * inv, fmaf(Jx, ux, Jy * uy), d);
-    // shifted terms: t = ux - us; 4.5 (c.us)(c.u - c.us) is e1 = 4.5 us t for (1, 3) and
-    // e1 +- 4.5 us uy for (5, 7) and (6, 8), folded into the pair's constant term: A1 = A + e1,
-    // A1 +- 4.5 us uy
-    const float t = SHIFT ? __fsub_rn(ux, us) : 0.0f;
-    if (SHIFT) A = fmaf(-1.5f * us, t, A);
-    const float ux45 = (4.5f * inv) * ux, uy45 = (4.5f * inv) * uy;
-    const float hs = 4.5f * us;
-    const float A1 = SHIFT ? fmaf(hs, t, A) : A, ev = SHIFT ? __fmul_rn(hs, uy) : 0.0f;
-    const float A5 = SHIFT ? __fadd_rn(A1, ev) : A, A6 = SHIFT ? __fsub_rn(A1, ev) : A;
-    const float om1 = 1.0f - omega;
-    const float k0 = omega * sc * (4.f / 9.f), k1 = omega * sc * (1.f / 9.f), k2 = omega * sc * (1.f / 36.f);
-    D[0] = fmaf(om1, D[0], k0 * A);
-    // The shifted terms use explicitly rounded operations: no multiply-add contraction may
-    // differ between the kernels that inline this, so every scheme stays bit-identical.
-#define LBGPU_PAIR(I, J, K, CU45, CJ, AP)                              \
-    {                                                                  \
-        const float cj = (CJ);                                         \
-        if (SHIFT) {                                                   \
-            const float a = __fmul_rn(K, fmaf(CU45, cj, (AP)));        \
-            const float b = __fmul_rn((3.0f * inv) * K, cj);          \
-            D[I] = fmaf(om1, D[I], __fadd_rn(a, b));                   \
-            D[J] = fmaf(om1, D[J], __fsub_rn(a, b));                   \
-        } else {                                                       \
-            const float a = K * fmaf(CU45, cj, A);                     \
-            const float b = ((3.0f * inv) * K) * cj;                   \
-            D[I] = fmaf(om1, D[I], a + b);                             \
-            D[J] = fmaf(om1, D[J], a - b);                             \
-        }                                                              \
-    }
-    LBGPU_PAIR(1, 3, k1, ux45, Jx, A1)
-    LBGPU_PAIR(2, 4, k1, uy45, Jy, A)
-    LBGPU_PAIR(5, 7, k2, __fadd_rn(ux45, uy45), __fadd_rn(Jx, Jy), A5)
-    LBGPU_PAIR(6, 8, k2, __fsub_rn(uy45, ux45), __fsub_rn(Jy, Jx), A6)
-#undef LBGPU_PAIR
-}
-
-
-// Working values of a kernel: decoded populations f for FP64/FP32, the stored offsets D as
-// float for 16-bit storage (see bgk_offsets); collide_w applies a node's rule to them.  Every
-// kernel of one storage type uses these, so all schemes agree bit for bit.
-template <class S> struct Work {
-    using W = typename Codec<S>::R;
-    static __device__ __forceinline__ W load(S v, int i, float inv) { return Codec<S>::dec(v, i, inv); }
-    static __device__ __forceinline__ S store(W w, int i, float sc) { return Codec<S>::enc(w, i, sc); }
-};
-template <> struct Work<__half> {
-    using W = float;
-    static __device__ __forceinline__ float load(__half v, int, float) { return __half2float(v); }
-    static __device__ __forceinline__ __half store(float w, int, float) { return __float2half_rn(w); }
-};
-template <> struct Work<__nv_bfloat16> {
-    using W = float;
-    static __device__ __forceinline__ float load(__nv_bfloat16 v, int, float) { return __bfloat162float(v); }
-    static __device__ __forceinline__ __nv_bfloat16 store(float w, int, float) { return __float2bfloat16_rn(w); }
-};
-
-// Stochastic rounding (codec.cuh) is a compile-time choice of a kernel (RS), so no store
-// carries a branch: RS kernels run only for 16-bit lattices with it on, whose collision key is
-// then never 0.
-// The random word of node (X, Y) for a collision key.
-template <class S, bool RS>
-__device__ __forceinline__ RsNode rs_node(const Geo &g, unsigned key, int X, int Y)
-{
-    if constexpr (RS && sizeof(S) == 2) {
-        const int q = (X - 1) & 3;
-        return RsNode{rs_mix(((unsigned)Y * (unsigned)(g.lx + 2) + (unsigned)(X - q)) ^ key), q};
-    }
-    return RsNode{0u, 0};
-}
-
-// A post-collision working value of direction i as stored: rounded to nearest, or (RS)
-// stochastically with the node's random word h.
-template <class S, bool RS>
-__device__ __forceinline__ S put(typename Work<S>::W w, int i, float sc, RsNode h)
-{
-    if constexpr (RS && sizeof(S) == 2) {
-        const unsigned p = rs_pair(h.hq, h.q >> 1, i);
-        return RsOps<S>::one(w, (h.q & 1) ? (p >> 16) : p);
-    }
-    return Work<S>::store(w, i, sc);
-}
-
-// Decode / encode of a value consumed at row Y (read-outs, uploads, initial states).
-template <class S>
-__device__ __forceinline__ typename Codec<S>::R dec_row(const Geo &g, S v, int i, float inv, int Y)
-{
-    if constexpr (sizeof(S) == 2) {
-        if (g.shift_u) return fmaf(Work<S>::load(v, i, inv), inv, g.shift_base(Y)[i]);
-    }
-    return Codec<S>::dec(v, i, inv);
-}
-
-template <class S>
-__device__ __forceinline__ S enc_row(const Geo &g, typename Codec<S>::R f, int i, float sc, int Y)
-{
-    if constexpr (sizeof(S) == 2) {
-        if (g.shift_u) return Work<S>::store(__fmul_rn(__fsub_rn(f, g.shift_base(Y)[i]), sc), i, sc);
-    }
-    return Codec<S>::enc(f, i, sc);
-}
-
-// A post-collision value of direction i at row Y, as stored in a population plane: with a row
-// shift it is relative to the row that consumes it after streaming, Y + c_iy (stale-slot copies
-// in the side store are consumed by the node itself and stay relative to row Y).
-// SH: 0 no shift, 1 shift (known at compile time), 2 decided by g.shift_u at run time.
-// Rows whose rebase values are all zero (shift_rebased false) store unchanged in every kernel.
-template <class S, int SH = 2>
-__device__ __forceinline__ typename Work<S>::W stored_out(const Geo &g, int Y, int i, typename Work<S>::W w,
-                                                          float sc)
-{
-    if constexpr (sizeof(S) == 2 && SH != 0) {
-        if (cy(i) != 0 && (SH == 1 || g.shift_u) && g.shift_rebased(Y))
-            return __fadd_rn(w, __fmul_rn(g.shift_rebase(Y)[i], sc));
-    }
-    return w;
-}
-
-// A non-BGK rule on one node's 16-bit offsets: decode, the generic rule, encode.  Out of line so
-// the bulk path keeps its registers (it runs for boundary and obstacle nodes only); the shifted
-// form is a separate function, because a larger callee costs the 64-register quad kernel spills.
-template <class S>
-static __device__ __noinline__ void boundary_offsets(const double *__restrict__ bc, Geo g, int t, int X,
-                                                     int Y, float D[9], double omega, float sc, float inv)
-{
-    float f[9];
-#pragma unroll
-    for (int i = 0; i < 9; ++i) f[i] = fmaf(D[i], inv, wgtf(i));
-    collide_node<S>(bc, g, t, X, Y, f, omega);
-#pragma unroll
-    for (int i = 0; i < 9; ++i) D[i] = (f[i] - wgtf(i)) * sc;
-}
-
-// The same with offsets from the row's shift equilibrium (base: S_i of the row).
-template <class S>
-static __device__ __noinline__ void boundary_offsets_shifted(const double *__restrict__ bc, int nb,
-                                                             const float *__restrict__ base, int t, int X, int Y,
-                                                             float D[9], double omega, float sc, float inv)
-{
-    float f[9];
-#pragma unroll
-    for (int i = 0; i < 9; ++i) f[i] = fmaf(D[i], inv, base[i]);
-    double p0, p1;
-    node_params(bc, nb, t, X, Y, p0, p1);
-    rules::collide<float>(t, f, (float)omega, (float)p0, (float)p1);
-#pragma unroll
-    for (int i = 0; i < 9; ++i) D[i] = (f[i] - base[i]) * sc;
-}
-
-template <class S, int SH = 2>
-__device__ __forceinline__ void collide_w(const double *__restrict__ bc, const Geo &g, int t, int X,
-                                          int Y, typename Work<S>::W w[9], double omega, float sc,
-                                          float inv)
-{
-    if constexpr (sizeof(S) == 2) {
-        if (t == TAG_BGK) {
-            if constexpr (SH == 1) bgk_offsets<true>(w, (float)omega, sc, inv, g.shift_u[Y]);
-            else if constexpr (SH == 0) bgk_offsets<false>(w, (float)omega, sc, inv, 0.0f);
-            else if (g.shift_u) bgk_offsets<true>(w, (float)omega, sc, inv, g.shift_u[Y]);
-            else bgk_offsets<false>(w, (float)omega, sc, inv, 0.0f);
-        } else {
-            float tmp[9];
-#pragma unroll
-            for (int i = 0; i < 9; ++i) tmp[i] = w[i];
-            if (SH == 1 || (SH == 2 && g.shift_u))
-                boundary_offsets_shifted<S>(bc, g.nb, g.shift_base(Y), t, X, Y, tmp, omega, sc, inv);
-            else
-                boundary_offsets<S>(bc, g, t, X, Y, tmp, omega, sc, inv);
-#pragma unroll
-            for (int i = 0; i < 9; ++i) w[i] = tmp[i];
-        }
-    } else {
-        collide_node<S>(bc, g, t, X, Y, w, omega);
-    }
-}
 
 // L2 prefetch for the block a few rows further down the grid (blocks run roughly in row order,
 // so those rows are read soon after, from L2): one thread a block issues the nine row segments
@@ -717,341 +413,6 @@ __global__ void __launch_bounds__(BX) k_stream(Geo g, const S *__restrict__ src,
     }
 }
 
-// ---- two steps per sweep (temporal blocking) ----------------------------------------------
-//
-// The GPU form of the reference's two-steps-per-sweep ("tight") idea (lb.c:442-572).  Each node
-// runs pull_node's arithmetic on the same inputs and the intermediate state is kept in the
-// storage type, so the result is identical to two single pull steps.
-//
-// Stale slots: step n+1 reads side parity (n+1)&1 (C_{n-1}); its new values go to the scratch
-// slot `side_tmp`, not to that parity, because neighbouring blocks may still read it for their
-// halo.  Step n+2 reads and writes parity n&1 for its own nodes only.  launch_pull2_finish then
-// moves the scratch into parity (n+1)&1 and swaps the two buffers' ghost rings: the state ends
-// in the buffer two single steps would not have left it in, and the read-outs take ghost values
-// from the other buffer.
-//
-// The kernel is a sweep (the shape of the reference's tight variants): a block of W + 2 threads
-// owns a strip of W columns and a segment of H rows and walks down it, keeping four rows of C_n
-// (W + 4 wide) and three rows of C_{n+1} (W + 2 wide) in shared memory.  Iteration t has C_n row
-// YL = y0 - 2 + t (fetched asynchronously during the previous iteration), fetches row YL + 1,
-// computes C_{n+1} on row YL - 1 (W + 2 nodes: one a thread) and C_{n+2} on row YL - 2, which it
-// writes.  Halo work is two columns a side and two rows a segment end (a few percent), and the
-// shared memory a block needs is small enough for several blocks a SM.
-template <class S, int W>
-constexpr size_t sweep2_r0_bytes() { return (4 * 9 * (size_t)(W + 4) * sizeof(S) + 15) / 16 * 16; }
-template <class S, int W>
-constexpr size_t sweep2_smem_bytes() { return sweep2_r0_bytes<S, W>() + 3 * 9 * (size_t)(W + 2) * sizeof(S); }
-
-template <class S, int W, int H, bool RS>
-__global__ void __launch_bounds__(W + 2) k_sweep2(Geo g, const S *__restrict__ src, S *__restrict__ dst,
-                                             const uint8_t *__restrict__ tag, const double *__restrict__ bc,
-                                             double omega, const S *__restrict__ side_a,
-                                             S *__restrict__ side_tmp, S *__restrict__ side_b, float sc,
-                                             float inv)
-{
-    constexpr int W0 = W + 4, W1 = W + 2;
-    extern __shared__ __align__(16) unsigned char sweep_smem[];
-    auto r0 = reinterpret_cast<S (*)[9][W0]>(sweep_smem);                 // C_n rows [4], slot = row mod 4
-    auto r1 = reinterpret_cast<S (*)[9][W1]>(sweep_smem + sweep2_r0_bytes<S, W>());   // C_{n+1} rows [3]
-    const int x0 = 1 + blockIdx.x * W, y0 = 1 + blockIdx.y * H;
-    const int tx = threadIdx.x;
-    const int yend = min(y0 + H, g.ly + 1);           // rows y0 .. yend-1 are this block's
-    // C_n row YL into ring slot YL mod 4 by asynchronous copies (cp.async; one commit group a row,
-    // empty for rows outside the array).  A copy unit is one element of 4 or 8 bytes, or two
-    // 2-byte elements from an even k (element x0-2+k of the row sits at an even index then, so
-    // the pair is 4-byte aligned); units may cover the row's padding (X = -1 or lx + 2), which is
-    // inside the allocation and never read back.
-    constexpr int E = sizeof(S) >= 4 ? 1 : 2;
-    constexpr unsigned UB = E * sizeof(S);
-    auto fetch = [&](int YL) {
-        if (YL >= 0 && YL <= g.ly + 1) {
-            const int sl = (YL + 4) % 4;
-            for (int u = tx; u < W0 / E; u += W + 2) {
-                const int k = u * E, X = x0 - 2 + k;
-                if (X + E - 1 >= 0 && X <= g.lx + 1) {
-                    const long long o = g.idx(X, YL);
-#pragma unroll
-                    for (int i = 0; i < 9; ++i) {
-                        const unsigned d = (unsigned)__cvta_generic_to_shared(&r0[sl][i][k]);
-                        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(plane(src, g, i) + o),
-                                     "n"(UB) : "memory");
-                    }
-                }
-            }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    fetch(y0 - 2);
-    for (int t = 0; y0 - 2 + t - 2 < yend; ++t) {
-        const int YL = y0 - 2 + t;
-        // row YL + 1 flies while rows YL - 1 and YL - 2 are computed; its slot held row YL - 3,
-        // last read before the previous iteration's second barrier
-        fetch(YL + 1);
-        asm volatile("cp.async.wait_group 1;" ::: "memory");   // this thread's copies of row YL landed
-        __syncthreads();                                      // everyone's
-        // step n+1 on row YL - 1, columns x0-1 .. x0+W
-        const int Y1 = YL - 1;
-        if (Y1 >= y0 - 1 && Y1 >= 1 && Y1 <= g.ly && Y1 <= yend) {
-            for (int k = tx; k < W1; k += W + 2) {
-                const int X = x0 - 1 + k;
-                if (X < 1 || X > g.lx) continue;
-                const bool edge = g.perimeter(X, Y1);
-                const int p = edge ? g.pidx(X, Y1) : 0;
-                typename Work<S>::W f[9];
-#pragma unroll
-                for (int i = 0; i < 9; ++i) {
-                    const int sx = X - cx(i), sy = Y1 - cy(i);
-                    f[i] = Work<S>::load(g.interior(sx, sy) ? r0[(sy + 4) % 4][i][sx - x0 + 2]
-                                                            : side_a[(size_t)i * g.nper + p], i, inv);
-                }
-                collide_w<S>(bc, g, tag[g.idx(X, Y1)], X, Y1, f, omega, sc, inv);
-                const int sl = (Y1 + 3) % 3;
-                const RsNode h = rs_node<S, RS>(g, g.rs_key, X, Y1);
-#pragma unroll
-                for (int i = 0; i < 9; ++i) r1[sl][i][k] = put<S, RS>(stored_out<S>(g, Y1, i, f[i], sc), i, sc, h);
-                if (edge && X >= x0 && X < x0 + W && Y1 >= y0 && Y1 < yend) {
-#pragma unroll
-                    for (int i = 0; i < 9; ++i)
-                        if (!g.interior(X - cx(i), Y1 - cy(i)))
-                            side_tmp[(size_t)i * g.nper + p] = put<S, RS>(f[i], i, sc, h);
-                }
-            }
-        }
-        __syncthreads();
-        // step n+2 on row YL - 2, columns x0 .. x0+W-1, to the other buffer
-        const int Y2 = YL - 2;
-        const int X = x0 + tx;
-        if (tx < W && Y2 >= y0 && Y2 < yend && X <= g.lx) {
-            const bool edge = g.perimeter(X, Y2);
-            const int p = edge ? g.pidx(X, Y2) : 0;
-            typename Work<S>::W f[9];
-#pragma unroll
-            for (int i = 0; i < 9; ++i) {
-                const int sx = X - cx(i), sy = Y2 - cy(i);
-                f[i] = Work<S>::load(g.interior(sx, sy) ? r1[(sy + 3) % 3][i][sx - x0 + 1]
-                                                        : side_b[(size_t)i * g.nper + p], i, inv);
-            }
-            const long long o = g.idx(X, Y2);
-            collide_w<S>(bc, g, tag[o], X, Y2, f, omega, sc, inv);
-            const RsNode h = rs_node<S, RS>(g, g.rs_key2, X, Y2);
-#pragma unroll
-            for (int i = 0; i < 9; ++i) plane(dst, g, i)[o] = put<S, RS>(stored_out<S>(g, Y2, i, f[i], sc), i, sc, h);
-            if (edge) {
-#pragma unroll
-                for (int i = 0; i < 9; ++i)
-                    if (!g.interior(X - cx(i), Y2 - cy(i))) side_b[(size_t)i * g.nper + p] = put<S, RS>(f[i], i, sc, h);
-            }
-        }
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");   // the last prefetch lands before the block ends
-}
-
-// ---- two steps per sweep, register form ---------------------------------------------------
-//
-// The same two steps as k_sweep2 (same node arithmetic, same stale-slot and scratch handling,
-// finished by k_pull2_finish), with both steps kept in registers: each warp owns a strip of
-// SW2_OUT = 28 columns and a segment of H rows and walks down it.  Lane l holds column
-// X = x0 - 2 + l (x0 - 2 .. x0 + 29); one iteration loads row R of C_n (nine populations of the
-// lane's column), shifts directions with c_ix = +-1 one lane across by shuffles, computes step
-// n+1 on row R - 1 (lanes 1..30 are valid) and step n+2 on row R - 2 (lanes 2..29, written).  A
-// population's row shift c_iy is the walk itself: directions with c_iy = +1 come from the row
-// two iterations back, c_iy = 0 from the previous one, c_iy = -1 from the current one, so each
-// step holds nine values of the rows behind it.  No shared memory and no block barrier: warps
-// are independent, the halo (two columns a side, shared with the neighbouring strips, and two
-// rows a segment end) is re-read from L2.
-constexpr int SW2_OUT = 28;   // output columns a warp
-
-// Direction groups of the walk (D2Q9 order of lb.c:48-55): c_iy = +1 {2, 5, 6}, 0 {0, 1, 3},
-// -1 {4, 7, 8}.
-template <class W>
-__device__ __forceinline__ W lane_shift(W v, int i)
-{
-    if (cx(i) == 1) return __shfl_up_sync(0xffffffffu, v, 1);     // from lane - 1
-    if (cx(i) == -1) return __shfl_down_sync(0xffffffffu, v, 1);  // from lane + 1
-    return v;
-}
-
-// One pull step of the walk on row Y at column X of this lane: the gathered populations from the
-// held rows (up: c_iy = +1, mid: c_iy = 0) and the current one (cur, already lane-shifted),
-// stale slots from `side` on the perimeter; collides into f.
-template <class S>
-__device__ __forceinline__ void walk_gather(const Geo &g, const typename Work<S>::W up[3],
-                                            const typename Work<S>::W mid[3],
-                                            const typename Work<S>::W cur[9], const S *__restrict__ side,
-                                            float inv, int X, int Y, bool edge, int p,
-                                            typename Work<S>::W f[9])
-{
-    f[2] = up[0]; f[5] = up[1]; f[6] = up[2];
-    f[0] = mid[0]; f[1] = mid[1]; f[3] = mid[2];
-    f[4] = cur[4]; f[7] = cur[7]; f[8] = cur[8];
-    if (edge) {
-#pragma unroll
-        for (int i = 0; i < 9; ++i)
-            if (!g.interior(X - cx(i), Y - cy(i))) f[i] = Work<S>::load(side[(size_t)i * g.nper + p], i, inv);
-    }
-}
-
-template <class S>
-__device__ __forceinline__ void walk_hold(typename Work<S>::W up_next[3], typename Work<S>::W up[3],
-                                          typename Work<S>::W mid[3], const typename Work<S>::W cur[9])
-{
-    up[0] = up_next[0]; up[1] = up_next[1]; up[2] = up_next[2];
-    up_next[0] = cur[2]; up_next[1] = cur[5]; up_next[2] = cur[6];
-    mid[0] = cur[0]; mid[1] = cur[1]; mid[2] = cur[3];
-}
-
-// Rows ahead of the walk prefetched into L2 (0: none), measured on the 16384 x 4096 channel
-// (GLUPS of two steps per sweep at 0 / 4 / 8 rows): FP64 29.7 / 38.8 / 33.3, FP32 77.3 / 62.1 / 62.0.
-#ifndef LBGPU_SWEEP2W_PF64
-#define LBGPU_SWEEP2W_PF64 4
-#endif
-#ifndef LBGPU_SWEEP2W_PF32
-#define LBGPU_SWEEP2W_PF32 0
-#endif
-template <class S>
-constexpr int sweep2w_pf() { return sizeof(S) == 8 ? LBGPU_SWEEP2W_PF64 : (sizeof(S) == 4 ? LBGPU_SWEEP2W_PF32 : 0); }
-#ifndef LBGPU_SWEEP2W_MINB64
-#define LBGPU_SWEEP2W_MINB64 4    // blocks of 4 warps a SM for FP64 (at most 128 registers)
-#endif
-#ifndef LBGPU_SWEEP2W_MINB32
-#define LBGPU_SWEEP2W_MINB32 6    // FP32 (at most 80 registers)
-#endif
-template <class S>
-constexpr int sweep2w_min_blocks()
-{
-    return sizeof(S) == 8 ? LBGPU_SWEEP2W_MINB64 : (sizeof(S) == 4 ? LBGPU_SWEEP2W_MINB32 : 5);
-}
-
-template <class S, int H, bool RS>
-__global__ void __launch_bounds__(128, sweep2w_min_blocks<S>()) k_sweep2w(Geo g, const S *__restrict__ src, S *__restrict__ dst,
-                                                 const uint8_t *__restrict__ tag, const double *__restrict__ bc,
-                                                 double omega, const S *__restrict__ side_a,
-                                                 S *__restrict__ side_tmp, S *__restrict__ side_b, float sc,
-                                                 float inv)
-{
-    using W = typename Work<S>::W;
-    const int lane = threadIdx.x & 31;
-    const int x0 = 1 + ((int)blockIdx.x * 4 + (int)(threadIdx.x >> 5)) * SW2_OUT;
-    if (x0 > g.lx) return;                                 // the whole warp
-    const int X = x0 - 2 + lane;
-    const int y0 = 1 + (int)blockIdx.y * H;
-    const int yend = min(y0 + H, g.ly + 1);                // rows y0 .. yend-1 are this warp's
-    const bool col_in = X >= 0 && X <= g.lx + 1;           // a column of the arrays
-    const bool x_int = X >= 1 && X <= g.lx;
-    const bool own_a = lane >= 2 && lane < 2 + SW2_OUT && x_int;   // owned columns (either step)
-    W a_up[3] = {}, a_upn[3] = {}, a_mid[3] = {};          // C_n rows behind the walk
-    W b_up[3] = {}, b_upn[3] = {}, b_mid[3] = {};          // C_{n+1} rows behind the walk
-    // Row R + 1 is loaded while row R is computed (its values are first used one iteration
-    // later), and with sweep2w_pf > 0 lane 0 prefetches into L2 the strip's row that many rows
-    // ahead: 32 elements from column x0 - 2, widened to 16-byte boundaries and by 16 bytes,
-    // skipped where the segment would pass the row's pitch (every byte inside its plane).
-    S raw[9];
-    auto fetch = [&](int R) {
-        if (col_in && R >= 0 && R <= g.ly + 1) {
-            const long long o = g.idx(X, R);
-#pragma unroll
-            for (int i = 0; i < 9; ++i) raw[i] = plane(src, g, i)[o];
-        } else {
-#pragma unroll
-            for (int i = 0; i < 9; ++i) raw[i] = S(0);
-        }
-    };
-    fetch(y0 - 2);
-    for (int R = y0 - 2; R <= yend + 1; ++R) {
-        // C_n row R, lane-shifted
-        W cur[9];
-#pragma unroll
-        for (int i = 0; i < 9; ++i) cur[i] = Work<S>::load(raw[i], i, inv);
-        fetch(R + 1);
-        if (sweep2w_pf<S>() > 0 && lane == 0) {
-            const int Rp = R + 1 + sweep2w_pf<S>();
-            constexpr int EB = (int)sizeof(S);
-            const long long e0 = g.idx(x0 - 2, Rp);                       // element of column x0 - 2
-            const long long b0 = (e0 * EB) & ~15LL, b1 = ((e0 + 32) * EB + 31) & ~15LL;
-            if (Rp <= g.ly + 1 && b1 <= ((long long)Rp + 1) * g.pitch * EB)
-#pragma unroll
-                for (int i = 0; i < 9; ++i)
-                    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(
-                                     reinterpret_cast<const char *>(plane(src, g, i)) + b0),
-                                 "r"((unsigned)(b1 - b0)) : "memory");
-        }
-#pragma unroll
-        for (int i = 0; i < 9; ++i) cur[i] = lane_shift(cur[i], i);
-        // step n+1 on row Y1 = R - 1: its C_{n+1} values in the storage type, lane-shifted
-        const int Y1 = R - 1;
-        W nxt[9];
-#pragma unroll
-        for (int i = 0; i < 9; ++i) nxt[i] = W(0);
-        if (R >= y0 && x_int && Y1 >= 1 && Y1 <= g.ly) {
-            const bool edge = g.perimeter(X, Y1);
-            const int p = edge ? g.pidx(X, Y1) : 0;
-            W f[9];
-            walk_gather<S>(g, a_up, a_mid, cur, side_a, inv, X, Y1, edge, p, f);
-            collide_w<S>(bc, g, tag[g.idx(X, Y1)], X, Y1, f, omega, sc, inv);
-            const RsNode h = rs_node<S, RS>(g, g.rs_key, X, Y1);
-#pragma unroll
-            for (int i = 0; i < 9; ++i)
-                nxt[i] = Work<S>::load(put<S, RS>(stored_out<S>(g, Y1, i, f[i], sc), i, sc, h), i, inv);
-            if (edge && own_a && lane < 2 + SW2_OUT && Y1 >= y0 && Y1 < yend) {
-#pragma unroll
-                for (int i = 0; i < 9; ++i)
-                    if (!g.interior(X - cx(i), Y1 - cy(i)))
-                        side_tmp[(size_t)i * g.nper + p] = put<S, RS>(f[i], i, sc, h);
-            }
-        }
-        walk_hold<S>(a_upn, a_up, a_mid, cur);
-#pragma unroll
-        for (int i = 0; i < 9; ++i) nxt[i] = lane_shift(nxt[i], i);
-        // step n+2 on row Y2 = R - 2, written for the owned columns
-        const int Y2 = R - 2;
-        if (R >= y0 + 2 && own_a && Y2 < yend) {
-            const bool edge = g.perimeter(X, Y2);
-            const int p = edge ? g.pidx(X, Y2) : 0;
-            W f[9];
-            walk_gather<S>(g, b_up, b_mid, nxt, side_b, inv, X, Y2, edge, p, f);
-            const long long o = g.idx(X, Y2);
-            collide_w<S>(bc, g, tag[o], X, Y2, f, omega, sc, inv);
-            const RsNode h = rs_node<S, RS>(g, g.rs_key2, X, Y2);
-#pragma unroll
-            for (int i = 0; i < 9; ++i) plane(dst, g, i)[o] = put<S, RS>(stored_out<S>(g, Y2, i, f[i], sc), i, sc, h);
-            if (edge) {
-#pragma unroll
-                for (int i = 0; i < 9; ++i)
-                    if (!g.interior(X - cx(i), Y2 - cy(i))) side_b[(size_t)i * g.nper + p] = put<S, RS>(f[i], i, sc, h);
-            }
-        }
-        walk_hold<S>(b_upn, b_up, b_mid, nxt);
-    }
-}
-
-// After k_sweep2: the scratch stale slots into parity (n+1)&1, and the ghost rings of the two
-// buffers exchanged (one thread per perimeter node and per ghost-ring node).
-template <class S>
-__global__ void k_pull2_finish(Geo g, S *__restrict__ b0, S *__restrict__ b1, const S *__restrict__ side_tmp,
-                               S *__restrict__ side_a)
-{
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < g.nper) {
-#pragma unroll
-        for (int i = 0; i < 9; ++i) side_a[(size_t)i * g.nper + k] = side_tmp[(size_t)i * g.nper + k];
-    }
-    const int ng = g.nghost();
-    if (k < ng) {
-        int X, Y;
-        if (k < g.lx + 2) { X = k; Y = 0; }
-        else if (k < 2 * (g.lx + 2)) { X = k - (g.lx + 2); Y = g.ly + 1; }
-        else if (k < 2 * (g.lx + 2) + g.ly) { X = 0; Y = k - 2 * (g.lx + 2) + 1; }
-        else { X = g.lx + 1; Y = k - 2 * (g.lx + 2) - g.ly + 1; }
-        const long long o = g.idx(X, Y);
-#pragma unroll
-        for (int i = 0; i < 9; ++i) {
-            const S t = plane(b0, g, i)[o];
-            plane(b0, g, i)[o] = plane(b1, g, i)[o];
-            plane(b1, g, i)[o] = t;
-        }
-    }
-}
-
 // ---- AA scheme ----------------------------------------------------------------------------
 
 // Even step at node (X, Y): own natural slots (stale ones from the side store) -> collide ->
@@ -1359,7 +720,7 @@ __device__ __forceinline__ void batch_strip(const BatchInst *__restrict__ insts,
     const BatchInst &d = insts[it.inst];
     const Geo g = d.g;
     const int passes = batch_passes(it.sp);
-    S *side = static_cast<S *>(d.side) + (size_t)((d.tau0 + k) & 1) * 9 * (size_t)g.nper;
+    S *side = static_cast<S *>(d.side) + (size_t)d.side_slot[(d.tau0 + k) & 1] * 9 * (size_t)g.nper;
     const double omega = d.omega;
     const float sc = d.scale, inv = d.inv_scale;
     if constexpr (KIND == BATCH_PULL4) {
@@ -1808,34 +1169,7 @@ __global__ void __launch_bounds__(BX) k_velocity_change(Geo g, int view, const S
     if ((threadIdx.x & 31) == 0) atomicMax(out, __float_as_uint(d));
 }
 
-inline unsigned cdiv(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
-
-template <class S> S *B(const DevLattice &d, int b) { return static_cast<S *>(d.buf[b]); }
-// The `other` argument of logical(): the pull scheme's second buffer, or the AA ring copy.
-template <class S> S *OTHER(const DevLattice &d, int cur)
-{
-    return d.buf[1] ? static_cast<S *>(d.buf[1 - cur]) : static_cast<S *>(d.ghost2);
-}
-template <class S> S *SIDE(const DevLattice &d, int p)
-{
-    return static_cast<S *>(d.side) + (size_t)(p & 1) * 9 * (size_t)d.g.nper;
-}
-// Pull scheme only: the scratch slot after the two parities (see k_sweep2).
-template <class S> S *SIDE_TMP(const DevLattice &d)
-{
-    return static_cast<S *>(d.side) + 2 * 9 * (size_t)d.g.nper;
-}
-
 }  // namespace
-
-// Run F<S>() with S the lattice's storage type.
-#define LBGPU_DISPATCH(d, BODY)                                        \
-    switch ((d).precision) {                                          \
-    case LBGPU_F64: { using S = double; BODY; } break;                \
-    case LBGPU_F32: { using S = float; BODY; } break;                 \
-    case LBGPU_F16: { using S = __half; BODY; } break;                \
-    default: { using S = __nv_bfloat16; BODY; } break;                \
-    }
 
 void launch_collide_inplace(const DevLattice &d, int cur, int side_par, cudaStream_t s)
 {
@@ -1913,76 +1247,6 @@ void launch_pull(const DevLattice &d, int src, int side_par, bool ghosts, cudaSt
         LBGPU_DISPATCH(d, (k_pull<S, false><<<grid, BX, 0, s>>>(d.g, B<S>(d, src), B<S>(d, 1 - src),
                            d.tag, d.bc, d.omega, SIDE<S>(d, side_par), d.scale, d.inv_scale)));
     }
-}
-
-template <class S, int W, int H, bool RS = false>
-static void launch_sweep2_t(const DevLattice &d, int src, int n_par, cudaStream_t s)
-{
-    constexpr size_t smem = sweep2_smem_bytes<S, W>();
-    cudaFuncSetAttribute(k_sweep2<S, W, H, RS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    dim3 grid(cdiv(d.g.lx, W), cdiv(d.g.ly, H));
-    k_sweep2<S, W, H, RS><<<grid, W + 2, smem, s>>>(d.g, B<S>(d, src), B<S>(d, 1 - src), d.tag, d.bc, d.omega,
-                                         SIDE<S>(d, n_par + 1), SIDE_TMP<S>(d), SIDE<S>(d, n_par), d.scale,
-                                         d.inv_scale);
-}
-
-// The register form (k_sweep2w) of the two-step sweep for the storage types whose bit is set in
-// LBGPU_SWEEP2_REG (1 FP64, 2 FP32, 4 FP16 / BF16); the others use the shared-memory form.
-// Measured on the 16384 x 4096 channel (GLUPS, register / shared-memory form): FP64 38.8 / 37.4,
-// FP32 77.3 / 70.4, FP16 58.1 / 63.0.
-#ifndef LBGPU_SWEEP2_REG
-#define LBGPU_SWEEP2_REG 3
-#endif
-#ifndef LBGPU_SWEEP2W_H
-#define LBGPU_SWEEP2W_H 128     // rows a warp walks
-#endif
-template <class S, bool RS = false>
-static void launch_sweep2w_t(const DevLattice &d, int src, int n_par, cudaStream_t s)
-{
-    const int strips = cdiv(d.g.lx, SW2_OUT);
-    dim3 grid(cdiv(strips, 4), cdiv(d.g.ly, LBGPU_SWEEP2W_H));
-    k_sweep2w<S, LBGPU_SWEEP2W_H, RS><<<grid, 128, 0, s>>>(d.g, B<S>(d, src), B<S>(d, 1 - src), d.tag, d.bc,
-                                                          d.omega, SIDE<S>(d, n_par + 1), SIDE_TMP<S>(d),
-                                                          SIDE<S>(d, n_par), d.scale, d.inv_scale);
-}
-
-void launch_pull2(const DevLattice &d, int src, int n_par, cudaStream_t s)
-{
-    constexpr bool reg64 = (LBGPU_SWEEP2_REG & 1) != 0, reg32 = (LBGPU_SWEEP2_REG & 2) != 0,
-                   reg16 = (LBGPU_SWEEP2_REG & 4) != 0;
-    switch (d.precision) {
-    case LBGPU_F64:
-        if (reg64) launch_sweep2w_t<double>(d, src, n_par, s);
-        else launch_sweep2_t<double, 126, 128>(d, src, n_par, s);
-        break;
-    case LBGPU_F32:
-        if (reg32) launch_sweep2w_t<float>(d, src, n_par, s);
-        else launch_sweep2_t<float, 126, 128>(d, src, n_par, s);
-        break;
-    case LBGPU_F16:
-        if (reg16) {
-            if (d.g.rs_key) launch_sweep2w_t<__half, true>(d, src, n_par, s);
-            else launch_sweep2w_t<__half>(d, src, n_par, s);
-        } else if (d.g.rs_key) {
-            launch_sweep2_t<__half, 126, 128, true>(d, src, n_par, s);
-        } else {
-            launch_sweep2_t<__half, 126, 128>(d, src, n_par, s);
-        }
-        break;
-    default:
-        if (reg16) {
-            if (d.g.rs_key) launch_sweep2w_t<__nv_bfloat16, true>(d, src, n_par, s);
-            else launch_sweep2w_t<__nv_bfloat16>(d, src, n_par, s);
-        } else if (d.g.rs_key) {
-            launch_sweep2_t<__nv_bfloat16, 126, 128, true>(d, src, n_par, s);
-        } else {
-            launch_sweep2_t<__nv_bfloat16, 126, 128>(d, src, n_par, s);
-        }
-        break;
-    }
-    const int nthreads = std::max(d.g.nper, d.g.nghost());
-    LBGPU_DISPATCH(d, (k_pull2_finish<S><<<cdiv(nthreads, 256), 256, 0, s>>>(d.g, B<S>(d, 0), B<S>(d, 1),
-                       SIDE_TMP<S>(d), SIDE<S>(d, n_par + 1))));
 }
 
 void launch_stream(const DevLattice &d, int src, int side_par, cudaStream_t s)

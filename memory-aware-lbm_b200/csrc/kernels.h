@@ -11,7 +11,11 @@ struct DevLattice {
     Geo g;
     int precision;       // LBGPU_F64 / F32 / F16 / BF16: element type of buf and side
     void *buf[2];        // population buffers (buf[1] unused by the AA scheme)
-    void *side;          // stale-slot store [2][9][nper] (+ a scratch [9][nper] for pull lattices)
+    void *side;          // stale-slot store: slots of [9][nper], two (AA) or three (pull)
+    int side_slot[2];    // the slot of each collision parity
+    int ghost_flip;      // 1: the ring that belongs to the second buffer is in the current one (launch_tile)
+    int rules_inside;    // some node off the perimeter has a boundary rule
+    int outlet_tiles;    // the extrapolated outlet's nodes lie where the tile kernel extrapolates them
     void *ghost2;        // AA only: the second buffer's ghost ring [9][nghost] (see logical())
     const uint8_t *tag;  // tag plane
     double *bc;          // boundary tables [8][2][nb]
@@ -34,10 +38,14 @@ void launch_pull(const DevLattice &d, int src, int side_par, bool ghosts, cudaSt
 // perimeter kernel).
 int pull_launches(const DevLattice &d, bool ghosts);
 void launch_stream(const DevLattice &d, int src, int side_par, cudaStream_t s);
-// Two pull steps in one sweep (temporal blocking): C_n in buffer src (n_par = n & 1) ->
-// C_{n+2} in buffer 1 - src, then the stale-slot scratch into parity n+1 and the two buffers'
-// ghost rings exchanged.  Pull lattices without ghost-ring output only.
-void launch_pull2(const DevLattice &d, int src, int n_par, cudaStream_t s);
+// Pull steps per launch of the tile kernel (tile.cu) for a run of `steps` steps from form C pending:
+// 0 where single steps are the faster way (or the only one).  `outlet`: the outlet is
+// extrapolated before every step.
+int tile_steps(const DevLattice &d, long long steps, bool outlet);
+// T pull steps (a count that tile_steps returned) in one launch: C_n in buffer src (n_par = n & 1)
+// -> C_{n+T} in buffer 1 - src, where T single steps would have left it in src: ghost_flip changes,
+// and the side store's slots change roles.  keys: rounding keys of the T collisions (16-bit).
+void launch_tile(DevLattice &d, int src, int n_par, int T, bool outlet, const unsigned *keys, cudaStream_t s);
 void launch_side_from_buf(const DevLattice &d, int b, int side_par, cudaStream_t s);
 // AA only: keep buffer b's ghost ring as the second buffer's (d.ghost2).
 void launch_ghost_copy(const DevLattice &d, int b, cudaStream_t s);
@@ -85,6 +93,7 @@ struct BatchInst {
     Geo g;
     void *buf[2];
     void *side;
+    int side_slot[2];
     const uint8_t *tag;
     const double *bc;
     double omega;

@@ -83,7 +83,7 @@ int Lattice::create(int lx_, int ly_, int precision_, int scheme_)
 
     const size_t nbuf = (scheme == LBGPU_AA) ? 1 : 2;
     const size_t pbytes = 9 * (size_t)d.g.plane * elem;
-    // two parities, and for the pull scheme the scratch of the two-step kernel
+    // two parities, and for the pull scheme the slot the tile kernel writes beside them
     const size_t sbytes = (scheme == LBGPU_PULL ? 3 : 2) * 9 * (size_t)d.g.nper * elem;
     void *p = nullptr;
     for (size_t b = 0; b < nbuf; ++b) {
@@ -100,6 +100,7 @@ int Lattice::create(int lx_, int ly_, int precision_, int scheme_)
     }
     LB_CUDA(cudaMalloc(&p, sbytes), "cudaMalloc(side store)");
     d.side = p;
+    reset_roles();
     LB_CUDA(cudaMemsetAsync(p, 0, sbytes, stream), "cudaMemset(side store)");
     LB_CUDA(cudaMalloc(&p, (size_t)d.g.plane), "cudaMalloc(tags)");
     d.tag = static_cast<const uint8_t *>(p);
@@ -119,6 +120,14 @@ int Lattice::create(int lx_, int ly_, int precision_, int scheme_)
     zgb_src_host.assign(4 * (size_t)d.g.nb, -1);
     cur = 0; form = FORM_L; pending = 0; n = 0;
     return check("lattice create");
+}
+
+// The state is written afresh: each parity's stale slots in its own slot, each ring in its buffer.
+void Lattice::reset_roles()
+{
+    d.side_slot[0] = 0;
+    d.side_slot[1] = 1;
+    d.ghost_flip = 0;
 }
 
 void Lattice::destroy()
@@ -162,7 +171,6 @@ void Lattice::view(int &v, int &par) const
 void Lattice::set_rs_keys(long long k)
 {
     d.g.rs_key = rs ? rs_key(rs_seed, (unsigned long long)k) : 0u;
-    d.g.rs_key2 = rs ? rs_key(rs_seed, (unsigned long long)(k + 1)) : 0u;
 }
 
 // ---- state machine (pull scheme) ------------------------------------------------------
@@ -253,18 +261,23 @@ int Lattice::step(int nsteps)
     if (nsteps < 0) return set_error(LB_ERR_ARG, "negative step count");
     launches = 0;
     for (int s = 0; s < nsteps; ++s) {
+        // a run of pull steps: several a launch, the state as single steps leave it
+        if (scheme == LBGPU_PULL && !ghosts && form == FORM_C && pending) {
+            if (const int T = tile_steps(d, nsteps - s, zgb_each_step)) {
+                unsigned keys[8] = {0};
+                for (int k = 0; rs && k < T; ++k) keys[k] = rs_key(rs_seed, (unsigned long long)(n + 1 + k));
+                launch_tile(d, cur, (int)(n & 1), T, zgb_each_step, keys, stream);
+                cur = 1 - cur;
+                n += T;
+                s += T - 1;
+                ++launches;
+                LB_TRY(check("tile steps"));
+                continue;
+            }
+        }
         if (zgb_each_step) LB_TRY(zgb_pass());
         if (scheme == LBGPU_AA) {
             LB_TRY(aa_step());
-        } else if (sweep_steps == 2 && nsteps - s >= 2 && !zgb_each_step && !ghosts && form == FORM_C && pending) {
-            // two steps in one sweep: C_n -> C_{n+2} in the other buffer, still pending
-            set_rs_keys(n + 1);
-            launch_pull2(d, cur, (int)(n & 1), stream);
-            launches += 2;
-            cur = 1 - cur;
-            n += 2;
-            ++s;
-            LB_TRY(check("two-step pull"));
         } else {
             LB_TRY(op_collide());
             LB_TRY(op_propagate());
@@ -485,8 +498,9 @@ int Lattice::upload_tag_plane(const uint8_t *plane)
     return LB_OK;
 }
 
-int Lattice::upload_tags(const uint8_t *tag_xy)
+int Lattice::upload_tags(const uint8_t *tag_xy, const uint8_t *zgb_row)
 {
+    int inside = 0, outlet = lx >= 4;
     for (int X = 0; X < lx + 2; ++X)
         for (int Y = 0; Y < ly + 2; ++Y) {
             const int t = tag_xy[(size_t)X * (ly + 2) + Y];
@@ -494,8 +508,15 @@ int Lattice::upload_tags(const uint8_t *tag_xy)
                 return set_error(LB_ERR_ARG, "tag %d at (%d,%d) out of range", t, X, Y);
             if (d.g.interior(X, Y) && t == LBGPU_TAG_NONE)
                 return set_error(LB_ERR_DYNAMICS, "interior node (%d,%d) has no dynamics", X, Y);
+            if (t >= LBGPU_TAG_UPPER_ZOUHE && X > 1 && X < lx && Y > 1 && Y < ly) inside = 1;
+            // an extrapolated row's pressure nodes anywhere but at its end, or the rows at the walls
+            const bool right = t == LBGPU_TAG_RIGHT_PRESSURE_ZOUHE || t == LBGPU_TAG_RIGHT_PRESSURE_REGULARIZED;
+            if (zgb_row && zgb_row[Y] && right && (X != lx || Y < 2 || Y > ly - 1)) outlet = 0;
         }
-    return upload_tags_xy(tag_xy);
+    LB_TRY(upload_tags_xy(tag_xy));
+    d.rules_inside = inside;
+    d.outlet_tiles = outlet;
+    return LB_OK;
 }
 
 // The host array in its own order to the device, transposed there (a host transpose writes one

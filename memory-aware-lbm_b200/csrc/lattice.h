@@ -32,7 +32,7 @@ struct Lattice {
     long long n = 0;     // index of the last collision (form C) or of the state (form L)
     bool ghosts = false; // keep the ghost ring exact (drop-in interface)
     bool zgb_each_step = false;  // native: extrapolated outlet before every step
-    int sweep_steps = 1;         // pull scheme: 2 = two steps per sweep where eligible (k_sweep2)
+    int sweep_steps = 1;         // lbgpu_set_sweep_steps (runs of pull steps share launches either way)
     cudaStream_t stream = nullptr;
     size_t bytes = 0;
     int launches = 0;    // kernels launched by the last public call
@@ -46,6 +46,7 @@ struct Lattice {
 
     int create(int lx, int ly, int precision, int scheme);
     void destroy();
+    void reset_roles();
 
     // per-step operations (asynchronous on `stream`)
     int op_collide();        // collide the current state in place or through the pull kernel
@@ -60,7 +61,8 @@ struct Lattice {
     // data movement
     int upload_bc(const double *bc);      // host [16*nb]
     int upload_zgb_src(const int *src);   // host [4*nb]
-    int upload_tags(const uint8_t *tag_xy);  // host tag[X*(ly+2)+Y], validated here
+    // host tag[X*(ly+2)+Y], validated here; zgb_row: rows of the extrapolated outlet, or null
+    int upload_tags(const uint8_t *tag_xy, const uint8_t *zgb_row);
     int upload_tag_plane(const uint8_t *plane);  // host plane in device layout
     int upload_records(int b, const double *host, int rs, int X0, int X1);
     // rows Y0..Y0+H-1 of columns X0..X1-1 from host records laid out like upload_records' (host

@@ -32,9 +32,9 @@ struct Geo {
     // some rebase[Y][i] is not zero, else 0 (a profile constant over bands of rows needs the
     // rebase only on the rows at a band's edge).
     const float *shift_u;
-    // 16-bit storage only: stochastic rounding keys (codec.cuh) of the launch's collision and,
-    // for the two-step sweep, of the second one; 0 rounds to nearest.
-    unsigned rs_key, rs_key2;
+    // 16-bit storage only: stochastic rounding key (codec.cuh) of the launch's collision; 0 rounds to
+    // nearest.
+    unsigned rs_key;
     __host__ __device__ __forceinline__ const float *shift_base(int Y) const { return shift_u + (ly + 2) + 9 * Y; }
     __host__ __device__ __forceinline__ const float *shift_rebase(int Y) const
     {
@@ -87,7 +87,6 @@ inline Geo make_geo(int lx, int ly, int elem_bytes)
     g.nper = 2 * lx + 2 * ly;
     g.shift_u = nullptr;
     g.rs_key = 0;
-    g.rs_key2 = 0;
     return g;
 }
 

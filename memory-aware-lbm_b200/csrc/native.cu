@@ -110,7 +110,7 @@ int lbgpu_set_geometry(lbgpu_lattice *h, double omega, const uint8_t *tag, const
     Lattice &L = h->L;
     if (zgb_wanted(zgb_row, L.ly) && L.lx < 2)
         return set_error(LB_ERR_ARG, "extrapolated outlet needs lx >= 2");
-    if (int rc = L.upload_tags(tag)) return rc;
+    if (int rc = L.upload_tags(tag, zgb_row)) return rc;
     return set_tables(L, omega, bc, zgb_row);
 }
 
@@ -182,7 +182,6 @@ int lbgpu_set_stochastic_rounding(lbgpu_lattice *h, int on, unsigned seed)
     L.rs = on != 0;
     L.rs_seed = seed;
     L.d.g.rs_key = 0;
-    L.d.g.rs_key2 = 0;
     return LB_OK;
 }
 
@@ -192,6 +191,7 @@ int lbgpu_set_populations(lbgpu_lattice *h, const double *f, const double *tmp)
     if (!f) return set_error(LB_ERR_ARG, "lbgpu_set_populations: null populations");
     Lattice &L = h->L;
     L.launches = 0;
+    L.reset_roles();
     if (L.scheme == LBGPU_AA) {
         // one buffer: the second buffer only matters through its stale slots (side parity 1,
         // read by the first odd step); the first buffer's own stale slots go to parity 0
@@ -244,6 +244,9 @@ int lbgpu_setup_cylinder(lbgpu_lattice *h, int obst_x, int obst_y, int obst_r, d
     lbgpu::launch_cylinder_tags(L.d, obst_x, obst_y, obst_r, wall_kind, L.stream);
     if (int rc = lbgpu::cuda_error(cudaGetLastError(), "cylinder tags")) return rc;
     if (int rc = set_tables(L, omega, bc.data(), zgb.data())) return rc;
+    L.d.rules_inside = 0;
+    L.d.outlet_tiles = L.lx >= 4;
+    L.reset_roles();
     L.launches = 0;
     for (int b = 0; b < 2; ++b)
         if (L.d.buf[b])

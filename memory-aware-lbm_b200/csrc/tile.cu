@@ -1,0 +1,142 @@
+// tile.cu -- runs of pull steps, several steps a launch on tiles in shared memory (tile.cuh): which
+// shape of tile a lattice takes, and the launch.
+#include "kernels.h"
+#include "node.cuh"
+
+namespace lbgpu {
+
+namespace {
+
+#include "tile.cuh"
+
+// The shapes by storage type and node count, from a sweep of about ten shapes over channels of 250 x 51 to 8192 x
+// 2048 (us a step in a graph of launches; the next best shape or the single-step kernel in parentheses):
+//   small lattices: many steps a launch on small tiles, so that every SM has a tile and the launch is
+//     shared: FP64 250 x 51 2.4 (4 steps 2.8, single 3.5), FP32 1.5 (1.9, 3.3), FP16 1.9 (2.2, 6.7)
+//   511 x 127: FP64 3.8 (5.0 with 2 steps, single 4.0), FP32 2.5 (2.6 with 8 steps, single 3.5)
+//   700 x 200: FP64 5.4 (5.6 with 2 steps), FP32 2.9 (3.2 on 32 x 8 tiles, single 4.3), FP16 3.5 (7.2)
+//   1024 x 256: FP64 7.4 (8.3 with 4 steps, single 7.0 in a graph and 9.0 launched), FP32 4.2 (5.2 with 2, 5.5)
+//   2047 x 511: FP64 21.9 (24.2 on 64 x 16, single 27.7), FP32 10.1 (11.1 with 4 steps, 12.8), FP16 11.4 (12.3)
+//   large: two steps, tiles whose halo is small against them, and few enough threads' registers for
+//     several blocks a SM: 8192 x 2048 FP64 233 (two blocks of 64 x 16; 236 with four of 32 x 16; single 355), FP32
+//     109 (five of 64 x 12; 111 with six of 64 x 8; single 187).  16-bit storage has k_pull4h there.
+// Large lattices prefetch the tile 100 (FP64) or 200 (FP32) blocks ahead into L2: 253 -> 233 and 120 -> 109 us;
+// 0.3 of that distance does half as much, 4 times it costs 15-30 % (evicted before it is read).
+using F64Small = TileShape<double, 16, 8, 8, 704, 1>;
+using F64Mid = TileShape<double, 32, 8, 4, 288, 2>;
+using F64Wide = TileShape<double, 32, 8, 2, 352, 3>;
+using F64Large = TileShape<double, 64, 16, 2, 512, 2>;
+using F32Small = TileShape<float, 16, 8, 8, 768, 1>;
+using F32Mid = TileShape<float, 32, 8, 4, 288, 3>;
+using F32Wide = TileShape<float, 32, 16, 4, 448, 2>;
+using F32Large = TileShape<float, 64, 12, 2, 224, 5>;
+template <class S> using HalfSmall = TileShape<S, 16, 8, 8, 384, 2>;
+template <class S> using HalfWide = TileShape<S, 32, 16, 4, 416, 3>;
+
+enum { TILE_SMALL = 0, TILE_MID = 1, TILE_WIDE = 2, TILE_LARGE = 3, TILE_NONE = 4 };
+
+// Node counts below which a shape is the fastest.
+constexpr long long kF64[3] = {40 << 10, 120 << 10, 3 << 20};
+constexpr long long kF32[3] = {40 << 10, 100 << 10, 700 << 10};
+constexpr long long kHalf[3] = {60 << 10, 60 << 10, 2 << 20};
+
+int tile_shape(const DevLattice &d)
+{
+    const long long n = (long long)d.g.lx * d.g.ly;
+    const long long *k = d.precision == LBGPU_F64 ? kF64 : (d.precision == LBGPU_F32 ? kF32 : kHalf);
+    return n < k[0] ? TILE_SMALL : (n < k[1] ? TILE_MID : (n < k[2] ? TILE_WIDE : TILE_LARGE));
+}
+
+template <class SH, bool RS, bool EXTRAP>
+void launch_shape(const DevLattice &d, int src, int n_par, int pf, const unsigned *keys, cudaStream_t s)
+{
+    using S = typename SH::S;
+    TileArgs<S> a;
+    a.g = d.g;
+    a.src = B<S>(d, src);
+    a.dst = B<S>(d, 1 - src);
+    a.tag = d.tag;
+    a.bc = d.bc;
+    a.zgb = d.zgb_src + 3 * d.g.nb;
+    a.omega = d.omega;
+    a.omega_f = (float)d.omega;
+    // step 1 reads the stale slots of C_{n-1}; the last step's replace those of C_n, which has them in
+    // its own slots, and the step's before it go to the free slot
+    a.stale1 = SIDE<S>(d, n_par + 1);
+    a.out_last = SIDE<S>(d, n_par);
+    a.out_prev = SIDE_FREE<S>(d);
+    a.sc = d.scale;
+    a.inv = d.inv_scale;
+    // the outlet's extrapolation reads three columns back: its tile must not be narrower
+    a.x_first = EXTRAP && d.g.lx > SH::W && (d.g.lx % SH::W == 1 || d.g.lx % SH::W == 2) ? -3 : 1;
+    a.nx = (int)cdiv(d.g.lx - a.x_first + 1, SH::W);
+    a.ny = (int)cdiv(d.g.ly, SH::H);
+    a.pf = a.x_first == 1 ? pf : 0;
+    a.rules_inside = d.rules_inside;
+    for (int k = 0; k < 8; ++k) a.keys[k] = keys[k];
+    cudaFuncSetAttribute(k_tile<SH, RS, EXTRAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SH::SMEM);
+    k_tile<SH, RS, EXTRAP><<<(unsigned)a.nx * (unsigned)a.ny, SH::NT, SH::SMEM, s>>>(a);
+}
+
+template <class SH>
+void launch_one(const DevLattice &d, int src, int n_par, bool outlet, int pf, const unsigned *keys, cudaStream_t s)
+{
+    if constexpr (sizeof(typename SH::S) == 2) {
+        if (keys[0] != 0) {
+            if (outlet) launch_shape<SH, true, true>(d, src, n_par, pf, keys, s);
+            else launch_shape<SH, true, false>(d, src, n_par, pf, keys, s);
+            return;
+        }
+    }
+    if (outlet) launch_shape<SH, false, true>(d, src, n_par, pf, keys, s);
+    else launch_shape<SH, false, false>(d, src, n_par, pf, keys, s);
+}
+
+template <class S>
+void launch_half(const DevLattice &d, int src, int n_par, int T, bool outlet, const unsigned *keys, cudaStream_t s)
+{
+    if (T == 8) launch_one<HalfSmall<S>>(d, src, n_par, outlet, 0, keys, s);
+    else launch_one<HalfWide<S>>(d, src, n_par, outlet, 0, keys, s);
+}
+
+}  // namespace
+
+int tile_steps(const DevLattice &d, long long steps, bool outlet)
+{
+    if (steps < 2 || (outlet && !d.outlet_tiles)) return 0;
+    const int shape = tile_shape(d);
+    if (d.precision == LBGPU_F16 || d.precision == LBGPU_BF16) {
+        // row-shifted offsets are rebased between rows, and large lattices have the quads of k_pull4h
+        if (d.g.shift_u || shape == TILE_LARGE) return 0;
+        return shape == TILE_SMALL && steps >= 8 ? 8 : (steps >= 4 ? 4 : 0);
+    }
+    if (shape == TILE_SMALL && steps >= 8) return 8;
+    if (steps >= 4 && (shape <= TILE_MID || (shape == TILE_WIDE && d.precision == LBGPU_F32))) return 4;
+    return 2;
+}
+
+void launch_tile(DevLattice &d, int src, int n_par, int T, bool outlet, const unsigned *keys, cudaStream_t s)
+{
+    const int shape = tile_shape(d);
+    switch (d.precision) {
+    case LBGPU_F64:
+        if (T == 8) launch_one<F64Small>(d, src, n_par, outlet, 0, keys, s);
+        else if (T == 4) launch_one<F64Mid>(d, src, n_par, outlet, 0, keys, s);
+        else if (shape == TILE_LARGE) launch_one<F64Large>(d, src, n_par, outlet, 100, keys, s);
+        else launch_one<F64Wide>(d, src, n_par, outlet, 0, keys, s);
+        break;
+    case LBGPU_F32:
+        if (T == 8) launch_one<F32Small>(d, src, n_par, outlet, 0, keys, s);
+        else if (T == 4 && shape == TILE_WIDE) launch_one<F32Wide>(d, src, n_par, outlet, 0, keys, s);
+        else if (T == 4) launch_one<F32Mid>(d, src, n_par, outlet, 0, keys, s);
+        else launch_one<F32Large>(d, src, n_par, outlet, shape == TILE_LARGE ? 200 : 0, keys, s);
+        break;
+    case LBGPU_F16: launch_half<__half>(d, src, n_par, T, outlet, keys, s); break;
+    default: launch_half<__nv_bfloat16>(d, src, n_par, T, outlet, keys, s); break;
+    }
+    const int a = (n_par + 1) & 1;
+    d.side_slot[a] = 3 - d.side_slot[0] - d.side_slot[1];
+    d.ghost_flip ^= 1;
+}
+
+}  // namespace lbgpu

@@ -1,0 +1,121 @@
+"""Runs of pull steps (several steps a launch on tiles) against single steps.
+
+The contract: lbgpu_step(n) leaves the state that n calls of lbgpu_step(1) leave, bit for bit, ghost ring
+and stale slots included, in every storage type, whatever tile shape the size takes.  Sizes lie at
+tile edges (one node more or less than a tile, one or two columns in the last tile) and on either
+side of the node counts where the shape changes.
+"""
+import numpy as np
+import pytest
+
+import lbgpu
+import oracle as O
+from helpers import describe_diff, same
+
+pytestmark = pytest.mark.gpu
+
+SCALE = {"f16": 10, "bf16": 6}
+
+
+def run(st, plan, precision, rs=None):
+    with lbgpu.Lattice(st.lx, st.ly, precision, "pull") as lat:
+        if precision in SCALE:
+            lat.set_offset_scale(SCALE[precision])
+        lat.set_geometry(st.omega, st.tag, st.bc, st.zgb)
+        lat.set_populations(st.lat, st.tmp)
+        if rs is not None:
+            lat.set_stochastic_rounding(True, rs)
+        for n in plan:
+            lat.step(n)
+        assert lat.steps_done == sum(plan)
+        return lat.populations(), lat.macros(), lat.moments()
+
+
+def agree(st, precision, plan, rs=None):
+    one = run(st, [1] * sum(plan), precision, rs)
+    got = run(st, plan, precision, rs)
+    assert same(got[0], one[0]), (precision, st.lx, st.ly, describe_diff(got[0], one[0]))
+    for a, b in zip(got[1], one[1]):
+        assert same(a, b)
+    assert same(got[2], one[2])
+    return got[0]
+
+
+EDGES = [(5, 4), (16, 8), (17, 9), (31, 25), (66, 33), (129, 17)]
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32", "f16", "bf16"])
+@pytest.mark.parametrize("size", EDGES)
+def test_every_boundary_rule_anywhere(precision, size):
+    lx, ly = size
+    st = O.random_boundary_lattice(lx, ly, seed=lx * 7 + ly)
+    for i, t in enumerate(range(3, 19)):     # and off the perimeter
+        st.tag[2 + (5 * i) % (lx - 2), 2 + (3 * i) % (ly - 2)] = t
+    got = agree(st, precision, [1, 2, 9, 13, 20])
+    if precision == "f64":
+        exp = O.run(st, 45).lat
+        assert same(got, exp), describe_diff(got, exp)
+
+
+# one and two columns past a multiple of every tile width, and a width below four columns
+@pytest.mark.parametrize("precision", ["f64", "f32", "f16", "bf16"])
+@pytest.mark.parametrize("size", [(17, 12), (34, 11), (65, 23), (130, 31), (67, 29)])
+def test_extrapolated_outlet(precision, size):
+    st = O.build_cylinder(O.Cylinder.reference_driver(*size))
+    got = agree(st, precision, [1, 7, 12, 23])
+    if precision == "f64":
+        exp = O.run(st, 43).lat
+        assert same(got, exp), describe_diff(got, exp)
+
+
+def test_extrapolated_outlet_of_a_custom_geometry():
+    """A pressure node of an extrapolated row before the row's end keeps single steps."""
+    st = O.build_cylinder(O.Cylinder.reference_driver(40, 20))
+    st.tag[20, 10] = 18
+    got = agree(st, "f64", [3, 14])
+    assert same(got, O.run(st, 17).lat)
+
+
+# either side of the node counts where the tile shape changes
+@pytest.mark.parametrize("precision,sizes", [
+    ("f64", [(257, 160), (401, 310), (2100, 1500)]),
+    ("f32", [(257, 160), (700, 200), (1030, 700)]),
+    ("f16", [(401, 160), (1030, 130)]),
+    ("bf16", [(401, 160), (1030, 130)]),
+])
+def test_every_tile_shape(precision, sizes):
+    for lx, ly in sizes:
+        def go(plan):
+            with lbgpu.Lattice(lx, ly, precision, "pull") as lat:
+                if precision in SCALE:
+                    lat.set_offset_scale(SCALE[precision])
+                lat.setup_cylinder(lx // 5 + 1, ly // 2 + 1, ly // 10 + 1, 0.03, 80.0, lbgpu.WALL_REGULARIZED,
+                                   lbgpu.OUTLET_CONST)
+                for n in plan:
+                    lat.step(n)
+                return lat.populations()
+        a, b = go([3, 15]), go([1] * 18)
+        assert same(a, b), (precision, lx, ly, describe_diff(a, b))
+
+
+@pytest.mark.parametrize("precision", ["f16", "bf16"])
+def test_stochastic_rounding(precision):
+    st = O.build_cylinder(O.Cylinder.baseline(150, 41))
+    agree(st, precision, [1, 8, 13, 21], rs=7)
+
+
+def test_infinite_and_nan_velocities_as_the_reference_has_them():
+    """The short forms of the FP64 rules stand aside where 0 times a velocity is not 0."""
+    st = O.random_boundary_lattice(40, 24, seed=11)
+    f = st.lat.reshape(42, 26, 9)
+    f[5, 5, 1] = np.inf
+    f[20, 12, 2] = -np.inf
+    f[30, 20, 0] = np.nan
+    f[12, 18] = 0.0
+    f[12, 18, 1] = 1e-3        # a density that nearly cancels
+    f[12, 18, 3] = -1e-3
+    f[33, 6, 5] = 1e200        # a velocity whose square overflows
+    for steps in (1, 2, 5):
+        got = run(st, [steps], "f64")[0]
+        exp = O.run(st, steps).lat
+        assert same(got, exp), steps
