@@ -6,10 +6,13 @@
 // two lists by the parity of their phase, so each list runs one kind at a time).  A launch
 // walks a work list of tiles (member, x0, y0, shape) of 128, 256 or 512 nodes, one per thread
 // (or four per thread): either one block per tile, or a persistent grid of (blocks per SM x
-// SMs) blocks strides through it.  Steps are grouped in chunks of 50 (an even count) captured
+// SMs) blocks strides through it.  Steps are grouped in chunks of 20 captured
 // once as a CUDA graph: the kernels read each member's buffers and parities from a device
 // descriptor array, so the same graph replays chunk after chunk; it is re-captured when the
 // membership or the launch form changes.
+// FP64 and FP32 pull members take two steps a launch on tiles in shared memory (tile.cuh), one work list of tiles for
+// all of them: 24 uneven channels of 8.6M nodes in FP32 119 -> 75 us a step, 24 of 5.7M nodes in FP64 162 -> 108,
+// 24 small ones (0.7M nodes) in FP32 20.7 -> 8.3.
 // A work item is a strip of tiles of one member stacked in y: its block reads the member's
 // descriptor once and steps the tiles one after another down the lattice, so the descriptor's
 // dependent loads are spread over the strip.  Tile widths and strip lengths are chosen per size
@@ -29,9 +32,13 @@ using lbgpu::set_error;
 namespace {
 
 constexpr int kClasses = 6;     // node-count classes: < 16K, 64K, 256K, 1M, 4M, above
-constexpr int kChunk = 50;      // steps per captured graph (even: buffer parities repeat)
-constexpr int kLists = 5;       // pull, pull four nodes a thread; AA of phase parity 0, 1 at rebuild;
-                                // the perimeters of the four-nodes-a-thread members
+constexpr int kChunk = 20;      // steps per captured graph (a multiple of 4: the buffers' and the side store's
+                                // parities repeat after two two-step launches)
+constexpr int kLists = 6;       // pull, pull four nodes a thread; AA of phase parity 0, 1 at rebuild;
+                                // the perimeters of the four-nodes-a-thread members; the tiles of the
+                                // pull members that take two steps a launch (list 0 holds them too,
+                                // for a single step)
+constexpr int kTiles = 5;
 constexpr int kQuad = 3;        // shape of the four-nodes-a-thread pull tiles (16-bit storage)
 constexpr int kMaxPasses = 64;  // tiles a block may step down one member
 
@@ -70,6 +77,7 @@ struct lbgpu_batch {
     cudaEvent_t order = nullptr;             // orders the batch stream against members' streams
     cudaGraphExec_t graph[2] = {nullptr, nullptr};   // one chunk, by aa_phase
     int launches = 0;
+    int chunk_launches = 0;                  // kernels of one chunk's graph
     bool rs = false;                         // some member rounds stochastically (set at rebuild)
     bool shift = false;                      // some member stores row-shifted offsets (set at rebuild)
 };
@@ -105,7 +113,19 @@ BatchInst describe(const Lattice &L)
     }
     b.rs = L.rs ? 1 : 0;
     b.rs_seed = L.rs_seed;
+    b.rules_inside = L.d.rules_inside;
     return b;
+}
+
+// Whether a descriptor still holds for a member (its collision number apart, of which kernels without
+// stochastic rounding use the parity only).
+bool describes(const BatchInst &b, const Lattice &L)
+{
+    const BatchInst now = describe(L);
+    return b.rs == now.rs && b.rs_seed == now.rs_seed && b.g.shift_u == now.g.shift_u && b.cur0 == now.cur0 &&
+           b.phase0 == now.phase0 && ((b.tau0 ^ now.tau0) & 1) == 0 && b.side_slot[0] == now.side_slot[0] &&
+           b.side_slot[1] == now.side_slot[1] && b.omega == now.omega && b.scale == now.scale &&
+           b.rules_inside == now.rules_inside;
 }
 
 // Stochastically rounded members key their collisions by number (tau0 + k), which a replayed
@@ -122,9 +142,20 @@ int refresh_collision_numbers(lbgpu_batch *b, int done)
                                        cudaMemcpyHostToDevice, b->stream), "update batch collision numbers");
 }
 
-// A member's host-side state after `m` batch steps (no launches).
-void advance(Lattice &L, int m)
+// Pull members of a storage type with a tile kernel take two steps a launch.
+bool takes_tiles(const Lattice &L)
 {
+    int w, h;
+    return L.scheme == LBGPU_PULL && lbgpu::batch_tile(L.precision, &w, &h);
+}
+
+// A member's host-side state after `m` batch steps (no launches); tiles: taken two a launch.
+void advance(Lattice &L, int m, bool tiles)
+{
+    if (tiles && takes_tiles(L)) {
+        for (; m >= lbgpu::BATCH_TILE_STEPS; m -= lbgpu::BATCH_TILE_STEPS) L.after_tile(lbgpu::BATCH_TILE_STEPS);
+        return;
+    }
     for (int s = 0; s < m; ++s) {
         if (L.scheme == LBGPU_PULL) {
             L.cur = 1 - L.cur;
@@ -174,7 +205,7 @@ void drop_graphs(lbgpu_batch *b)
 // Rebuild descriptors and work lists from the members' current states.
 int rebuild(lbgpu_batch *b)
 {
-    std::vector<BatchWork> work[kLists];
+    std::vector<BatchWork> work[kLists], inner;
     b->h_inst.assign(b->members.size(), BatchInst{});
     for (size_t i = 0; i < b->members.size(); ++i) {
         lbgpu_lattice *m = b->members[i];
@@ -189,10 +220,19 @@ int rebuild(lbgpu_batch *b)
         for (int y0 = 1; y0 <= L.ly; y0 += th)
             for (int x0 = 1; x0 <= L.lx; x0 += tw)
                 work[s].push_back(BatchWork{(int)i, x0, y0, lbgpu::batch_sp(sh, np)});
+        int w, h;
+        if (takes_tiles(L) && lbgpu::batch_tile(b->precision, &w, &h))
+            for (int y0 = 1; y0 <= L.ly; y0 += h)
+                for (int x0 = 1; x0 <= L.lx; x0 += w) {
+                    const bool ring = x0 == 1 || y0 == 1 || x0 + w > L.lx || y0 + h > L.ly;
+                    (ring ? work[kTiles] : inner).push_back(BatchWork{(int)i, x0, y0, 0});
+                }
         if (s == 1)   // its perimeter, one block a run of `threads` perimeter nodes
             for (int p0 = 0; p0 < 2 * L.lx + 2 * L.ly; p0 += b->threads)
                 work[4].push_back(BatchWork{(int)i, p0, 1, lbgpu::batch_sp(sh, 1)});
     }
+    // every member's outer tiles first: their boundary rules make them the longest
+    work[kTiles].insert(work[kTiles].end(), inner.begin(), inner.end());
     b->aa_phase = 0;
     b->rs = false;
     b->shift = false;
@@ -229,11 +269,12 @@ int rebuild(lbgpu_batch *b)
     return LB_OK;
 }
 
-// k-th step of a chunk: one launch per non-empty work list.
-void launch_step(lbgpu_batch *b, int k)
+// k-th single step of a chunk: one launch per non-empty work list (without_tiled: not of the list whose
+// members take two steps a launch).
+void launch_step(lbgpu_batch *b, int k, bool without_tiled)
 {
-    for (int s = 0; s < kLists; ++s) {
-        if (!b->nwork[s]) continue;
+    for (int s = 0; s < kTiles; ++s) {
+        if (!b->nwork[s] || (s == 0 && without_tiled)) continue;
         int kind = s == 0 ? lbgpu::BATCH_PULL : (s == 1 ? lbgpu::BATCH_PULL4 : lbgpu::BATCH_PERIM);
         if (s == 2 || s == 3) {
             const int phase = (s == 2) ? b->aa_phase : 1 - b->aa_phase;
@@ -248,11 +289,16 @@ void launch_step(lbgpu_batch *b, int k)
     }
 }
 
-int launches_per_step(const lbgpu_batch *b)
+// Steps 2 unit and 2 unit + 1 of a chunk.
+void launch_unit(lbgpu_batch *b, int unit)
 {
-    int n = 0;
-    for (int s = 0; s < kLists; ++s) n += b->nwork[s] ? 1 : 0;
-    return n;
+    if (b->nwork[kTiles]) {
+        lbgpu::launch_batch_tile(b->precision, b->d_inst, b->d_work[kTiles], b->nwork[kTiles], unit, b->stream);
+        ++b->launches;
+    }
+    const bool tiled = b->nwork[kTiles] > 0;
+    launch_step(b, 2 * unit, tiled);
+    launch_step(b, 2 * unit + 1, tiled);
 }
 
 int capture_chunk(lbgpu_batch *b)
@@ -260,7 +306,8 @@ int capture_chunk(lbgpu_batch *b)
     cudaGraph_t g = nullptr;
     if (int rc = batch_error(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "begin capture")) return rc;
     const int before = b->launches;
-    for (int k = 0; k < kChunk; ++k) launch_step(b, k);
+    for (int u = 0; u < kChunk / 2; ++u) launch_unit(b, u);
+    b->chunk_launches = b->launches - before;
     b->launches = before;
     cudaError_t e = cudaStreamEndCapture(b->stream, &g);
     if (e != cudaSuccess) return batch_error(e, "end capture");
@@ -471,16 +518,22 @@ int lbgpu_batch_step(lbgpu_batch *b, int nsteps)
         --nsteps;
         b->dirty = true;
     }
-    // rounding switched (or reseeded), or a row shift set or cleared, on a member since the
-    // descriptors were written
+    // what a member's descriptor says no longer holds: rounding switched (or reseeded), a row shift set or
+    // cleared, another geometry, or the member stepped on its own since
     for (size_t i = 0; i < b->members.size() && !b->dirty; ++i)
-        if (b->members[i] && (i >= b->h_inst.size() || b->h_inst[i].rs != (b->members[i]->L.rs ? 1 : 0) ||
-                              b->h_inst[i].rs_seed != b->members[i]->L.rs_seed ||
-                              b->h_inst[i].g.shift_u != b->members[i]->L.d.g.shift_u))
-            b->dirty = true;
+        if (b->members[i] && (i >= b->h_inst.size() || !describes(b->h_inst[i], b->members[i]->L))) b->dirty = true;
     if (b->dirty)
         if (int rc = rebuild(b)) return rc;
     if (int rc = order_before(b)) return rc;
+    // An odd count takes its single step first: what follows runs in pairs of steps.
+    if (nsteps & 1) {
+        launch_step(b, 0, false);
+        for (lbgpu_lattice *m : b->members)
+            if (m) advance(m->L, 1, false);
+        b->aa_phase ^= 1;      // the AA lists swap their kind of step
+        --nsteps;
+        if (int rc = refresh_collision_numbers(b, 0)) return rc;
+    }
     int done = 0;
     while (nsteps - done >= kChunk) {
         if (any_rs && done)
@@ -488,27 +541,22 @@ int lbgpu_batch_step(lbgpu_batch *b, int nsteps)
         if (!b->graph[b->aa_phase])
             if (int rc = capture_chunk(b)) return rc;
         if (int rc = batch_error(cudaGraphLaunch(b->graph[b->aa_phase], b->stream), "graph launch")) return rc;
-        b->launches += kChunk * launches_per_step(b);
+        b->launches += b->chunk_launches;
         done += kChunk;
     }
     const int rem = nsteps - done;
     if (any_rs && done && rem)
         if (int rc = refresh_collision_numbers(b, done)) return rc;
-    for (int k = 0; k < rem; ++k) launch_step(b, k);
+    for (int u = 0; u < rem / 2; ++u) launch_unit(b, u);
     if (int rc = lbgpu::cuda_error(cudaGetLastError(), "batch step")) return rc;
     for (lbgpu_lattice *m : b->members)
-        if (m) advance(m->L, nsteps);
+        if (m) advance(m->L, nsteps, true);
     if (int rc = order_after(b)) return rc;
-    if ((rem & 1) || any_rs) {
-        // parities changed (or stochastically rounded members count collisions): new
-        // descriptors before the next call (a chunk's graph reads them); on odd remainders the
-        // AA lists swap their kind of step
-        if (rem & 1) b->aa_phase ^= 1;
-        for (size_t i = 0; i < b->members.size(); ++i)
-            if (b->members[i]) b->h_inst[i] = describe(b->members[i]->L);
-        if (int rc = batch_error(cudaMemcpyAsync(b->d_inst, b->h_inst.data(), b->h_inst.size() * sizeof(BatchInst),
-                                                 cudaMemcpyHostToDevice, b->stream), "update batch members"))
-            return rc;
+    if ((rem & 3) || any_rs) {
+        // two-step launches in an odd number turned buffers and side store over (or stochastically
+        // rounded members count collisions): new descriptors before the next call, whose graphs read
+        // them
+        if (int rc = refresh_collision_numbers(b, 0)) return rc;
         if (int rc = batch_error(cudaStreamSynchronize(b->stream), "update batch members")) return rc;
     }
     return LB_OK;

@@ -43,9 +43,9 @@ void launch_stream(const DevLattice &d, int src, int side_par, cudaStream_t s);
 // extrapolated before every step.
 int tile_steps(const DevLattice &d, long long steps, bool outlet);
 // T pull steps (a count that tile_steps returned) in one launch: C_n in buffer src (n_par = n & 1)
-// -> C_{n+T} in buffer 1 - src, where T single steps would have left it in src: ghost_flip changes,
-// and the side store's slots change roles.  keys: rounding keys of the T collisions (16-bit).
-void launch_tile(DevLattice &d, int src, int n_par, int T, bool outlet, const unsigned *keys, cudaStream_t s);
+// -> C_{n+T} in buffer 1 - src, where T single steps would have left it in src: the caller turns
+// ghost_flip over and changes the side store's slots' roles (Lattice::after_tile).  keys: rounding keys of the T collisions (16-bit).
+void launch_tile(const DevLattice &d, int src, int n_par, int T, bool outlet, const unsigned *keys, cudaStream_t s);
 void launch_side_from_buf(const DevLattice &d, int b, int side_par, cudaStream_t s);
 // AA only: keep buffer b's ghost ring as the second buffer's (d.ghost2).
 void launch_ghost_copy(const DevLattice &d, int b, cudaStream_t s);
@@ -98,6 +98,7 @@ struct BatchInst {
     const double *bc;
     double omega;
     float scale, inv_scale;
+    int rules_inside;
     int scheme, cur0, phase0, tau0;   // tau0 + k: the collision number of step k of a chunk
     unsigned rs_seed;                 // 16-bit members: stochastic rounding seed (rs != 0)
     int rs;
@@ -121,6 +122,11 @@ __host__ __device__ inline int batch_sp(int shape, int passes) { return shape | 
 // row-shifted offsets; the kernels then carry those paths.
 void launch_batch(int precision, int kind, int threads, bool persistent, int flags, const BatchInst *insts,
                   const BatchWork *work, int nwork, int grid, int k, cudaStream_t s);
+// The batch's tile kernel (tile.cu): nodes of a tile, false where the storage type has none; and two
+// steps (BATCH_TILE_STEPS) of every tile of a work list, launch `unit` since the descriptors.
+constexpr int BATCH_TILE_STEPS = 2;
+bool batch_tile(int precision, int *w, int *h);
+void launch_batch_tile(int precision, const BatchInst *insts, const BatchWork *work, int nwork, int unit, cudaStream_t s);
 // Resident blocks per SM of the persistent kernel of a kind and block size.
 int batch_blocks_per_sm(int precision, int kind, int threads);
 

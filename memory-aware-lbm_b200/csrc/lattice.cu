@@ -267,8 +267,7 @@ int Lattice::step(int nsteps)
                 unsigned keys[8] = {0};
                 for (int k = 0; rs && k < T; ++k) keys[k] = rs_key(rs_seed, (unsigned long long)(n + 1 + k));
                 launch_tile(d, cur, (int)(n & 1), T, zgb_each_step, keys, stream);
-                cur = 1 - cur;
-                n += T;
+                after_tile(T);
                 s += T - 1;
                 ++launches;
                 LB_TRY(check("tile steps"));
@@ -284,6 +283,15 @@ int Lattice::step(int nsteps)
         }
     }
     return LB_OK;
+}
+
+void Lattice::after_tile(int T)
+{
+    const int a = (int)((n + 1) & 1);
+    d.side_slot[a] = 3 - d.side_slot[0] - d.side_slot[1];
+    d.ghost_flip ^= 1;
+    cur = 1 - cur;
+    n += T;
 }
 
 long long Lattice::steps_done() const

@@ -86,6 +86,8 @@ struct Lattice {
     unsigned rs_seed = 0;
     // the keys of collision k (and k + 1, two-step sweep) into d.g before a collision launch
     void set_rs_keys(long long k);
+    // the host's side of a tile launch of T steps: slots and rings change roles (kernels.h launch_tile)
+    void after_tile(int T);
     long long vel_samples = 0;
     int check(const char *what);   // cudaGetLastError -> error code
     int side_par_stale() const { return (int)((n + 1) & 1); }

@@ -30,6 +30,10 @@ using F32Small = TileShape<float, 16, 8, 8, 768, 1>;
 using F32Mid = TileShape<float, 32, 8, 4, 288, 3>;
 using F32Wide = TileShape<float, 32, 16, 4, 448, 2>;
 using F32Large = TileShape<float, 64, 12, 2, 224, 5>;
+// Batches advance every member by the same steps, two at a time, and fill the GPU: the large lattices' tiles,
+// with FP64's in halves because members are small (71 against 72 GLUPS on one large lattice).
+using F64Batch = TileShape<double, 32, 16, 2, 256, 4>;
+using F32Batch = F32Large;
 template <class S> using HalfSmall = TileShape<S, 16, 8, 8, 384, 2>;
 template <class S> using HalfWide = TileShape<S, 32, 16, 4, 416, 3>;
 
@@ -71,6 +75,9 @@ void launch_shape(const DevLattice &d, int src, int n_par, int pf, const unsigne
     a.x_first = EXTRAP && d.g.lx > SH::W && (d.g.lx % SH::W == 1 || d.g.lx % SH::W == 2) ? -3 : 1;
     a.nx = (int)cdiv(d.g.lx - a.x_first + 1, SH::W);
     a.ny = (int)cdiv(d.g.ly, SH::H);
+    // a long launch loses more to the ring's rows read out of order than its tail costs (FP32 16384 x 4096 414 us a
+    // step row by row, 433 ring first; 4096 x 1024 35.5 and 34.0, 1024 x 256 4.8 and 3.6; FP64 is faster ring first throughout)
+    a.ring_first = sizeof(S) == 8 || (long long)a.nx * a.ny < 12000;
     a.pf = a.x_first == 1 ? pf : 0;
     a.rules_inside = d.rules_inside;
     for (int k = 0; k < 8; ++k) a.keys[k] = keys[k];
@@ -115,7 +122,7 @@ int tile_steps(const DevLattice &d, long long steps, bool outlet)
     return 2;
 }
 
-void launch_tile(DevLattice &d, int src, int n_par, int T, bool outlet, const unsigned *keys, cudaStream_t s)
+void launch_tile(const DevLattice &d, int src, int n_par, int T, bool outlet, const unsigned *keys, cudaStream_t s)
 {
     const int shape = tile_shape(d);
     switch (d.precision) {
@@ -134,9 +141,24 @@ void launch_tile(DevLattice &d, int src, int n_par, int T, bool outlet, const un
     case LBGPU_F16: launch_half<__half>(d, src, n_par, T, outlet, keys, s); break;
     default: launch_half<__nv_bfloat16>(d, src, n_par, T, outlet, keys, s); break;
     }
-    const int a = (n_par + 1) & 1;
-    d.side_slot[a] = 3 - d.side_slot[0] - d.side_slot[1];
-    d.ghost_flip ^= 1;
+}
+
+bool batch_tile(int precision, int *w, int *h)
+{
+    if (precision == LBGPU_F64) { *w = F64Batch::W; *h = F64Batch::H; return true; }
+    if (precision == LBGPU_F32) { *w = F32Batch::W; *h = F32Batch::H; return true; }
+    return false;
+}
+
+void launch_batch_tile(int precision, const BatchInst *insts, const BatchWork *work, int nwork, int unit, cudaStream_t s)
+{
+    if (precision == LBGPU_F64) {
+        cudaFuncSetAttribute(k_batch_tile<F64Batch, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F64Batch::SMEM);
+        k_batch_tile<F64Batch, false><<<nwork, F64Batch::NT, F64Batch::SMEM, s>>>(insts, work, unit);
+    } else {
+        cudaFuncSetAttribute(k_batch_tile<F32Batch, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F32Batch::SMEM);
+        k_batch_tile<F32Batch, false><<<nwork, F32Batch::NT, F32Batch::SMEM, s>>>(insts, work, unit);
+    }
 }
 
 }  // namespace lbgpu

@@ -52,16 +52,17 @@ struct TileArgs {
     float sc, inv, omega_f;
     int x_first;               // column of the first tile (1, or less, see launch_tile)
     int nx, ny;                // tiles
+    int ring_first;            // their order (tile_place)
     int pf;                    // tiles ahead whose nodes are prefetched into L2
     int rules_inside;          // some node off the perimeter has a boundary rule
     unsigned keys[8];          // stochastic rounding keys of the steps
 };
 
-// Block b's tile: the outer ring of tiles first (their boundary rules make them the longest, and a
-// launch ends with its last block), then the others row by row.
-__device__ __forceinline__ void tile_place(unsigned b, int nx, int ny, int &tx, int &ty)
+// Block b's tile: row by row, or the outer ring of tiles first (their boundary rules make them the longest, and
+// a launch ends with its last block) and then the others row by row.
+__device__ __forceinline__ void tile_place(unsigned b, int nx, int ny, int ring_first, int &tx, int &ty)
 {
-    if (nx < 3 || ny < 3) {
+    if (!ring_first || nx < 3 || ny < 3) {
         ty = (int)(b / (unsigned)nx);
         tx = (int)(b - (unsigned)ty * (unsigned)nx);
         return;
@@ -411,27 +412,16 @@ __device__ __forceinline__ void tile_steps(const TileArgs<S> &a, S *sm, uint8_t 
     }
 }
 
+// The T steps of the tile at (x0, y0) by one block.
 template <class SH, bool RS, bool EXTRAP>
-__global__ void __launch_bounds__(SH::NT, SH::MINB) k_tile(const __grid_constant__ TileArgs<typename SH::S> a)
+__device__ __forceinline__ void tile_block(const TileArgs<typename SH::S> &a, unsigned char *smem, int x0, int y0)
 {
     using S = typename SH::S;
-    extern __shared__ __align__(16) unsigned char tile_smem[];
-    S *sm = reinterpret_cast<S *>(tile_smem);
-    uint8_t *stag = tile_smem + SH::POPS;
+    S *sm = reinterpret_cast<S *>(smem);
+    uint8_t *stag = smem + SH::POPS;
     unsigned short *list = reinterpret_cast<unsigned short *>(stag + SH::TAGS);
-    int *nlist = reinterpret_cast<int *>(tile_smem + SH::SMEM - 16);
-    int tx, ty;
-    tile_place(blockIdx.x, a.nx, a.ny, tx, ty);
-    const int x0 = a.x_first + tx * SH::W, y0 = 1 + ty * SH::H;
+    int *nlist = reinterpret_cast<int *>(smem + SH::SMEM - 16);
     constexpr int E = SH::T - 1;
-    if (a.pf > 0 && threadIdx.x < 9 * SH::H && blockIdx.x + (unsigned)a.pf < gridDim.x) {
-        int px, py;
-        tile_place(blockIdx.x + (unsigned)a.pf, a.nx, a.ny, px, py);
-        const int Yp = 1 + py * SH::H + (int)threadIdx.x % SH::H, Xp = a.x_first + px * SH::W;
-        if (Yp <= a.g.ly && Xp >= 1 && Xp + SH::W - 1 <= a.g.lx)
-            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(plane(a.src, a.g, (int)threadIdx.x / SH::H) + a.g.idx(Xp, Yp)),
-                         "n"(SH::W * (int)sizeof(S)) : "memory");
-    }
     const bool inside = !a.rules_inside && x0 - E >= 2 && x0 + SH::W - 1 + E <= a.g.lx - 1 && y0 - E >= 2 && y0 + SH::H - 1 + E <= a.g.ly - 1;
     if (inside) {
         tile_steps<S, SH, 1, false, RS, EXTRAP>(a, sm, stag, list, nlist, x0, y0);
@@ -440,4 +430,59 @@ __global__ void __launch_bounds__(SH::NT, SH::MINB) k_tile(const __grid_constant
         __syncthreads();
         tile_steps<S, SH, 1, true, RS, EXTRAP>(a, sm, stag, list, nlist, x0, y0);
     }
+}
+
+template <class SH, bool RS, bool EXTRAP>
+__global__ void __launch_bounds__(SH::NT, SH::MINB) k_tile(const __grid_constant__ TileArgs<typename SH::S> a)
+{
+    extern __shared__ __align__(16) unsigned char tile_smem[];
+    if (a.pf > 0 && threadIdx.x < 9 * SH::H && blockIdx.x + (unsigned)a.pf < gridDim.x) {
+        int px, py;
+        tile_place(blockIdx.x + (unsigned)a.pf, a.nx, a.ny, a.ring_first, px, py);
+        const int Yp = 1 + py * SH::H + (int)threadIdx.x % SH::H, Xp = a.x_first + px * SH::W;
+        if (Yp <= a.g.ly && Xp >= 1 && Xp + SH::W - 1 <= a.g.lx)
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(plane(a.src, a.g, (int)threadIdx.x / SH::H) + a.g.idx(Xp, Yp)),
+                         "n"(SH::W * (int)sizeof(typename SH::S)) : "memory");
+    }
+    int tx, ty;
+    tile_place(blockIdx.x, a.nx, a.ny, a.ring_first, tx, ty);
+    tile_block<SH, RS, EXTRAP>(a, tile_smem, a.x_first + tx * SH::W, 1 + ty * SH::H);
+}
+
+// T steps of every tile of a batch's work list (x0, y0: the tile's first node): launch `unit` of a
+// chunk, so a member's state is where `unit` launches have taken it from its descriptor's.
+template <class SH, bool RS>
+__global__ void __launch_bounds__(SH::NT, SH::MINB) k_batch_tile(const BatchInst *__restrict__ insts,
+                                                                 const BatchWork *__restrict__ work, int unit)
+{
+    using S = typename SH::S;
+    extern __shared__ __align__(16) unsigned char tile_smem[];
+    const BatchWork it = work[blockIdx.x];
+    const BatchInst &d = insts[it.inst];
+    TileArgs<S> a;
+    a.g = d.g;
+    const int src = d.cur0 ^ (unit & 1), pa = d.tau0 & 1;      // T is even: step 1's parity is the descriptor's
+    a.src = static_cast<const S *>(d.buf[src]);
+    a.dst = static_cast<S *>(d.buf[src ^ 1]);
+    a.tag = d.tag;
+    a.bc = d.bc;
+    a.zgb = nullptr;
+    a.omega = d.omega;
+    a.omega_f = (float)d.omega;
+    const size_t slot = 9 * (size_t)d.g.nper;
+    const int now = d.side_slot[pa], spare = 3 - d.side_slot[0] - d.side_slot[1];
+    S *side = static_cast<S *>(d.side);
+    a.stale1 = side + slot * ((unit & 1) ? spare : now);
+    a.out_prev = side + slot * ((unit & 1) ? now : spare);
+    a.out_last = side + slot * d.side_slot[pa ^ 1];
+    a.sc = d.scale;
+    a.inv = d.inv_scale;
+    a.x_first = 1;
+    a.rules_inside = d.rules_inside;
+    if (RS) {
+#pragma unroll
+        for (int k = 0; k < SH::T; ++k)
+            a.keys[k] = d.rs ? rs_key(d.rs_seed, (unsigned long long)(d.tau0 + unit * SH::T + k)) : 0u;
+    }
+    tile_block<SH, RS, false>(a, tile_smem, it.x0, it.y0);
 }
