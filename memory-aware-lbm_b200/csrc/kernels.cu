@@ -19,6 +19,7 @@
 // prefetches into L2 the rows a block a few rows further down will read
 // (cp.async.bulk.prefetch.L2, distances measured per kernel).  Runs of pull steps advance several
 // steps a launch in shared memory instead (tile.cu).
+#include <algorithm>
 #include "kernels.h"
 #include "node.cuh"
 
@@ -867,21 +868,33 @@ __global__ void k_ghost_copy(Geo g, const S *__restrict__ buf, S *__restrict__ r
 
 // Current state of columns [X0, X1) (all rows) as FP64 node records of `rs` doubles:
 // populations in slots 0..8 and, when `dynp` is given, the host dynamics pointer bits in
-// slot 9 (the host Node layout).
+// slot 9 (the host Node layout).  A block takes 32 columns x 8 rows: its reads run along x, as the
+// planes do, and its writes along y, as the records do (576 bytes a column; the writes may go over
+// the link to pinned host memory).
 template <class S>
-__global__ void __launch_bounds__(BX) k_readout(Geo g, int view, const S *__restrict__ cur,
-                                                const S *__restrict__ other,
-                                                const S *__restrict__ side, int X0, int X1,
-                                                double *__restrict__ out, int rs,
-                                                const uint64_t *__restrict__ dynp, float inv)
+__global__ void __launch_bounds__(256) k_readout(Geo g, int view, const S *__restrict__ cur,
+                                                 const S *__restrict__ other,
+                                                 const S *__restrict__ side, int X0, int X1,
+                                                 double *__restrict__ out, int rs,
+                                                 const uint64_t *__restrict__ dynp, float inv)
 {
-    const int Y = blockIdx.x * BX + threadIdx.x;
-    const int X = X0 + blockIdx.y;
-    if (Y > g.ly + 1 || X >= X1) return;
-    const size_t r = ((size_t)(X - X0) * (g.ly + 2) + Y) * rs;
+    __shared__ double rec[32][8 * 10 + 1];
+    const int Xb = X0 + blockIdx.x * 32, Yb = blockIdx.y * 8;
+    {
+        const int c = threadIdx.x & 31, r = threadIdx.x >> 5, X = Xb + c, Y = Yb + r;
+        if (X < X1 && Y <= g.ly + 1) {
 #pragma unroll
-    for (int i = 0; i < 9; ++i) out[r + i] = (double)logical(g, view, cur, other, side, X, Y, i, inv);
-    if (dynp) out[r + 9] = __longlong_as_double((long long)dynp[(size_t)X * (g.ly + 2) + Y]);
+            for (int i = 0; i < 9; ++i) rec[c][r * rs + i] = (double)logical(g, view, cur, other, side, X, Y, i, inv);
+            if (rs > 9) rec[c][r * rs + 9] = dynp ? __longlong_as_double((long long)dynp[(size_t)X * (g.ly + 2) + Y]) : 0.0;
+        }
+    }
+    __syncthreads();
+    const int rows = min(8, g.ly + 2 - Yb), run = rows * rs;
+    for (int k = threadIdx.x; k < 32 * run; k += 256) {
+        const int c = k / run, e = k - c * run;
+        if (Xb + c < X1 && (rs == 9 || dynp || e % rs != 9))
+            out[((size_t)(Xb + c - X0) * (g.ly + 2) + Yb) * rs + e] = rec[c][e];
+    }
 }
 
 // FP64 node records of columns [X0, X1) into buffer b (inverse of k_readout).
@@ -1011,23 +1024,30 @@ __global__ void __launch_bounds__(BX) k_cylinder_tags(Geo g, uint8_t *__restrict
 template <class S>
 __global__ void __launch_bounds__(BX) k_macros(Geo g, int view, const S *__restrict__ cur,
                                                const S *__restrict__ other,
-                                               const S *__restrict__ side, double *__restrict__ rho,
+                                               const S *__restrict__ side, int Y0, double *__restrict__ rho,
                                                double *__restrict__ ux, double *__restrict__ uy,
                                                float inv)
 {
     using R = typename Codec<S>::R;
     const int X = blockIdx.x * BX + threadIdx.x + 1;
-    const int Y = blockIdx.y + 1;
+    const int Y = Y0 + blockIdx.y;
     if (X > g.lx) return;
     R f[9];
 #pragma unroll
     for (int i = 0; i < 9; ++i) f[i] = logical(g, view, cur, other, side, X, Y, i, inv);
     R r, u, v;
     rules::macros<R>(f, r, u, v);
-    const size_t k = (size_t)(Y - 1) * g.lx + (X - 1);
+    const size_t k = (size_t)(Y - Y0) * g.lx + (X - 1);
     if (rho) rho[k] = (double)r;
     if (ux) ux[k] = (double)u;
     if (uy) uy[k] = (double)v;
+}
+
+__global__ void __launch_bounds__(256) k_scaled(const double *__restrict__ in, double scale, double *__restrict__ out,
+                                                long long n)
+{
+    for (long long k = (long long)blockIdx.x * 256 + threadIdx.x; k < n; k += (long long)gridDim.x * 256)
+        out[k] = __dmul_rn(in[k], scale);
 }
 
 // ---- FP64 reductions of the current state ----------------------------------------------
@@ -1409,8 +1429,8 @@ void launch_readout(const DevLattice &d, int view, int cur, int side_par, int X0
                     double *out, int rec_stride, const uint64_t *dynp, cudaStream_t s)
 {
     if (X1 <= X0) return;
-    dim3 grid(cdiv(d.g.ly + 2, BX), X1 - X0);
-    LBGPU_DISPATCH(d, (k_readout<S><<<grid, BX, 0, s>>>(d.g, view, B<S>(d, cur), OTHER<S>(d, cur),
+    dim3 grid(cdiv(X1 - X0, 32), cdiv(d.g.ly + 2, 8));
+    LBGPU_DISPATCH(d, (k_readout<S><<<grid, 256, 0, s>>>(d.g, view, B<S>(d, cur), OTHER<S>(d, cur),
                        SIDE<S>(d, side_par), X0, X1, out, rec_stride, dynp, d.inv_scale)));
 }
 
@@ -1505,12 +1525,17 @@ void launch_accumulate_velocity(const DevLattice &d, int view, int cur, int side
                        OTHER<S>(d, cur), SIDE<S>(d, side_par), acc, d.inv_scale)));
 }
 
-void launch_macros(const DevLattice &d, int view, int cur, int side_par, double *rho, double *ux,
+void launch_macros(const DevLattice &d, int view, int cur, int side_par, int Y0, int Y1, double *rho, double *ux,
                    double *uy, cudaStream_t s)
 {
-    dim3 grid(cdiv(d.g.lx, BX), d.g.ly);
+    dim3 grid(cdiv(d.g.lx, BX), Y1 - Y0);
     LBGPU_DISPATCH(d, (k_macros<S><<<grid, BX, 0, s>>>(d.g, view, B<S>(d, cur), OTHER<S>(d, cur),
-                       SIDE<S>(d, side_par), rho, ux, uy, d.inv_scale)));
+                       SIDE<S>(d, side_par), Y0, rho, ux, uy, d.inv_scale)));
+}
+
+void launch_scaled(const double *in, double scale, double *out, long long n, cudaStream_t s)
+{
+    k_scaled<<<std::min<unsigned>(cdiv(n, 256), 148 * 8), 256, 0, s>>>(in, scale, out, n);
 }
 
 }  // namespace lbgpu

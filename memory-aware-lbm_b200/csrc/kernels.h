@@ -64,8 +64,11 @@ void launch_periodic(const DevLattice &d, int b, cudaStream_t s);
 // pressure-regularized outlet) written on the device.
 void launch_cylinder_tags(const DevLattice &d, int ox, int oy, int r, int wall_kind, cudaStream_t s);
 void launch_init_cylinder(const DevLattice &d, int b, double umax, cudaStream_t s);
-void launch_macros(const DevLattice &d, int view, int cur, int side_par, double *rho, double *ux,
+// Density and velocity of rows Y0..Y1-1 ([Y - Y0][X - 1]; any pointer may be null).
+void launch_macros(const DevLattice &d, int view, int cur, int side_par, int Y0, int Y1, double *rho, double *ux,
                    double *uy, cudaStream_t s);
+// out[k] = in[k] * scale
+void launch_scaled(const double *in, double scale, double *out, long long n, cudaStream_t s);
 // FP64 reductions of the current state (mass, momentum, obstacle force, kinetic energy,
 // non-finite nodes, fluid mass) into out[8]; `partial` is scratch of (ly+2)*8 doubles.
 void launch_moments(const DevLattice &d, int view, int cur, int side_par, double *partial,

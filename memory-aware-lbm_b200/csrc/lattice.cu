@@ -2,9 +2,11 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include "codec.cuh"
 #include "lattice.h"
+#include "readback.h"
 #include "lbgpu.h"
 
 namespace lbgpu {
@@ -40,6 +42,56 @@ int cuda_error(cudaError_t e, const char *what)
 int last_error() { return g_err; }
 const char *last_error_string() { return g_msg; }
 void clear_error() { g_err = 0; g_msg[0] = 0; }
+
+// ---- device memory ---------------------------------------------------------------------
+namespace {
+constexpr int kPools = 64;
+std::mutex g_mem_mu;
+cudaMemPool_t g_pool[kPools] = {};
+int g_lattices = 0;
+}  // namespace
+
+cudaError_t device_alloc(void **p, size_t bytes, int device, cudaStream_t s)
+{
+    *p = nullptr;
+    if (bytes > kPoolBytes) return cudaMalloc(p, bytes);
+    if (device < 0 || device >= kPools) return cudaErrorInvalidDevice;
+    cudaMemPool_t pool;
+    {
+        std::lock_guard<std::mutex> lock(g_mem_mu);
+        if (!g_pool[device]) {
+            cudaMemPoolProps props = {};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = device;
+            if (cudaError_t e = cudaMemPoolCreate(&g_pool[device], &props)) return e;
+            unsigned long long keep = 256ull << 20;
+            cudaMemPoolSetAttribute(g_pool[device], cudaMemPoolAttrReleaseThreshold, &keep);
+        }
+        pool = g_pool[device];
+    }
+    return cudaMallocFromPoolAsync(p, bytes, pool, s);
+}
+
+cudaError_t device_free(void *p, size_t bytes, cudaStream_t s)
+{
+    return bytes > kPoolBytes ? cudaFree(p) : cudaFreeAsync(p, s);
+}
+
+void memory_hold()
+{
+    std::lock_guard<std::mutex> lock(g_mem_mu);
+    ++g_lattices;
+}
+
+void memory_drop()
+{
+    std::lock_guard<std::mutex> lock(g_mem_mu);
+    if (--g_lattices > 0) return;
+    for (cudaMemPool_t pool : g_pool)
+        if (pool) cudaMemPoolTrimTo(pool, 0);
+    read_back_release();
+}
 
 #define LB_TRY(expr)                                \
     do {                                            \
@@ -81,41 +133,37 @@ int Lattice::create(int lx_, int ly_, int precision_, int scheme_)
     LB_CUDA(cudaGetDevice(&device), "cudaGetDevice");
     LB_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate");
 
+    // One allocation for everything, its parts on 256-byte boundaries; all zero but the slots without
+    // an extrapolated row.
     const size_t nbuf = (scheme == LBGPU_AA) ? 1 : 2;
     const size_t pbytes = 9 * (size_t)d.g.plane * elem;
     // two parities, and for the pull scheme the slot the tile kernel writes beside them
     const size_t sbytes = (scheme == LBGPU_PULL ? 3 : 2) * 9 * (size_t)d.g.nper * elem;
-    void *p = nullptr;
-    for (size_t b = 0; b < nbuf; ++b) {
-        LB_CUDA(cudaMalloc(&p, pbytes), "cudaMalloc(populations)");
-        d.buf[b] = p;
-        LB_CUDA(cudaMemsetAsync(p, 0, pbytes, stream), "cudaMemset(populations)");
+    const size_t gbytes = scheme == LBGPU_AA ? 9 * (size_t)d.g.nghost() * elem : 0;
+    const size_t part[8] = {pbytes, nbuf == 2 ? pbytes : 0, gbytes, sbytes, (size_t)d.g.plane,
+                            16 * (size_t)d.g.nb * sizeof(double), 2 * (size_t)(ly + 2) * sizeof(double),
+                            4 * (size_t)d.g.nb * sizeof(int)};
+    size_t at[9] = {0};
+    for (int k = 0; k < 8; ++k) {
+        at[k + 1] = at[k] + (part[k] + 255) / 256 * 256;
+        bytes += part[k];
     }
-    if (scheme == LBGPU_AA) {
-        const size_t gbytes = 9 * (size_t)d.g.nghost() * elem;
-        LB_CUDA(cudaMalloc(&p, gbytes), "cudaMalloc(ghost ring)");
-        d.ghost2 = p;
-        LB_CUDA(cudaMemsetAsync(p, 0, gbytes, stream), "cudaMemset(ghost ring)");
-        bytes += gbytes;
-    }
-    LB_CUDA(cudaMalloc(&p, sbytes), "cudaMalloc(side store)");
-    d.side = p;
+    memory_hold();
+    held = true;
+    memory_bytes = at[8];
+    LB_CUDA(device_alloc(&memory, memory_bytes, device, stream), "device memory (lattice)");
+    char *m = static_cast<char *>(memory);
+    LB_CUDA(cudaMemsetAsync(m, 0, at[7], stream), "cudaMemset(lattice)");
+    LB_CUDA(cudaMemsetAsync(m + at[7], 0xff, part[7], stream), "cudaMemset(zgb slots)");
+    d.buf[0] = m + at[0];
+    d.buf[1] = nbuf == 2 ? m + at[1] : nullptr;
+    d.ghost2 = gbytes ? m + at[2] : nullptr;
+    d.side = m + at[3];
+    d.tag = reinterpret_cast<const uint8_t *>(m + at[4]);
+    d.bc = reinterpret_cast<double *>(m + at[5]);
+    d.zrho = reinterpret_cast<double *>(m + at[6]);
+    d.zgb_src = reinterpret_cast<const int *>(m + at[7]);
     reset_roles();
-    LB_CUDA(cudaMemsetAsync(p, 0, sbytes, stream), "cudaMemset(side store)");
-    LB_CUDA(cudaMalloc(&p, (size_t)d.g.plane), "cudaMalloc(tags)");
-    d.tag = static_cast<const uint8_t *>(p);
-    LB_CUDA(cudaMemsetAsync(p, 0, (size_t)d.g.plane, stream), "cudaMemset(tags)");
-    LB_CUDA(cudaMalloc(&p, 16 * (size_t)d.g.nb * sizeof(double)), "cudaMalloc(tables)");
-    d.bc = static_cast<double *>(p);
-    LB_CUDA(cudaMemsetAsync(p, 0, 16 * (size_t)d.g.nb * sizeof(double), stream), "cudaMemset");
-    LB_CUDA(cudaMalloc(&p, 4 * (size_t)d.g.nb * sizeof(int)), "cudaMalloc(zgb slots)");
-    d.zgb_src = static_cast<const int *>(p);
-    LB_CUDA(cudaMemsetAsync(p, 0xff, 4 * (size_t)d.g.nb * sizeof(int), stream), "cudaMemset");
-    LB_CUDA(cudaMalloc(&p, 2 * (size_t)(ly + 2) * sizeof(double)), "cudaMalloc(zgb rho)");
-    d.zrho = static_cast<double *>(p);
-    LB_CUDA(cudaMemsetAsync(p, 0, 2 * (size_t)(ly + 2) * sizeof(double), stream), "cudaMemset");
-    bytes += nbuf * pbytes + sbytes + (size_t)d.g.plane + 16 * (size_t)d.g.nb * 8 +
-            4 * (size_t)d.g.nb * 4 + 2 * (size_t)(ly + 2) * 8;
     bc_host.assign(16 * (size_t)d.g.nb, 0.0);
     zgb_src_host.assign(4 * (size_t)d.g.nb, -1);
     cur = 0; form = FORM_L; pending = 0; n = 0;
@@ -133,19 +181,19 @@ void Lattice::reset_roles()
 void Lattice::destroy()
 {
     if (stream) cudaStreamSynchronize(stream);
-    for (int b = 0; b < 2; ++b) if (d.buf[b]) cudaFree(d.buf[b]);
-    if (d.side) cudaFree(d.side);
-    if (d.ghost2) cudaFree(d.ghost2);
-    if (d.tag) cudaFree(const_cast<uint8_t *>(d.tag));
-    if (d.bc) cudaFree(d.bc);
-    if (d.zgb_src) cudaFree(const_cast<int *>(d.zgb_src));
-    if (d.zrho) cudaFree(d.zrho);
+    if (memory) device_free(memory, memory_bytes, stream);
+    memory = nullptr;
     if (stage) cudaFree(stage);
     if (red_scratch) cudaFree(red_scratch);
     if (vel_acc) cudaFree(vel_acc);
     if (shift) cudaFree(shift);
     red_scratch = nullptr; vel_acc = nullptr; vel_samples = 0; shift = nullptr;
-    if (stream) cudaStreamDestroy(stream);
+    if (stream) {
+        cudaStreamSynchronize(stream);    // the memory is the pool's again
+        cudaStreamDestroy(stream);
+    }
+    if (held) memory_drop();
+    held = false;
     d = DevLattice{};
     stage = nullptr; stage_bytes = 0; stream = nullptr;
 }
@@ -390,6 +438,23 @@ int Lattice::readout_records(double *host, int rs, const uint64_t *dynp_dev, int
     return check("readout");
 }
 
+int Lattice::readout_populations(double *host)
+{
+    int v, par;
+    view(v, par);
+    const size_t col = (size_t)(ly + 2) * 9;
+    const cudaError_t e = read_back(
+        device, stream, lx + 2, col * sizeof(double),
+        [&](long long x0, long long x1, double *dst) {
+            launch_readout(d, v, cur, par, (int)x0, (int)x1, dst, 9, nullptr, stream);
+        },
+        [&](long long x0, long long x1, const double *src) {
+            std::memcpy(host + (size_t)x0 * col, src, (size_t)(x1 - x0) * col * sizeof(double));
+        });
+    d2h_bytes += (size_t)(lx + 2) * col * sizeof(double);
+    return cuda_error(e, "readout");
+}
+
 int Lattice::init_side_from(int b, int par)
 {
     launch_side_from_buf(d, b, par, stream);
@@ -406,20 +471,29 @@ int Lattice::init_cylinder(double umax)
 
 int Lattice::get_macros(double *rho, double *ux, double *uy)
 {
-    const size_t nn = (size_t)lx * ly;
-    double *dev = nullptr;
-    LB_CUDA(cudaMalloc(&dev, 3 * nn * sizeof(double)), "cudaMalloc(macros)");
     int v, par;
     view(v, par);
-    launch_macros(d, v, cur, par, dev, dev + nn, dev + 2 * nn, stream);
-    int rc = check("macros");
-    if (rc == LB_OK && rho) rc = cuda_error(cudaMemcpyAsync(rho, dev, nn * 8, cudaMemcpyDeviceToHost, stream), "macros");
-    if (rc == LB_OK && ux) rc = cuda_error(cudaMemcpyAsync(ux, dev + nn, nn * 8, cudaMemcpyDeviceToHost, stream), "macros");
-    if (rc == LB_OK && uy) rc = cuda_error(cudaMemcpyAsync(uy, dev + 2 * nn, nn * 8, cudaMemcpyDeviceToHost, stream), "macros");
-    if (rc == LB_OK) rc = cuda_error(cudaStreamSynchronize(stream), "macros");
-    d2h_bytes += nn * 8 * ((rho != nullptr) + (ux != nullptr) + (uy != nullptr));
-    cudaFree(dev);
-    return rc;
+    double *const to[3] = {rho, ux, uy};
+    int n = 0;
+    double *field[3];
+    for (double *p : to)
+        if (p) field[n++] = p;
+    // one item a row: its values of each field wanted, one field after the other in a chunk
+    const cudaError_t e = read_back(
+        device, stream, n ? ly : 0, (size_t)n * lx * sizeof(double),
+        [&](long long y0, long long y1, double *dst) {
+            const size_t m = (size_t)(y1 - y0) * lx;
+            double *at[3];
+            int k = 0;
+            for (int j = 0; j < 3; ++j) at[j] = to[j] ? dst + m * k++ : nullptr;
+            launch_macros(d, v, cur, par, (int)y0 + 1, (int)y1 + 1, at[0], at[1], at[2], stream);
+        },
+        [&](long long y0, long long y1, const double *src) {
+            const size_t m = (size_t)(y1 - y0) * lx;
+            for (int k = 0; k < n; ++k) std::memcpy(field[k] + (size_t)y0 * lx, src + m * k, m * sizeof(double));
+        });
+    d2h_bytes += (size_t)n * lx * ly * sizeof(double);
+    return cuda_error(e, "macros");
 }
 
 int Lattice::moments(double out[8])
@@ -462,14 +536,20 @@ int Lattice::velocity_average(double *ux, double *uy, long long *samples)
     const size_t nn = (size_t)lx * ly;
     if (samples) *samples = vel_samples;
     if (!vel_acc || vel_samples == 0) return set_error(LB_ERR_STATE, "no velocity samples accumulated");
-    if (ux) LB_CUDA(cudaMemcpyAsync(ux, vel_acc, nn * 8, cudaMemcpyDeviceToHost, stream), "velocity average");
-    if (uy) LB_CUDA(cudaMemcpyAsync(uy, vel_acc + nn, nn * 8, cudaMemcpyDeviceToHost, stream), "velocity average");
-    LB_CUDA(cudaStreamSynchronize(stream), "velocity average");
-    d2h_bytes += nn * 8 * ((ux != nullptr) + (uy != nullptr));
     const double k = 1.0 / (double)vel_samples;
-    for (size_t i = 0; i < nn; ++i) {
-        if (ux) ux[i] *= k;
-        if (uy) uy[i] *= k;
+    double *const to[2] = {ux, uy};
+    for (int j = 0; j < 2; ++j) {
+        if (!to[j]) continue;
+        const cudaError_t e = read_back(
+            device, stream, ly, (size_t)lx * sizeof(double),
+            [&](long long y0, long long y1, double *dst) {
+                launch_scaled(vel_acc + (size_t)j * nn + (size_t)y0 * lx, k, dst, (y1 - y0) * lx, stream);
+            },
+            [&](long long y0, long long y1, const double *src) {
+                std::memcpy(to[j] + (size_t)y0 * lx, src, (size_t)(y1 - y0) * lx * sizeof(double));
+            });
+        LB_CUDA(e, "velocity average");
+        d2h_bytes += nn * 8;
     }
     return LB_OK;
 }

@@ -311,7 +311,7 @@ int lbgpu_get_populations(lbgpu_lattice *h, double *f)
 {
     if (int rc = bad_handle(h, "lbgpu_get_populations")) return rc;
     if (!f) return set_error(LB_ERR_ARG, "lbgpu_get_populations: null output");
-    return h->L.readout_records(f, 9, nullptr, 0, h->L.lx + 2);
+    return h->L.readout_populations(f);
 }
 
 int lbgpu_get_macros(lbgpu_lattice *h, double *rho, double *ux, double *uy)

@@ -85,7 +85,7 @@ extern "C" int lbgpu_get_macros_noalloc(lbgpu_lattice *h, double *rho, double *u
     if (rc == LB_OK) {
         int v, par;
         L.view(v, par);
-        lbgpu::launch_macros(L.d, v, L.cur, par, s, s + nodes, s + 2 * nodes, L.stream);
+        lbgpu::launch_macros(L.d, v, L.cur, par, 1, L.ly + 1, s, s + nodes, s + 2 * nodes, L.stream);
         rc = L.check("lbgpu_get_macros_noalloc");
     }
     double *dst[3] = {rho, ux, uy};

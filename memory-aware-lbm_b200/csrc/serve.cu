@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cstring>
+#include <memory>
 #include <thread>
 #include <vector>
 #include "lattice.h"
@@ -36,7 +37,7 @@ struct Req {
     float change = -1.0f;
     bool active = false, done = false;
     bool solo = false;           // stepped on its own stream instead of in the batch
-    std::vector<double> ux, uy;
+    std::unique_ptr<double[]> fields;   // ux, then uy (want_fields, once done)
 };
 
 // The velocity-change kernel reports a non-finite velocity as 3e38: such a request has
@@ -110,7 +111,9 @@ int start(lbgpu_server *s, Req &q, int id)
     if (int rc = lbgpu_setup_cylinder(q.lat, r.obst_x, r.obst_y, r.obst_r, r.umax, r.re,
                                       LBGPU_WALL_BOUNCEBACK, LBGPU_OUTLET_CONST, nullptr))
         return rc;
-    if (int rc = serr(cudaMalloc(&q.prev, 8 * (size_t)r.lx * r.ly), "cudaMalloc(velocity snapshot)")) return rc;
+    if (int rc = serr(lbgpu::device_alloc(&q.prev, 8 * (size_t)r.lx * r.ly, q.lat->L.device, q.lat->L.stream),
+                      "device memory (velocity snapshot)"))
+        return rc;
     // the snapshot starts as the initial velocity (the first check compares against it)
     lbgpu::Lattice &L = q.lat->L;
     int v, par;
@@ -124,7 +127,7 @@ int start(lbgpu_server *s, Req &q, int id)
 
 void release(Req &q)
 {
-    if (q.prev) cudaFree(q.prev);
+    if (q.prev) lbgpu::device_free(q.prev, 8 * (size_t)q.spec.lx * q.spec.ly, q.lat->L.stream);
     q.prev = nullptr;
     if (q.lat) lbgpu_destroy(q.lat);
     q.lat = nullptr;
@@ -260,9 +263,8 @@ int lbgpu_server_submit(lbgpu_server *s, const lbgpu_request *r, int *id)
                          r->lx, r->ly, r->max_steps, s->check_every);
     if (request_bytes(s, *r, scheme_of(s, *r)) > s->budget)
         return set_error(LB_ERR_CAPACITY, "lbgpu_server_submit: a %d x %d lattice exceeds the budget", r->lx, r->ly);
-    Req q;
-    q.spec = *r;
-    s->reqs.push_back(q);
+    s->reqs.emplace_back();
+    s->reqs.back().spec = *r;
     if (id) *id = (int)s->reqs.size() - 1;
     return LB_OK;
 }
@@ -353,9 +355,9 @@ int lbgpu_server_run(lbgpu_server *s, int batched)
             if (q.steps >= q.spec.max_steps || conv || diverged) {
                 q.converged = diverged ? -1 : (conv ? 1 : 0);
                 if (q.spec.want_fields) {
-                    q.ux.resize((size_t)q.spec.lx * q.spec.ly);
-                    q.uy.resize((size_t)q.spec.lx * q.spec.ly);
-                    if ((rc = lbgpu_get_macros(q.lat, nullptr, q.ux.data(), q.uy.data()))) break;
+                    const size_t nodes = (size_t)q.spec.lx * q.spec.ly;
+                    q.fields.reset(new double[2 * nodes]);   // not zeroed: every value is written
+                    if ((rc = lbgpu_get_macros(q.lat, nullptr, q.fields.get(), q.fields.get() + nodes))) break;
                 }
                 if (batched && !q.solo && (rc = lbgpu_batch_remove(batch, q.slot))) break;
                 q.finish = now_s(t0);
@@ -387,8 +389,9 @@ int lbgpu_server_result(lbgpu_server *s, int id, lbgpu_result *out, double *ux, 
     out->nodes = (long long)q.spec.lx * q.spec.ly;
     out->done = q.done ? 1 : 0;
     out->solo = q.solo ? 1 : 0;
-    if (ux && !q.ux.empty()) std::memcpy(ux, q.ux.data(), q.ux.size() * sizeof(double));
-    if (uy && !q.uy.empty()) std::memcpy(uy, q.uy.data(), q.uy.size() * sizeof(double));
+    const size_t nodes = (size_t)q.spec.lx * q.spec.ly;
+    if (ux && q.fields) std::memcpy(ux, q.fields.get(), nodes * sizeof(double));
+    if (uy && q.fields) std::memcpy(uy, q.fields.get() + nodes, nodes * sizeof(double));
     return LB_OK;
 }
 

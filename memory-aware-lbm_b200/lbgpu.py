@@ -271,16 +271,15 @@ class Lattice:
         _check(lib().lbgpu_synchronize(self.h))
 
     def populations(self):
-        out = np.zeros((self.lx + 2) * (self.ly + 2) * 9)
+        out = np.empty((self.lx + 2) * (self.ly + 2) * 9)
         _check(lib().lbgpu_get_populations(self.h, _p(out)))
         return out.reshape(self.lx + 2, self.ly + 2, 9)
 
     def macros(self):
-        n = self.lx * self.ly
-        rho, ux, uy = np.zeros(n), np.zeros(n), np.zeros(n)
+        # one uninitialised block: every value is written, and one large block takes its pages cheaper
+        rho, ux, uy = np.empty((3, self.ly, self.lx))
         _check(lib().lbgpu_get_macros(self.h, _p(rho), _p(ux), _p(uy)))
-        shp = (self.ly, self.lx)
-        return rho.reshape(shp), ux.reshape(shp), uy.reshape(shp)
+        return rho, ux, uy
 
     def macros_noalloc(self):
         """lbgpu_get_macros_noalloc: the same read-out through the library's fixed scratch."""
@@ -300,11 +299,10 @@ class Lattice:
         _check(lib().lbgpu_velocity_accumulate(self.h))
 
     def velocity_average(self):
-        n = self.lx * self.ly
-        ux, uy = np.zeros(n), np.zeros(n)
+        ux, uy = np.empty((2, self.ly, self.lx))
         k = ctypes.c_longlong()
         _check(lib().lbgpu_velocity_average(self.h, _p(ux), _p(uy), ctypes.byref(k)))
-        return ux.reshape(self.ly, self.lx), uy.reshape(self.ly, self.lx), k.value
+        return ux, uy, k.value
 
     def velocity_reset(self):
         _check(lib().lbgpu_velocity_reset(self.h))
@@ -615,13 +613,14 @@ class Server:
         r = self.requests[rid]
         ux = uy = None
         if fields:
-            ux = np.zeros((r.ly, r.lx))
-            uy = np.zeros((r.ly, r.lx))
+            ux, uy = (np.empty if r.want_fields else np.zeros)((2, r.ly, r.lx))
         _check(lib().lbgpu_server_result(self.h, int(rid), ctypes.byref(res),
                                          None if ux is None else _p(ux),
                                          None if uy is None else _p(uy)))
         out = {k: getattr(res, k) for k, _ in Result._fields_}
         if fields:
+            if r.want_fields and not out["done"]:    # nothing was written
+                ux[:], uy[:] = 0.0, 0.0
             out["ux"], out["uy"] = ux, uy
         return out
 
