@@ -51,6 +51,11 @@ struct DropIn {
     bool pops_dirty = false;
     bool dynp_dirty = true;
     bool bc_force = true;       // upload tables at the next refresh even if unchanged
+    // Pinned scratch of scratch_doubles(): the outlet columns of the state, those that the stream of the last
+    // collision gives (ahead: they are there and still hold), the outlet densities of a two-step call.
+    void *scratch_mem = nullptr;
+    double *scratch = nullptr;
+    bool ahead = false;
     bool tmp_is_stream = false; // tmpLattice holds the stream of lattice (collide_with_stream)
     int sync_mode = LB_SYNC_OUTLET;
     bool pinned[3] = {false, false, false};         // host arrays, then the dynamics pointers
@@ -190,19 +195,23 @@ int refresh_params(DropIn *c)
     // object (bitwise, as a memcmp would) and the tables go up only when one changed or a pass
     // forced it (a rescan, or device-side writes of the two-step outlet)
     if (c->bc_new.size() != L.bc_host.size()) c->bc_new = L.bc_host;
-    bool changed = c->bc_force;
+    size_t lo = c->bc_new.size(), hi = 0;
     double *bcn = c->bc_new.data();
     for (const DropIn::SlotRead &r : c->slot_reads)
         for (int j = 0; j < 2; ++j) {
             const double v = *r.src[j];
             if (std::memcmp(&bcn[r.off[j]], &v, sizeof(double)) != 0) {
                 bcn[r.off[j]] = v;
-                changed = true;
+                lo = std::min(lo, r.off[j]);
+                hi = std::max(hi, r.off[j] + 1);
             }
         }
-    if (changed) {
+    if (c->bc_force) {
         if (int rc = L.upload_bc(c->bc_new.data())) return rc;
         c->bc_force = false;
+    } else {
+        // an outlet that changes every step: its entries only, and nothing waits for them
+        if (int rc = L.upload_bc_range(c->bc_new.data(), lo, hi)) return rc;
     }
     return LB_OK;
 }
@@ -225,17 +234,29 @@ int upload_dynp(DropIn *c)
     return LB_OK;
 }
 
-void pin_host(Simulation *sim, DropIn *c)
+size_t scratch_cols(const Simulation *sim) { return 2 * (size_t)(sim->ly + 2) * 10; }   // two columns of records
+size_t scratch_doubles(const Simulation *sim) { return 2 * scratch_cols(sim) + 2 * (size_t)(sim->ly + 2); }
+
+bool pinning_allowed()
 {
     const char *e = getenv("LBGPU_PIN");
-    if (e && e[0] == '0') return;
+    return !(e && e[0] == '0');
+}
+
+// Pinning pays for arrays that are copied whole again and again or are large: registering 5 MB takes 7 ms and
+// unregistering 0.5, a pageable copy of them 0.4; at 64 MB it is 11 and 2 against 5.
+constexpr size_t kPinBytes = (size_t)64 << 20;
+
+void pin_host(Simulation *sim, DropIn *c)
+{
+    if (!pinning_allowed()) return;
     const size_t nodes = (size_t)(sim->lx + 2) * (sim->ly + 2);
     // the dynamics pointers too: the first read-out uploads them (the vector never reallocates)
     void *chunks[3] = {sim->memoryChunk, sim->tmpMemoryChunk, c->dynp.data()};
     const size_t bytes[3] = {nodes * sizeof(Node), nodes * sizeof(Node), c->dynp.size() * sizeof(uint64_t)};
     for (int k = 0; k < 3; ++k) {
         if (c->pinned[k] || !chunks[k] || !bytes[k]) continue;
-        if (cudaHostRegister(chunks[k], bytes[k], cudaHostRegisterPortable) == cudaSuccess) {
+        if (cudaHostRegister(chunks[k], bytes[k], cudaHostRegisterPortable | cudaHostRegisterMapped) == cudaSuccess) {
             c->pinned[k] = true;
             c->pinned_ptr[k] = chunks[k];
         } else {
@@ -255,13 +276,26 @@ int create_device(Simulation *sim, DropIn *c)
     }
     L.ghosts = true;
     c->created = true;
-    pin_host(sim, c);
+    if ((size_t)(sim->lx + 2) * (sim->ly + 2) * sizeof(Node) >= kPinBytes) pin_host(sim, c);
+    // (registered: 0.7 ms, where cudaHostAlloc takes 1.7)
+    const size_t bytes = (scratch_doubles(sim) * sizeof(double) + 4095) / 4096 * 4096;
+    if (pinning_allowed() && !c->scratch_mem) c->scratch_mem = aligned_alloc(4096, bytes);
+    if (c->scratch_mem && !c->scratch) {
+        void *dev = nullptr;
+        if (cudaHostRegister(c->scratch_mem, bytes, cudaHostRegisterPortable | cudaHostRegisterMapped) == cudaSuccess) {
+            if (cudaHostGetDevicePointer(&dev, c->scratch_mem, 0) == cudaSuccess && dev == c->scratch_mem)
+                c->scratch = static_cast<double *>(c->scratch_mem);
+            else
+                cudaHostUnregister(c->scratch_mem);
+        }
+        cudaGetLastError();   // without it the copies go through pageable memory
+    }
     return LB_OK;
 }
 
 // Bring the device copy up to date before an entry point runs (`tables`: the entry collides,
 // so omega and the boundary data objects are re-read; a pure stream never reads them).
-DropIn *prepare(Simulation *sim, const char *fn, bool tables = true)
+DropIn *prepare(Simulation *sim, const char *fn, bool tables = true, bool streams = false)
 {
     DropIn *c = ctx_of(sim);
     if (!c) {
@@ -269,6 +303,8 @@ DropIn *prepare(Simulation *sim, const char *fn, bool tables = true)
         return nullptr;
     }
     Lattice &L = c->L;
+    // the columns brought along hold for a stream of the state as the last call left it
+    if (!streams || c->tags_dirty || c->pops_dirty) c->ahead = false;
     if (!c->created && create_device(sim, c) != LB_OK) return nullptr;
     // The population uploads go first: they are asynchronous copies from the pinned host
     // arrays, so the host's scan of the dynamics pointers below runs while they transfer.
@@ -300,8 +336,22 @@ DropIn *prepare(Simulation *sim, const char *fn, bool tables = true)
     return c;
 }
 
-// Copy back what the sync mode asks for.
-void finish(Simulation *sim, DropIn *c)
+// The GPU's address of the pinned host array that sim->lattice points to, or null.
+double *mapped_lattice(Simulation *sim, DropIn *c)
+{
+    Node *host = chunk_of(sim->lattice);
+    for (int k = 0; k < 2; ++k)
+        if (c->pinned[k] && c->pinned_ptr[k] == host) {
+            void *dev = nullptr;
+            if (cudaHostGetDevicePointer(&dev, host, 0) == cudaSuccess) return static_cast<double *>(dev);
+            cudaGetLastError();
+        }
+    return nullptr;
+}
+
+// Copy back what the sync mode asks for.  collided: the state is a collision that the caller's next
+// call will stream.
+void finish(Simulation *sim, DropIn *c, bool collided = false)
 {
     Lattice &L = c->L;
     if (c->sync_mode == LB_SYNC_NONE) return;
@@ -309,12 +359,45 @@ void finish(Simulation *sim, DropIn *c)
     Node *host = chunk_of(sim->lattice);
     const size_t col = (size_t)(sim->ly + 2);
     if (c->sync_mode == LB_SYNC_FULL) {
+        pin_host(sim, c);
         L.readout_records(reinterpret_cast<double *>(host), 10, c->dynp_dev, 0, sim->lx + 2);
         return;
     }
-    // columns lx-2 and lx-1 are adjacent in the host's y-contiguous node array: one read-out
+    // columns lx-2 and lx-1 are adjacent in the host's y-contiguous node array: one read-out, written by the kernel
+    // itself into the array where it is pinned and into the pinned scratch where it is not (a copy
+    // command and its wait after the kernel took longer than the columns)
+    const int X0 = sim->lx >= 2 ? sim->lx - 2 : 0, X1 = sim->lx;
+    if (!c->scratch) {
+        L.readout_records(reinterpret_cast<double *>(host + (size_t)X0 * col), 10, c->dynp_dev, X0, X1);
+        return;
+    }
+    double *const dev = mapped_lattice(sim, c), *out = dev ? dev + (size_t)X0 * col * 10 : c->scratch;
+    if (collided && L.form == lbgpu::FORM_C && !L.pending) {
+        lbgpu::launch_readout_both(L.d, L.cur, (int)((L.n + 1) & 1), X0, X1, out, c->scratch + scratch_cols(sim), 10, c->dynp_dev, L.stream);
+        L.d2h_bytes += (size_t)(X1 - X0) * col * sizeof(Node);
+    } else {
+        int v, par;
+        L.view(v, par);
+        lbgpu::launch_readout(L.d, v, L.cur, par, X0, X1, out, 10, c->dynp_dev, L.stream);
+        collided = false;
+    }
+    ++L.launches;
+    L.d2h_bytes += (size_t)(X1 - X0) * col * sizeof(Node);
+    if (L.check("readout") || lbgpu::cuda_error(cudaStreamSynchronize(L.stream), "readout")) return;
+    if (!dev) std::memcpy(static_cast<void *>(host + (size_t)X0 * col), c->scratch, (size_t)(X1 - X0) * col * sizeof(Node));
+    c->ahead = collided;
+}
+
+// After a stream whose outlet columns the collision before it brought along.
+bool finish_ahead(Simulation *sim, DropIn *c)
+{
+    if (!c->ahead || c->sync_mode != LB_SYNC_OUTLET || c->dynp_dirty) return false;
+    const size_t col = (size_t)(sim->ly + 2);
     const int X0 = sim->lx >= 2 ? sim->lx - 2 : 0;
-    L.readout_records(reinterpret_cast<double *>(host + (size_t)X0 * col), 10, c->dynp_dev, X0, sim->lx);
+    std::memcpy(static_cast<void *>(chunk_of(sim->lattice) + (size_t)X0 * col), c->scratch + scratch_cols(sim),
+                (size_t)(sim->lx - X0) * col * sizeof(Node));
+    c->ahead = false;
+    return true;
 }
 
 void swap_host(Simulation *sim)
@@ -378,25 +461,40 @@ void two_steps(Simulation *sim, const char *fn, int need_x, int need_y)
         if (L.zgb_pass()) return;
     }
     if (L.op_collide() || L.op_propagate()) return;
-    c->bc_force = true;  // the tables now hold the extrapolated densities
-    if (sim->lx >= 2 && (pressureBoundary || myrho1 || myrho2)) {
-        std::vector<double> zr(2 * (size_t)(sim->ly + 2));
-        if (lbgpu::cuda_error(cudaMemcpyAsync(zr.data(), L.d.zrho, zr.size() * 8, cudaMemcpyDeviceToHost,
-                                              L.stream), fn) ||
-            lbgpu::cuda_error(cudaStreamSynchronize(L.stream), fn))
-            return;
-        L.d2h_bytes += zr.size() * 8;
-        for (int k = 1; k <= sim->ly - 1; ++k) {
-            if (myrho1) myrho1[k] = zr[2 * k];
-            if (myrho2 && sim->lx >= 3) myrho2[k] = zr[2 * k + 1];
-        }
-        if (pressureBoundary)
-            for (int Y = 2; Y <= sim->ly - 1; ++Y) {
-                pressureBoundary[Y].rho = 4. / 3. * zr[2 * Y] - 1. / 3. * zr[2 * Y + 1];
-                pressureBoundary[Y].uPar = 0.;
-            }
+    c->bc_force = true;  // the tables now hold the extrapolated densities (unless they are read back below)
+    const bool rows = sim->lx >= 2 && (pressureBoundary || myrho1 || myrho2);
+    std::vector<double> pageable;
+    double *zr = nullptr;
+    if (rows) {
+        const size_t n = 2 * (size_t)(sim->ly + 2);
+        if (!c->scratch) pageable.resize(n);
+        zr = c->scratch ? c->scratch + 2 * scratch_cols(sim) : pageable.data();
+        if (lbgpu::cuda_error(cudaMemcpyAsync(zr, L.d.zrho, n * 8, cudaMemcpyDeviceToHost, L.stream), fn)) return;
+        L.d2h_bytes += n * 8;
     }
     finish(sim, c);
+    if (!rows) return;
+    // (after finish, whose wait the densities' copy shares)
+    if (lbgpu::cuda_error(cudaStreamSynchronize(L.stream), fn)) return;
+    for (int k = 1; k <= sim->ly - 1; ++k) {
+        if (myrho1) myrho1[k] = zr[2 * k];
+        if (myrho2 && sim->lx >= 3) myrho2[k] = zr[2 * k + 1];
+    }
+    if (pressureBoundary)
+        for (int Y = 2; Y <= sim->ly - 1; ++Y) {
+            pressureBoundary[Y].rho = 4. / 3. * zr[2 * Y] - 1. / 3. * zr[2 * Y + 1];
+            pressureBoundary[Y].uPar = 0.;
+        }
+    // what the device wrote into its tables, so that the next call uploads only what the driver changes
+    const int nb = L.d.g.nb;
+    for (int k = 0; k < 4 * nb; ++k) {
+        const int src = L.zgb_src_host[k];
+        if (src < 0) continue;
+        const size_t at = (size_t)((4 + k / nb) * 2) * nb + k % nb;
+        c->bc_new[at] = 4. / 3. * zr[2 * src] - 1. / 3. * zr[2 * src + 1];
+        c->bc_new[at + nb] = 0.;
+    }
+    c->bc_force = false;
 }
 
 }  // namespace
@@ -454,8 +552,10 @@ void destructSim(Simulation *sim)
     if (c) {
         if (c->created) {
             if (c->dynp_dev) cudaFree(c->dynp_dev);
+            if (c->scratch) cudaHostUnregister(c->scratch_mem);
             c->L.destroy();
         }
+        free(c->scratch_mem);
         for (int k = 0; k < 3; ++k)   // before the dynamics-pointer vector goes with c
             if (c->pinned[k]) cudaHostUnregister(c->pinned_ptr[k]);
         delete c;
@@ -487,19 +587,19 @@ void collide(Simulation *sim)
     c->L.launches = 0;
     c->tmp_is_stream = false;
     if (c->L.op_collide()) return;
-    finish(sim, c);
+    finish(sim, c, true);
 }
 void collide_openmp(Simulation *sim) { collide(sim); }
 
 void propagate(Simulation *sim)
 {
-    DropIn *c = prepare(sim, "propagate", false);
+    DropIn *c = prepare(sim, "propagate", false, true);
     if (!c) return;
     c->L.launches = 0;
     c->tmp_is_stream = false;
     if (c->L.op_propagate()) return;
     swap_host(sim);
-    finish(sim, c);
+    if (!finish_ahead(sim, c)) finish(sim, c);
 }
 void propagate_openmp(Simulation *sim) { propagate(sim); }
 
@@ -510,7 +610,7 @@ void collide_with_stream(Simulation *sim)
     c->L.launches = 0;
     if (c->L.op_collide()) return;
     c->tmp_is_stream = true;
-    finish(sim, c);
+    finish(sim, c, true);
 }
 void collide_with_stream_openmp(Simulation *sim) { collide_with_stream(sim); }
 
@@ -523,10 +623,11 @@ void finalize_stream(Simulation *sim)
         swap_host(sim);  // nothing on the device yet: the host arrays are the state
         return;
     }
-    c = prepare(sim, "finalize_stream", false);
+    c = prepare(sim, "finalize_stream", false, true);
     if (!c) return;
     Lattice &L = c->L;
     L.launches = 0;
+    if (!c->tmp_is_stream) c->ahead = false;
     if (c->tmp_is_stream) {
         if (L.op_propagate()) return;  // the second array holds the stream of the collided state
     } else if (L.form == lbgpu::FORM_C && L.pending) {
@@ -541,7 +642,7 @@ void finalize_stream(Simulation *sim)
     }
     c->tmp_is_stream = false;
     swap_host(sim);
-    finish(sim, c);
+    if (!finish_ahead(sim, c)) finish(sim, c);
 }
 
 // ---- two-step forms (lb.c:442-1779) -------------------------------------------------------

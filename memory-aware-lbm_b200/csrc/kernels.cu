@@ -872,11 +872,10 @@ __global__ void k_ghost_copy(Geo g, const S *__restrict__ buf, S *__restrict__ r
 // planes do, and its writes along y, as the records do (576 bytes a column; the writes may go over
 // the link to pinned host memory).
 template <class S>
-__global__ void __launch_bounds__(256) k_readout(Geo g, int view, const S *__restrict__ cur,
-                                                 const S *__restrict__ other,
-                                                 const S *__restrict__ side, int X0, int X1,
-                                                 double *__restrict__ out, int rs,
-                                                 const uint64_t *__restrict__ dynp, float inv)
+__device__ __forceinline__ void readout_block(const Geo &g, int view, const S *__restrict__ cur,
+                                              const S *__restrict__ other, const S *__restrict__ side, int X0, int X1,
+                                              double *__restrict__ out, int rs, const uint64_t *__restrict__ dynp,
+                                              float inv)
 {
     __shared__ double rec[32][8 * 10 + 1];
     const int Xb = X0 + blockIdx.x * 32, Yb = blockIdx.y * 8;
@@ -897,6 +896,30 @@ __global__ void __launch_bounds__(256) k_readout(Geo g, int view, const S *__res
     }
 }
 
+template <class S>
+__global__ void __launch_bounds__(256) k_readout(Geo g, int view, const S *__restrict__ cur,
+                                                 const S *__restrict__ other,
+                                                 const S *__restrict__ side, int X0, int X1,
+                                                 double *__restrict__ out, int rs,
+                                                 const uint64_t *__restrict__ dynp, float inv)
+{
+    readout_block(g, view, cur, other, side, X0, X1, out, rs, dynp, inv);
+}
+
+// The same columns of a collided state as it is (out0) and of the state that its stream gives (out1), in one
+// launch: the drop-in interface hands out the one after the collision and the other after the
+// stream, which itself launches nothing then.
+template <class S>
+__global__ void __launch_bounds__(256) k_readout_both(Geo g, const S *__restrict__ cur, const S *__restrict__ other,
+                                                      const S *__restrict__ side, int X0, int X1,
+                                                      double *__restrict__ out0, double *__restrict__ out1, int rs,
+                                                      const uint64_t *__restrict__ dynp, float inv)
+{
+    const bool streamed = blockIdx.z != 0;
+    readout_block(g, streamed ? VIEW_PULL_PENDING : VIEW_DIRECT, cur, other, side, X0, X1, streamed ? out1 : out0, rs,
+                  dynp, inv);
+}
+
 // FP64 node records of columns [X0, X1) into buffer b (inverse of k_readout).
 template <class S>
 __global__ void __launch_bounds__(BX) k_upload(Geo g, const double *__restrict__ in, int rs, int X0,
@@ -914,36 +937,41 @@ __global__ void __launch_bounds__(BX) k_upload(Geo g, const double *__restrict__
 
 // ---- outlet extrapolation, periodic wrap, initial state, macroscopic fields ---------------
 
-// Density of the post-stream state at columns lx-1 and lx-2 for every row (the inputs of the
-// zero-gradient outlet, unsteady.c:205-214 and lb.c:471-480).
+// Density of the post-stream state at column X of row Y (an input of the zero-gradient outlet).
 template <class S>
-__global__ void k_zgb_rho(Geo g, int view, const S *__restrict__ cur, const S *__restrict__ other,
-                          const S *__restrict__ side, double *__restrict__ zrho, float inv)
+__device__ __forceinline__ double state_density(const Geo &g, int view, const S *__restrict__ cur, const S *__restrict__ other,
+                                                const S *__restrict__ side, int X, int Y, float inv)
 {
-    using R = typename Codec<S>::R;
-    const int Y = blockIdx.x * blockDim.x + threadIdx.x;
-    if (Y > g.ly + 1) return;
-    R f[9];
+    typename Codec<S>::R f[9];
 #pragma unroll
-    for (int i = 0; i < 9; ++i) f[i] = logical(g, view, cur, other, side, g.lx - 1, Y, i, inv);
-    zrho[2 * Y] = (double)rules::density(f);
-#pragma unroll
-    for (int i = 0; i < 9; ++i) f[i] = logical(g, view, cur, other, side, g.lx - 2, Y, i, inv);
-    zrho[2 * Y + 1] = (double)rules::density(f);
+    for (int i = 0; i < 9; ++i) f[i] = logical(g, view, cur, other, side, X, Y, i, inv);
+    return (double)rules::density(f);
 }
 
-// Pressure-table slots fed by the extrapolation: rho = 4/3 rho1 - 1/3 rho2, uPar = 0.
-__global__ void k_zgb_apply(int nb, const int *__restrict__ zgb_src, const double *__restrict__ zrho,
-                            double *__restrict__ bc)
+// The zero-gradient outlet before a step (unsteady.c:205-214 and lb.c:471-480), one launch: the first ly + 2
+// threads write the densities of columns lx-1 and lx-2 of their row, the others the pressure-table slots fed
+// by the extrapolation, rho = 4/3 rho1 - 1/3 rho2, uPar = 0, from densities of their own (18 loads more a
+// slot; a second launch that waited for the first one's cost 4 us a step).
+template <class S>
+__global__ void k_zgb(Geo g, int view, const S *__restrict__ cur, const S *__restrict__ other,
+                      const S *__restrict__ side, const int *__restrict__ zgb_src, double *__restrict__ zrho,
+                      double *__restrict__ bc, float inv)
 {
     using O = Ar<double>;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= 4 * nb) return;
-    const int src = zgb_src[k];
-    if (src < 0) return;
-    const int tb = 4 + k / nb, c = k % nb;
-    bc[(tb * 2 + 0) * nb + c] = O::S(O::M(4. / 3., zrho[2 * src]), O::M(1. / 3., zrho[2 * src + 1]));
-    bc[(tb * 2 + 1) * nb + c] = 0.0;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, k = t - (g.ly + 2);
+    if (k >= 4 * g.nb) return;
+    const int Y = k < 0 ? t : zgb_src[k];
+    if (Y < 0) return;
+    const double r1 = state_density(g, view, cur, other, side, g.lx - 1, Y, inv);
+    const double r2 = state_density(g, view, cur, other, side, g.lx - 2, Y, inv);
+    if (k < 0) {
+        zrho[2 * Y] = r1;
+        zrho[2 * Y + 1] = r2;
+    } else {
+        const int tb = 4 + k / g.nb, c = k % g.nb;
+        bc[(tb * 2 + 0) * g.nb + c] = O::S(O::M(4. / 3., r1), O::M(1. / 3., r2));
+        bc[(tb * 2 + 1) * g.nb + c] = 0.0;
+    }
 }
 
 // Periodic wrap of buffer b (pull form L): the slots a boundary node would receive from across
@@ -1434,6 +1462,15 @@ void launch_readout(const DevLattice &d, int view, int cur, int side_par, int X0
                        SIDE<S>(d, side_par), X0, X1, out, rec_stride, dynp, d.inv_scale)));
 }
 
+void launch_readout_both(const DevLattice &d, int cur, int side_par, int X0, int X1, double *out0, double *out1,
+                         int rec_stride, const uint64_t *dynp, cudaStream_t s)
+{
+    if (X1 <= X0) return;
+    dim3 grid(cdiv(X1 - X0, 32), cdiv(d.g.ly + 2, 8), 2);
+    LBGPU_DISPATCH(d, (k_readout_both<S><<<grid, 256, 0, s>>>(d.g, B<S>(d, cur), OTHER<S>(d, cur), SIDE<S>(d, side_par),
+                       X0, X1, out0, out1, rec_stride, dynp, d.inv_scale)));
+}
+
 void launch_upload(const DevLattice &d, int b, const double *in, int rec_stride, int X0, int X1,
                    int Y0, int H, cudaStream_t s)
 {
@@ -1469,15 +1506,10 @@ void launch_tags_from_xy(const DevLattice &d, const uint8_t *in, cudaStream_t s)
     k_tags_from_xy<<<grid, dim3(32, 8), 0, s>>>(d.g, in, const_cast<uint8_t *>(d.tag));
 }
 
-void launch_zgb_rho(const DevLattice &d, int view, int cur, int side_par, cudaStream_t s)
+void launch_zgb(const DevLattice &d, int view, int cur, int side_par, cudaStream_t s)
 {
-    LBGPU_DISPATCH(d, (k_zgb_rho<S><<<cdiv(d.g.ly + 2, 128), 128, 0, s>>>(d.g, view, B<S>(d, cur),
-                       OTHER<S>(d, cur), SIDE<S>(d, side_par), d.zrho, d.inv_scale)));
-}
-
-void launch_zgb_apply(const DevLattice &d, cudaStream_t s)
-{
-    k_zgb_apply<<<cdiv(4LL * d.g.nb, 256), 256, 0, s>>>(d.g.nb, d.zgb_src, d.zrho, d.bc);
+    LBGPU_DISPATCH(d, (k_zgb<S><<<cdiv(d.g.ly + 2 + 4LL * d.g.nb, 128), 128, 0, s>>>(d.g, view, B<S>(d, cur),
+                       OTHER<S>(d, cur), SIDE<S>(d, side_par), d.zgb_src, d.zrho, d.bc, d.inv_scale)));
 }
 
 void launch_periodic(const DevLattice &d, int b, cudaStream_t s)

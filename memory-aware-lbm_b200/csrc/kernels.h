@@ -51,14 +51,18 @@ void launch_side_from_buf(const DevLattice &d, int b, int side_par, cudaStream_t
 void launch_ghost_copy(const DevLattice &d, int b, cudaStream_t s);
 void launch_readout(const DevLattice &d, int view, int cur, int side_par, int X0, int X1,
                     double *out, int rec_stride, const uint64_t *dynp, cudaStream_t s);
+// launch_readout of a collided pull state as it is (out0) and as its stream gives it (out1; side_par: the
+// parity of the collision before).
+void launch_readout_both(const DevLattice &d, int cur, int side_par, int X0, int X1, double *out0, double *out1,
+                         int rec_stride, const uint64_t *dynp, cudaStream_t s);
 // Records of columns X0..X1-1, rows Y0..Y0+H-1 (in: [X - X0][Y - Y0][rec_stride] doubles) into
 // buffer b.
 void launch_upload(const DevLattice &d, int b, const double *in, int rec_stride, int X0, int X1,
                    int Y0, int H, cudaStream_t s);
 // Tag plane from a device copy of a host-order tag array tag_xy[X * (ly + 2) + Y].
 void launch_tags_from_xy(const DevLattice &d, const uint8_t *in, cudaStream_t s);
-void launch_zgb_rho(const DevLattice &d, int view, int cur, int side_par, cudaStream_t s);
-void launch_zgb_apply(const DevLattice &d, cudaStream_t s);
+// The extrapolated outlet of the state entering a step: zrho of every row and the tables' slots.
+void launch_zgb(const DevLattice &d, int view, int cur, int side_par, cudaStream_t s);
 void launch_periodic(const DevLattice &d, int b, cudaStream_t s);
 // Tag plane of the cylinder channel (obstacle disk, walls of wall_kind, regularized inlet,
 // pressure-regularized outlet) written on the device.

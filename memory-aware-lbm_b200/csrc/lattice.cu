@@ -183,7 +183,7 @@ void Lattice::destroy()
     if (stream) cudaStreamSynchronize(stream);
     if (memory) device_free(memory, memory_bytes, stream);
     memory = nullptr;
-    if (stage) cudaFree(stage);
+    if (stage) device_free(stage, stage_bytes, stream);
     if (red_scratch) cudaFree(red_scratch);
     if (vel_acc) cudaFree(vel_acc);
     if (shift) cudaFree(shift);
@@ -278,9 +278,8 @@ int Lattice::zgb_pass()
         return set_error(LB_ERR_STATE, "extrapolated outlet requested on a collided state");
     int v, par;
     view(v, par);
-    launch_zgb_rho(d, v, cur, par, stream);
-    launch_zgb_apply(d, stream);
-    launches += 2;
+    launch_zgb(d, v, cur, par, stream);
+    ++launches;
     return check("zgb pass");
 }
 
@@ -348,13 +347,16 @@ long long Lattice::steps_done() const
     return n;
 }
 
+// Results up to this size are copied from a device buffer; larger ones go through read_back.
+static constexpr size_t kStagedBytes = (size_t)1 << 20;
+
 // ---- data movement --------------------------------------------------------------------
 int Lattice::ensure_stage(size_t need)
 {
     if (stage_bytes >= need) return LB_OK;
-    if (stage) { cudaStreamSynchronize(stream); cudaFree(stage); stage = nullptr; stage_bytes = 0; }
+    if (stage) { cudaStreamSynchronize(stream); device_free(stage, stage_bytes, stream); stage = nullptr; stage_bytes = 0; }
     void *p = nullptr;
-    LB_CUDA(cudaMalloc(&p, need), "cudaMalloc(staging)");
+    LB_CUDA(device_alloc(&p, need, device, stream), "device memory (staging)");
     stage = static_cast<double *>(p);
     stage_bytes = need;
     return LB_OK;
@@ -440,6 +442,8 @@ int Lattice::readout_records(double *host, int rs, const uint64_t *dynp_dev, int
 
 int Lattice::readout_populations(double *host)
 {
+    // small ones through the device staging: pinned memory that nobody holds yet takes 1.7 ms to get
+    if ((size_t)(lx + 2) * (ly + 2) * 72 <= kStagedBytes) return readout_records(host, 9, nullptr, 0, lx + 2);
     int v, par;
     view(v, par);
     const size_t col = (size_t)(ly + 2) * 9;
@@ -478,6 +482,17 @@ int Lattice::get_macros(double *rho, double *ux, double *uy)
     double *field[3];
     for (double *p : to)
         if (p) field[n++] = p;
+    const size_t nn = (size_t)lx * ly;
+    if (n && n * nn * sizeof(double) <= kStagedBytes) {
+        LB_TRY(ensure_stage(3 * nn * sizeof(double)));
+        launch_macros(d, v, cur, par, 1, ly + 1, stage, stage + nn, stage + 2 * nn, stream);
+        LB_TRY(check("macros"));
+        for (int j = 0; j < 3; ++j)
+            if (to[j])
+                LB_CUDA(cudaMemcpyAsync(to[j], stage + j * nn, nn * sizeof(double), cudaMemcpyDeviceToHost, stream), "macros");
+        d2h_bytes += n * nn * sizeof(double);
+        return cuda_error(cudaStreamSynchronize(stream), "macros");
+    }
     // one item a row: its values of each field wanted, one field after the other in a chunk
     const cudaError_t e = read_back(
         device, stream, n ? ly : 0, (size_t)n * lx * sizeof(double),
@@ -563,6 +578,17 @@ int Lattice::upload_bc(const double *bc)
     // the copy reads bc_host asynchronously: wait so the caller may reuse its array and
     // the next refresh may overwrite bc_host
     LB_CUDA(cudaStreamSynchronize(stream), "upload tables");
+    return LB_OK;
+}
+
+int Lattice::upload_bc_range(const double *bc, size_t lo, size_t hi)
+{
+    if (hi <= lo) return LB_OK;
+    std::memcpy(bc_host.data() + lo, bc + lo, (hi - lo) * sizeof(double));
+    // a copy from pageable memory has taken its source when the call returns, so nothing waits here
+    LB_CUDA(cudaMemcpyAsync(d.bc + lo, bc_host.data() + lo, (hi - lo) * sizeof(double), cudaMemcpyHostToDevice,
+                            stream), "upload tables");
+    h2d_bytes += (hi - lo) * sizeof(double);
     return LB_OK;
 }
 

@@ -77,6 +77,7 @@ struct Lattice {
 
     // data movement
     int upload_bc(const double *bc);      // host [16*nb]
+    int upload_bc_range(const double *bc, size_t lo, size_t hi);  // entries lo..hi-1 of them, without waiting
     int upload_zgb_src(const int *src);   // host [4*nb]
     // host tag[X*(ly+2)+Y], validated here; zgb_row: rows of the extrapolated outlet, or null
     int upload_tags(const uint8_t *tag_xy, const uint8_t *zgb_row);
