@@ -210,8 +210,8 @@ int lbgpu_synchronize(lbgpu_lattice *lat);
 /* ---- batches: many independent lattices in one launch per step --------------------------
  * No counterpart in the reference (one lattice per process).  Members are lattices of the
  * batch's precision, pull or AA, with constant-density outlets (an extrapolated outlet is
- * stepped on its own).  lbgpu_batch_step advances every member by nsteps: one launch per step (per two
- * steps for FP64 and FP32) for the pull members and one per step for each phase of the AA members walks a
+ * stepped on its own).  lbgpu_batch_step advances every member by nsteps: one launch per two steps
+ * for the pull members (per step where one stores row-shifted offsets) and one per step for each phase of the AA members walks a
  * work list of tiles; chunks of 20 steps are replayed as a CUDA graph.  Each member's result is bit-identical to stepping it alone.  The batch does not
  * own its members; remove a member before destroying it.  Steps are asynchronous on the batch's
  * stream and ordered with the members' own streams. */

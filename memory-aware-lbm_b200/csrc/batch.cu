@@ -10,9 +10,9 @@
 // once as a CUDA graph: the kernels read each member's buffers and parities from a device
 // descriptor array, so the same graph replays chunk after chunk; it is re-captured when the
 // membership or the launch form changes.
-// FP64 and FP32 pull members take two steps a launch on tiles in shared memory (tile.cuh), one work list of tiles for
+// Pull members take two steps a launch on tiles in shared memory (tile.cuh), one work list of tiles for
 // all of them: 24 uneven channels of 8.6M nodes in FP32 119 -> 75 us a step, 24 of 5.7M nodes in FP64 162 -> 108,
-// 24 small ones (0.7M nodes) in FP32 20.7 -> 8.3.
+// 24 small ones (0.7M nodes) in FP32 20.7 -> 8.3, 48 of 13.4M nodes in FP16 153 -> 101 (packed pairs of nodes).
 // A work item is a strip of tiles of one member stacked in y: its block reads the member's
 // descriptor once and steps the tiles one after another down the lattice, so the descriptor's
 // dependent loads are spread over the strip.  Tile widths and strip lengths are chosen per size
@@ -36,8 +36,8 @@ constexpr int kChunk = 20;      // steps per captured graph (a multiple of 4: th
                                 // parities repeat after two two-step launches)
 constexpr int kLists = 6;       // pull, pull four nodes a thread; AA of phase parity 0, 1 at rebuild;
                                 // the perimeters of the four-nodes-a-thread members; the tiles of the
-                                // pull members that take two steps a launch (list 0 holds them too,
-                                // for a single step)
+                                // pull members where they take two steps a launch (lists 0, 1 and 4 hold
+                                // them too, for a single step)
 constexpr int kTiles = 5;
 constexpr int kQuad = 3;        // shape of the four-nodes-a-thread pull tiles (16-bit storage)
 constexpr int kMaxPasses = 64;  // tiles a block may step down one member
@@ -142,17 +142,13 @@ int refresh_collision_numbers(lbgpu_batch *b, int done)
                                        cudaMemcpyHostToDevice, b->stream), "update batch collision numbers");
 }
 
-// Pull members of a storage type with a tile kernel take two steps a launch.
-bool takes_tiles(const Lattice &L)
-{
-    int w, h;
-    return L.scheme == LBGPU_PULL && lbgpu::batch_tile(L.precision, &w, &h);
-}
+// Pull members can take two steps a launch, but for row-shifted offsets (rebased between rows).
+bool takes_tiles(const Lattice &L) { return L.scheme == LBGPU_PULL && !L.d.g.shift_u; }
 
-// A member's host-side state after `m` batch steps (no launches); tiles: taken two a launch.
+// A member's host-side state after `m` batch steps (no launches); tiles: pull members took two a launch.
 void advance(Lattice &L, int m, bool tiles)
 {
-    if (tiles && takes_tiles(L)) {
+    if (tiles && L.scheme == LBGPU_PULL) {
         for (; m >= lbgpu::BATCH_TILE_STEPS; m -= lbgpu::BATCH_TILE_STEPS) L.after_tile(lbgpu::BATCH_TILE_STEPS);
         return;
     }
@@ -206,6 +202,11 @@ void drop_graphs(lbgpu_batch *b)
 int rebuild(lbgpu_batch *b)
 {
     std::vector<BatchWork> work[kLists], inner;
+    int w, h;
+    lbgpu::batch_tile(b->precision, &w, &h);
+    bool tiled = true;      // all pull members, or none: their single-step lists are shared
+    for (const lbgpu_lattice *m : b->members)
+        if (m && m->L.scheme == LBGPU_PULL && !takes_tiles(m->L)) tiled = false;
     b->h_inst.assign(b->members.size(), BatchInst{});
     for (size_t i = 0; i < b->members.size(); ++i) {
         lbgpu_lattice *m = b->members[i];
@@ -220,8 +221,7 @@ int rebuild(lbgpu_batch *b)
         for (int y0 = 1; y0 <= L.ly; y0 += th)
             for (int x0 = 1; x0 <= L.lx; x0 += tw)
                 work[s].push_back(BatchWork{(int)i, x0, y0, lbgpu::batch_sp(sh, np)});
-        int w, h;
-        if (takes_tiles(L) && lbgpu::batch_tile(b->precision, &w, &h))
+        if (tiled && L.scheme == LBGPU_PULL)
             for (int y0 = 1; y0 <= L.ly; y0 += h)
                 for (int x0 = 1; x0 <= L.lx; x0 += w) {
                     const bool ring = x0 == 1 || y0 == 1 || x0 + w > L.lx || y0 + h > L.ly;
@@ -269,12 +269,12 @@ int rebuild(lbgpu_batch *b)
     return LB_OK;
 }
 
-// k-th single step of a chunk: one launch per non-empty work list (without_tiled: not of the list whose
-// members take two steps a launch).
+// k-th single step of a chunk: one launch per non-empty work list (without_tiled: not of the pull members'
+// lists, which take two steps a launch).
 void launch_step(lbgpu_batch *b, int k, bool without_tiled)
 {
     for (int s = 0; s < kTiles; ++s) {
-        if (!b->nwork[s] || (s == 0 && without_tiled)) continue;
+        if (!b->nwork[s] || (without_tiled && (s == 0 || s == 1 || s == 4))) continue;
         int kind = s == 0 ? lbgpu::BATCH_PULL : (s == 1 ? lbgpu::BATCH_PULL4 : lbgpu::BATCH_PERIM);
         if (s == 2 || s == 3) {
             const int phase = (s == 2) ? b->aa_phase : 1 - b->aa_phase;
@@ -293,7 +293,7 @@ void launch_step(lbgpu_batch *b, int k, bool without_tiled)
 void launch_unit(lbgpu_batch *b, int unit)
 {
     if (b->nwork[kTiles]) {
-        lbgpu::launch_batch_tile(b->precision, b->d_inst, b->d_work[kTiles], b->nwork[kTiles], unit, b->stream);
+        lbgpu::launch_batch_tile(b->precision, b->rs, b->d_inst, b->d_work[kTiles], b->nwork[kTiles], unit, b->stream);
         ++b->launches;
     }
     const bool tiled = b->nwork[kTiles] > 0;
@@ -550,7 +550,7 @@ int lbgpu_batch_step(lbgpu_batch *b, int nsteps)
     for (int u = 0; u < rem / 2; ++u) launch_unit(b, u);
     if (int rc = lbgpu::cuda_error(cudaGetLastError(), "batch step")) return rc;
     for (lbgpu_lattice *m : b->members)
-        if (m) advance(m->L, nsteps, true);
+        if (m) advance(m->L, nsteps, b->nwork[kTiles] > 0);
     if (int rc = order_after(b)) return rc;
     if ((rem & 3) || any_rs) {
         // two-step launches in an odd number turned buffers and side store over (or stochastically

@@ -40,8 +40,8 @@ int pull_launches(const DevLattice &d, bool ghosts);
 void launch_stream(const DevLattice &d, int src, int side_par, cudaStream_t s);
 // Pull steps per launch of the tile kernel (tile.cu) for a run of `steps` steps from form C pending:
 // 0 where single steps are the faster way (or the only one).  `outlet`: the outlet is
-// extrapolated before every step.
-int tile_steps(const DevLattice &d, long long steps, bool outlet);
+// extrapolated before every step; `rs`: stored values are rounded stochastically.
+int tile_steps(const DevLattice &d, long long steps, bool outlet, bool rs);
 // T pull steps (a count that tile_steps returned) in one launch: C_n in buffer src (n_par = n & 1)
 // -> C_{n+T} in buffer 1 - src, where T single steps would have left it in src: the caller turns
 // ghost_flip over and changes the side store's slots' roles (Lattice::after_tile).  keys: rounding keys of the T collisions (16-bit).
@@ -129,11 +129,11 @@ __host__ __device__ inline int batch_sp(int shape, int passes) { return shape | 
 // row-shifted offsets; the kernels then carry those paths.
 void launch_batch(int precision, int kind, int threads, bool persistent, int flags, const BatchInst *insts,
                   const BatchWork *work, int nwork, int grid, int k, cudaStream_t s);
-// The batch's tile kernel (tile.cu): nodes of a tile, false where the storage type has none; and two
-// steps (BATCH_TILE_STEPS) of every tile of a work list, launch `unit` since the descriptors.
+// The batch's tile kernel (tile.cu): nodes of a tile; and two steps (BATCH_TILE_STEPS) of every tile of a work
+// list, launch `unit` since the descriptors (rs: some member rounds stochastically).
 constexpr int BATCH_TILE_STEPS = 2;
-bool batch_tile(int precision, int *w, int *h);
-void launch_batch_tile(int precision, const BatchInst *insts, const BatchWork *work, int nwork, int unit, cudaStream_t s);
+void batch_tile(int precision, int *w, int *h);
+void launch_batch_tile(int precision, bool rs, const BatchInst *insts, const BatchWork *work, int nwork, int unit, cudaStream_t s);
 // Resident blocks per SM of the persistent kernel of a kind and block size.
 int batch_blocks_per_sm(int precision, int kind, int threads);
 

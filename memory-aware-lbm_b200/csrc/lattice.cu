@@ -310,7 +310,7 @@ int Lattice::step(int nsteps)
     for (int s = 0; s < nsteps; ++s) {
         // a run of pull steps: several a launch, the state as single steps leave it
         if (scheme == LBGPU_PULL && !ghosts && form == FORM_C && pending) {
-            if (const int T = tile_steps(d, nsteps - s, zgb_each_step)) {
+            if (const int T = tile_steps(d, nsteps - s, zgb_each_step, rs)) {
                 unsigned keys[8] = {0};
                 for (int k = 0; rs && k < T; ++k) keys[k] = rs_key(rs_seed, (unsigned long long)(n + 1 + k));
                 launch_tile(d, cur, (int)(n & 1), T, zgb_each_step, keys, stream);

@@ -14,12 +14,14 @@ namespace {
 //   small lattices: many steps a launch on small tiles, so that every SM has a tile and the launch is
 //     shared: FP64 250 x 51 2.4 (4 steps 2.8, single 3.5), FP32 1.5 (1.9, 3.3), FP16 1.9 (2.2, 6.7)
 //   511 x 127: FP64 3.8 (5.0 with 2 steps, single 4.0), FP32 2.5 (2.6 with 8 steps, single 3.5)
-//   700 x 200: FP64 5.4 (5.6 with 2 steps), FP32 2.9 (3.2 on 32 x 8 tiles, single 4.3), FP16 3.5 (7.2)
+//   700 x 200: FP64 5.4 (5.6 with 2 steps), FP32 2.9 (3.2 on 32 x 8 tiles, single 4.3), FP16 3.4 (3.5 on 416 threads, single 7.2)
 //   1024 x 256: FP64 7.4 (8.3 with 4 steps, single 7.0 in a graph and 9.0 launched), FP32 4.2 (5.2 with 2, 5.5)
-//   2047 x 511: FP64 21.9 (24.2 on 64 x 16, single 27.7), FP32 10.1 (11.1 with 4 steps, 12.8), FP16 11.4 (12.3)
+//   2047 x 511: FP64 21.9 (24.2 on 64 x 16, single 27.7), FP32 10.1 (11.1 with 4 steps, 12.8), FP16 8.9 (10.0 with 2 steps, 12.3)
 //   large: two steps, tiles whose halo is small against them, and few enough threads' registers for
 //     several blocks a SM: 8192 x 2048 FP64 233 (two blocks of 64 x 16; 236 with four of 32 x 16; single 355), FP32
-//     109 (five of 64 x 12; 111 with six of 64 x 8; single 187).  16-bit storage has k_pull4h there.
+//     109 (five of 64 x 12; 111 with six of 64 x 8; single 187), FP16 93 (97 with prefetch; single 109);
+//     16384 x 4096 FP16 342 (single 388), with stochastic rounding 398 (single 398: its hash and
+//     multiplies bind), so those keep k_pull4h from 24M nodes on; 4096 x 1024 31 and 38.
 // Large lattices prefetch the tile 100 (FP64) or 200 (FP32) blocks ahead into L2: 253 -> 233 and 120 -> 109 us;
 // 0.3 of that distance does half as much, 4 times it costs 15-30 % (evicted before it is read).
 using F64Small = TileShape<double, 16, 8, 8, 704, 1>;
@@ -35,7 +37,8 @@ using F32Large = TileShape<float, 64, 12, 2, 224, 5>;
 using F64Batch = TileShape<double, 32, 16, 2, 256, 4>;
 using F32Batch = F32Large;
 template <class S> using HalfSmall = TileShape<S, 16, 8, 8, 384, 2>;
-template <class S> using HalfWide = TileShape<S, 32, 16, 4, 416, 3>;
+template <class S> using HalfWide = TileShape<S, 32, 16, 4, 448, 3>;
+template <class S> using HalfLarge = TileShape<S, 64, 12, 2, 224, 5>;
 
 enum { TILE_SMALL = 0, TILE_MID = 1, TILE_WIDE = 2, TILE_LARGE = 3, TILE_NONE = 4 };
 
@@ -103,19 +106,20 @@ template <class S>
 void launch_half(const DevLattice &d, int src, int n_par, int T, bool outlet, const unsigned *keys, cudaStream_t s)
 {
     if (T == 8) launch_one<HalfSmall<S>>(d, src, n_par, outlet, 0, keys, s);
-    else launch_one<HalfWide<S>>(d, src, n_par, outlet, 0, keys, s);
+    else if (T == 4) launch_one<HalfWide<S>>(d, src, n_par, outlet, 0, keys, s);
+    else launch_one<HalfLarge<S>>(d, src, n_par, outlet, 0, keys, s);
 }
 
 }  // namespace
 
-int tile_steps(const DevLattice &d, long long steps, bool outlet)
+int tile_steps(const DevLattice &d, long long steps, bool outlet, bool rs)
 {
     if (steps < 2 || (outlet && !d.outlet_tiles)) return 0;
     const int shape = tile_shape(d);
     if (d.precision == LBGPU_F16 || d.precision == LBGPU_BF16) {
-        // row-shifted offsets are rebased between rows, and large lattices have the quads of k_pull4h
-        if (d.g.shift_u || shape == TILE_LARGE) return 0;
-        return shape == TILE_SMALL && steps >= 8 ? 8 : (steps >= 4 ? 4 : 0);
+        if (d.g.shift_u) return 0;          // row-shifted offsets are rebased between rows
+        if (rs && (long long)d.g.lx * d.g.ly >= (24ll << 20)) return 0;
+        return shape == TILE_SMALL && steps >= 8 ? 8 : (steps >= 4 && shape != TILE_LARGE ? 4 : 2);
     }
     if (shape == TILE_SMALL && steps >= 8) return 8;
     if (steps >= 4 && (shape <= TILE_MID || (shape == TILE_WIDE && d.precision == LBGPU_F32))) return 4;
@@ -143,21 +147,38 @@ void launch_tile(const DevLattice &d, int src, int n_par, int T, bool outlet, co
     }
 }
 
-bool batch_tile(int precision, int *w, int *h)
+namespace {
+
+template <class SH, bool RS>
+void launch_batch_shape(const BatchInst *insts, const BatchWork *work, int nwork, int unit, cudaStream_t s)
 {
-    if (precision == LBGPU_F64) { *w = F64Batch::W; *h = F64Batch::H; return true; }
-    if (precision == LBGPU_F32) { *w = F32Batch::W; *h = F32Batch::H; return true; }
-    return false;
+    cudaFuncSetAttribute(k_batch_tile<SH, RS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SH::SMEM);
+    k_batch_tile<SH, RS><<<nwork, SH::NT, SH::SMEM, s>>>(insts, work, unit);
 }
 
-void launch_batch_tile(int precision, const BatchInst *insts, const BatchWork *work, int nwork, int unit, cudaStream_t s)
+template <class S>
+void launch_batch_half(bool rs, const BatchInst *insts, const BatchWork *work, int nwork, int unit, cudaStream_t s)
 {
-    if (precision == LBGPU_F64) {
-        cudaFuncSetAttribute(k_batch_tile<F64Batch, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F64Batch::SMEM);
-        k_batch_tile<F64Batch, false><<<nwork, F64Batch::NT, F64Batch::SMEM, s>>>(insts, work, unit);
-    } else {
-        cudaFuncSetAttribute(k_batch_tile<F32Batch, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F32Batch::SMEM);
-        k_batch_tile<F32Batch, false><<<nwork, F32Batch::NT, F32Batch::SMEM, s>>>(insts, work, unit);
+    if (rs) launch_batch_shape<HalfLarge<S>, true>(insts, work, nwork, unit, s);
+    else launch_batch_shape<HalfLarge<S>, false>(insts, work, nwork, unit, s);
+}
+
+}  // namespace
+
+void batch_tile(int precision, int *w, int *h)
+{
+    *w = precision == LBGPU_F64 ? F64Batch::W : (precision == LBGPU_F32 ? F32Batch::W : HalfLarge<__half>::W);
+    *h = precision == LBGPU_F64 ? F64Batch::H : (precision == LBGPU_F32 ? F32Batch::H : HalfLarge<__half>::H);
+}
+
+void launch_batch_tile(int precision, bool rs, const BatchInst *insts, const BatchWork *work, int nwork, int unit,
+                       cudaStream_t s)
+{
+    switch (precision) {
+    case LBGPU_F64: launch_batch_shape<F64Batch, false>(insts, work, nwork, unit, s); break;
+    case LBGPU_F32: launch_batch_shape<F32Batch, false>(insts, work, nwork, unit, s); break;
+    case LBGPU_F16: launch_batch_half<__half>(rs, insts, work, nwork, unit, s); break;
+    default: launch_batch_half<__nv_bfloat16>(rs, insts, work, nwork, unit, s); break;
     }
 }
 

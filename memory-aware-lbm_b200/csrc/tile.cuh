@@ -15,6 +15,8 @@
 //   FP64  16384 x 4096 1476 -> 978  (HBM -> 68 GLUPS at 67 B an update, FP64 pipe half busy)
 //   FP32  1024 x 256   8.2 -> 3.6
 //   FP32  8192 x 2048  189 -> 111   (HBM -> 151 GLUPS at 32 B an update, 114 instructions an update)
+//   FP16  2047 x 511   14.4 -> 7.7, 4096 x 1024 36 -> 26, 16384 x 4096 384 -> 346 (issue: 139 instructions an update in
+//         k_pull4h), with stochastic rounding 14.9 -> 9.3, 37.8 -> 29.7 (the single kernel from 24M nodes on)
 // Loading the tiles by TMA instead (whole boxes of nine planes into a third buffer, results stored by TMA)
 // ran at 124-129 GLUPS where this form had 134 (FP32 before the pairs) and 63 against 67 (FP64): the extra
 // buffer costs resident blocks, and their overlap is what hides the latencies of both halves.
@@ -190,7 +192,7 @@ __device__ __forceinline__ void tile_bulk(const TileArgs<S> &a, int t, typename 
 }
 
 // Step s (1..T) of the tile: the region of W + 2 (T - s) by H + 2 (T - s) nodes, one node a thread.  Only
-// blocks whose region stays off the perimeter (and FP32 ones then run tile_step_pairs) have EDGE
+// blocks whose region stays off the perimeter (all but FP64 then run tile_step_pairs) have EDGE
 // false and skip the tests of lattice bounds.  Nodes with boundary rules (250-500 operations, mostly one after
 // another) are listed at step 1 and run packed in warps of their own beside the others: left in
 // their places, one or two lanes of every row's warp would hold the whole warp that long.
@@ -277,11 +279,58 @@ __device__ __forceinline__ void tile_step(const TileArgs<S> &a, S *__restrict__ 
     }
 }
 
-// Two nodes side by side, as one load or store of twice the width.  FP32 runs pairs (172 -> 114 instructions
+// Two nodes side by side, as one load or store of twice the width.  FP32 and 16-bit storage run pairs (FP32 172 -> 114 instructions
 // an update, 134 -> 150 GLUPS at 8192 x 2048: addresses, loop and stores are shared and the arithmetic packed); FP64
 // does not (its arithmetic is not packed, and two nodes' registers halve the resident warps: 66 -> 56 GLUPS).
-template <class S> struct Pair;
-template <> struct Pair<float> { using V = float2; };
+template <class S>
+__device__ __forceinline__ float2 pair_load(const S *p)            // p on a pair's boundary
+{
+    if constexpr (sizeof(S) == 4) return *reinterpret_cast<const float2 *>(p);
+    else {
+        const unsigned w = *reinterpret_cast<const unsigned *>(p);
+        return make_float2(Half2Ops<S>::lo(w), Half2Ops<S>::hi(w));
+    }
+}
+
+template <class S>
+__device__ __forceinline__ float2 pair_gather(const S *p)          // p anywhere
+{
+    return make_float2(Work<S>::load(p[0], 0, 0.0f), Work<S>::load(p[1], 0, 0.0f));
+}
+
+// Direction i of the pair as stored; rs: its stochastic rounding bits (16-bit, RS).
+template <class S, bool RS>
+__device__ __forceinline__ void pair_store(S *p, float2 f, unsigned rs)
+{
+    if constexpr (sizeof(S) == 4) *reinterpret_cast<float2 *>(p) = f;
+    else *reinterpret_cast<unsigned *>(p) = RS ? RsOps<S>::pack(f.x, f.y, rs) : Half2Ops<S>::pack(f.x, f.y);
+}
+
+// The rounding bits of nodes X, X + 1 of a row (rs_node, put): the bits of a quad's pair p are m (2 (9 p + i) + 1)
+// with m the quad's hash times codec.cuh's constant; a pair that starts at an even X takes the upper
+// half of one of them and the lower half of the next.
+template <bool SPLIT>
+struct PairBits {
+    unsigned ma, oa, mb, ob;
+    __device__ __forceinline__ unsigned bits(int i) const
+    {
+        const unsigned a = ma * (unsigned)(2 * i + 1) + oa;
+        return SPLIT ? __byte_perm(a, mb * (unsigned)(2 * i + 1) + ob, 0x5432) : a;
+    }
+};
+
+template <bool SPLIT>
+__device__ __forceinline__ PairBits<SPLIT> pair_bits(const Geo &g, unsigned key, int X, int Y)
+{
+    const int q = (X - 1) & 3;          // 0 or 2; split pairs 1 or 3
+    const unsigned row = (unsigned)Y * (unsigned)(g.lx + 2);
+    PairBits<SPLIT> b;
+    b.ma = rs_mix((row + (unsigned)(X - q)) ^ key) * 0x9e3779b9u;
+    b.oa = (q & 2) ? 18u * b.ma : 0u;
+    b.mb = SPLIT && q == 3 ? rs_mix((row + (unsigned)(X + 1)) ^ key) * 0x9e3779b9u : b.ma;
+    b.ob = SPLIT && q == 1 ? 18u * b.ma : 0u;
+    return b;
+}
 
 __device__ __forceinline__ unsigned long long x2(float2 v) { return *reinterpret_cast<unsigned long long *>(&v); }
 __device__ __forceinline__ float2 f2(unsigned long long v) { return *reinterpret_cast<float2 *>(&v); }
@@ -335,14 +384,43 @@ __device__ __forceinline__ void bgk_pair(float2 f[9], float omega)
 #undef LBGPU_RELAX2
 }
 
-// Step s of a tile that holds no perimeter node and no boundary rule, two nodes a thread (FP32).
+// bgk_offsets<false> on two nodes, in the same way.
+__device__ __forceinline__ void bgk_offsets_pair(float2 D[9], float omega, float sc, float inv)
+{
+    const float2 sum = add2(add2(add2(add2(D[0], D[1]), add2(D[2], D[3])), add2(add2(D[4], D[5]), add2(D[6], D[7]))), D[8]);
+    const float2 d = mul2(c2(inv), sum);
+    const float2 Jx = add2(add2(sub2(D[1], D[3]), sub2(D[5], D[6])), sub2(D[8], D[7]));
+    const float2 Jy = add2(add2(sub2(D[2], D[4]), sub2(D[5], D[8])), sub2(D[6], D[7]));
+    const float2 ir = make_float2(__fdividef(1.0f, 1.0f + d.x), __fdividef(1.0f, 1.0f + d.y));
+    const float2 q = mul2(c2(inv), ir);
+    const float2 ux = mul2(Jx, q), uy = mul2(Jy, q);
+    const float2 A = fma2(c2(-1.5f * inv), fma2(Jx, ux, mul2(Jy, uy)), d);
+    const float2 ux45 = mul2(c2(4.5f * inv), ux), uy45 = mul2(c2(4.5f * inv), uy);
+    const float om1 = 1.0f - omega;
+    const float k0 = omega * sc * (4.f / 9.f), k1 = omega * sc * (1.f / 9.f), k2 = omega * sc * (1.f / 36.f);
+    const float b1 = (3.0f * inv) * k1, b2 = (3.0f * inv) * k2;
+    D[0] = fma2(c2(om1), D[0], mul2(c2(k0), A));
+#define LBGPU_PAIR2(I, J, K, B, CU45, CJ)                             \
+    {                                                                 \
+        const float2 cj = (CJ);                                       \
+        const float2 a = mul2(c2(K), fma2(CU45, cj, A));              \
+        D[I] = fma2(c2(om1), D[I], fma2(c2(B), cj, a));               \
+        D[J] = fma2(c2(om1), D[J], fma2(c2(-(B)), cj, a));            \
+    }
+    LBGPU_PAIR2(1, 3, k1, b1, ux45, Jx)
+    LBGPU_PAIR2(2, 4, k1, b1, uy45, Jy)
+    LBGPU_PAIR2(5, 7, k2, b2, add2(ux45, uy45), add2(Jx, Jy))
+    LBGPU_PAIR2(6, 8, k2, b2, sub2(uy45, ux45), sub2(Jy, Jx))
+#undef LBGPU_PAIR2
+}
+
+// Step s of a tile that holds no perimeter node and no boundary rule, two nodes a thread (FP32 and 16-bit).
 // The pairs of step s start at column x0 - (T - s): a step later they start one column on, so the
 // two populations that a pair takes from x - 1 or x + 1 were stored (or, T being even, lie in the
 // planes) as one pair, and only those of the three directions along y are read one by one.
-template <class S, class SH, int s>
+template <class S, class SH, int s, bool RS>
 __device__ __forceinline__ void tile_step_pairs(const TileArgs<S> &a, S *__restrict__ sm, uint8_t *__restrict__ stag, int x0, int y0)
 {
-    using V = typename Pair<S>::V;
     constexpr int E = SH::T - s, WP = (SH::W + 2 * E) / 2, HS = SH::H + 2 * E, O = s - 1, RW = SH::RW, PL = SH::PL;
     const Geo &g = a.g;
     const S *rd = sm + (size_t)(s & 1) * (SH::NBUF - 1) * SH::B1;
@@ -354,7 +432,7 @@ __device__ __forceinline__ void tile_step_pairs(const TileArgs<S> &a, S *__restr
     for (; r < HS; c += SH::NT % WP, r += SH::NT / WP, r += c >= WP ? 1 : 0, c -= c >= WP ? WP : 0) {
         const int q = (r + O) * RW + (2 * c + O);
         const unsigned go = (unsigned)r * pitch + (unsigned)c * (unsigned)(2 * sizeof(S));
-        V f[9];
+        float2 f[9];
         unsigned t;
         if (s == 1) {
             const uint8_t *gt = a.tag + o0 + (go / (unsigned)sizeof(S));
@@ -363,23 +441,21 @@ __device__ __forceinline__ void tile_step_pairs(const TileArgs<S> &a, S *__restr
 #pragma unroll
             for (int i = 0; i < 9; ++i) {
                 const S *p = reinterpret_cast<const S *>(gs + ((long long)i * g.plane - (long long)cy(i) * g.pitch) * (long long)sizeof(S)) - cx(i);
-                if (cx(i) != 0) f[i] = *reinterpret_cast<const V *>(p);
-                else { f[i].x = p[0]; f[i].y = p[1]; }
+                f[i] = cx(i) != 0 ? pair_load(p) : pair_gather(p);
             }
             *reinterpret_cast<unsigned short *>(stag + q) = (unsigned short)t;
         } else {
             t = stag[q] | ((unsigned)stag[q + 1] << 8);
             const S *p = rd + q;
 #pragma unroll
-            for (int i = 0; i < 9; ++i) {
-                if (cx(i) != 0) f[i] = *reinterpret_cast<const V *>(p + (i * PL - cy(i) * RW - cx(i)));
-                else { f[i].x = p[i * PL - cy(i) * RW]; f[i].y = p[i * PL - cy(i) * RW + 1]; }
-            }
+            for (int i = 0; i < 9; ++i)
+                f[i] = cx(i) != 0 ? pair_load(p + (i * PL - cy(i) * RW - cx(i))) : pair_gather(p + (i * PL - cy(i) * RW));
         }
         if (t == 0x0101u) {
-            bgk_pair(f, a.omega_f);
+            if constexpr (sizeof(S) == 2) bgk_offsets_pair(f, a.omega_f, a.sc, a.inv);
+            else bgk_pair(f, a.omega_f);
         } else {
-            S h[9];
+            float h[9];
 #pragma unroll
             for (int i = 0; i < 9; ++i) h[i] = f[i].x;
             tile_bulk<S>(a, (int)(t & 0xffu), h);
@@ -389,13 +465,17 @@ __device__ __forceinline__ void tile_step_pairs(const TileArgs<S> &a, S *__restr
 #pragma unroll
             for (int i = 0; i < 9; ++i) f[i].y = h[i];
         }
+        constexpr bool SPLIT = (E & 1) != 0;              // x0 is odd: X = x0 - E + 2 c is even
+        PairBits<SPLIT> b = {};
+        if constexpr (RS) b = pair_bits<SPLIT>(g, a.keys[s - 1], x0 - E + 2 * c, y0 - E + r);
         if (s == SH::T) {
             char *gd = reinterpret_cast<char *>(a.dst + o0) + go;
 #pragma unroll
-            for (int i = 0; i < 9; ++i) *reinterpret_cast<V *>(gd + (long long)i * g.plane * (long long)sizeof(S)) = f[i];
+            for (int i = 0; i < 9; ++i)
+                pair_store<S, RS>(reinterpret_cast<S *>(gd + (long long)i * g.plane * (long long)sizeof(S)), f[i], RS ? b.bits(i) : 0u);
         } else {
 #pragma unroll
-            for (int i = 0; i < 9; ++i) *reinterpret_cast<V *>(wr + i * PL + q) = f[i];
+            for (int i = 0; i < 9; ++i) pair_store<S, RS>(wr + i * PL + q, f[i], RS ? b.bits(i) : 0u);
         }
     }
 }
@@ -404,7 +484,7 @@ template <class S, class SH, int s, bool EDGE, bool RS, bool EXTRAP>
 __device__ __forceinline__ void tile_steps(const TileArgs<S> &a, S *sm, uint8_t *stag, unsigned short *list, int *nlist,
                                            int x0, int y0)
 {
-    if constexpr (!EDGE && sizeof(S) == 4) tile_step_pairs<S, SH, s>(a, sm, stag, x0, y0);
+    if constexpr (!EDGE && sizeof(S) <= 4) tile_step_pairs<S, SH, s, RS>(a, sm, stag, x0, y0);
     else tile_step<S, SH, s, EDGE, RS, EXTRAP>(a, sm, stag, list, nlist, x0, y0);
     if constexpr (s < SH::T) {
         __syncthreads();
@@ -479,10 +559,13 @@ __global__ void __launch_bounds__(SH::NT, SH::MINB) k_batch_tile(const BatchInst
     a.inv = d.inv_scale;
     a.x_first = 1;
     a.rules_inside = d.rules_inside;
-    if (RS) {
+    if constexpr (RS) {
+        if (d.rs) {
 #pragma unroll
-        for (int k = 0; k < SH::T; ++k)
-            a.keys[k] = d.rs ? rs_key(d.rs_seed, (unsigned long long)(d.tau0 + unit * SH::T + k)) : 0u;
+            for (int k = 0; k < SH::T; ++k) a.keys[k] = rs_key(d.rs_seed, (unsigned long long)(d.tau0 + unit * SH::T + k));
+            tile_block<SH, true, false>(a, tile_smem, it.x0, it.y0);
+            return;
+        }
     }
-    tile_block<SH, RS, false>(a, tile_smem, it.x0, it.y0);
+    tile_block<SH, false, false>(a, tile_smem, it.x0, it.y0);
 }

@@ -80,15 +80,16 @@ def test_extrapolated_outlet_of_a_custom_geometry():
 @pytest.mark.parametrize("precision,sizes", [
     ("f64", [(257, 160), (401, 310), (2100, 1500)]),
     ("f32", [(257, 160), (700, 200), (1030, 700)]),
-    ("f16", [(401, 160), (1030, 130)]),
-    ("bf16", [(401, 160), (1030, 130)]),
+    ("f16", [(401, 160), (1030, 130), (2100, 1500)]),
+    ("bf16", [(401, 160), (1030, 130), (2100, 1500)]),
+    ("f16r", [(401, 160), (1030, 130), (2100, 1500)]),
+    ("bf16r", [(401, 160), (1030, 130)]),
 ])
 def test_every_tile_shape(precision, sizes):
     for lx, ly in sizes:
         def go(plan):
-            with lbgpu.Lattice(lx, ly, precision, "pull") as lat:
-                if precision in SCALE:
-                    lat.set_offset_scale(SCALE[precision])
+            with lbgpu.Lattice(lx, ly, lbgpu.storage_form(precision)[0], "pull") as lat:
+                lbgpu.configure_storage(lat, precision, 0.03, 9)
                 lat.setup_cylinder(lx // 5 + 1, ly // 2 + 1, ly // 10 + 1, 0.03, 80.0, lbgpu.WALL_REGULARIZED,
                                    lbgpu.OUTLET_CONST)
                 for n in plan:
