@@ -1061,8 +1061,7 @@ __global__ void __launch_bounds__(BX) k_macros(Geo g, int view, const S *__restr
     const int Y = Y0 + blockIdx.y;
     if (X > g.lx) return;
     R f[9];
-#pragma unroll
-    for (int i = 0; i < 9; ++i) f[i] = logical(g, view, cur, other, side, X, Y, i, inv);
+    load_state(g, view, cur, other, side, X, Y, inv, f);
     R r, u, v;
     rules::macros<R>(f, r, u, v);
     const size_t k = (size_t)(Y - Y0) * g.lx + (X - 1);
@@ -1104,29 +1103,44 @@ __global__ void __launch_bounds__(RED_THREADS) k_moments_rows(Geo g, int view, c
 {
     const int Y = blockIdx.x + 1;
     double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int X = 1 + threadIdx.x; X <= g.lx; X += RED_THREADS) {
-        double f[9];
-        bool bad = false;
+    // four nodes' loads in flight a thread, summed in the order of X
+    constexpr int U = sizeof(S) == 8 ? 2 : 4;
+    for (int Xu = 1 + threadIdx.x; Xu <= g.lx; Xu += U * RED_THREADS) {
+        typename Codec<S>::R w[U][9];
+        int tags[U];
 #pragma unroll
-        for (int i = 0; i < 9; ++i) {
-            f[i] = (double)logical(g, view, cur, other, side, X, Y, i, inv);
-            bad |= !isfinite(f[i]);
+        for (int u = 0; u < U; ++u) {
+            const int X = min(Xu + u * RED_THREADS, g.lx);
+            load_state(g, view, cur, other, side, X, Y, inv, w[u]);
+            tags[u] = tag[g.idx(X, Y)];
         }
-        const double rho = ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7])) + f[8];
-        const double jx = (f[1] - f[3]) + (f[5] - f[6]) + (f[8] - f[7]);
-        const double jy = (f[2] - f[4]) + (f[5] - f[8]) + (f[6] - f[7]);
-        acc[0] += rho; acc[1] += jx; acc[2] += jy;
-        acc[6] += bad ? 1.0 : 0.0;
-        const int t = tag[g.idx(X, Y)];
-        if (t == TAG_BGK) {
-            acc[5] += (jx * jx + jy * jy) / (2.0 * rho);
-            acc[7] += rho;
-        } else if (t == TAG_BOUNCE && X >= 2 && X <= g.lx - 1 && Y >= 2 && Y <= g.ly - 1) {
 #pragma unroll
-            for (int i = 1; i < 9; ++i) {
-                if (tag[g.idx(X - cx(i), Y - cy(i))] != TAG_BOUNCE) {
-                    acc[3] += 2.0 * cx(i) * f[i];
-                    acc[4] += 2.0 * cy(i) * f[i];
+        for (int u = 0; u < U; ++u) {
+            const int X = Xu + u * RED_THREADS;
+            if (X > g.lx) break;
+            double f[9];
+            bool bad = false;
+#pragma unroll
+            for (int i = 0; i < 9; ++i) {
+                f[i] = (double)w[u][i];
+                bad |= !isfinite(f[i]);
+            }
+            const double rho = ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7])) + f[8];
+            const double jx = (f[1] - f[3]) + (f[5] - f[6]) + (f[8] - f[7]);
+            const double jy = (f[2] - f[4]) + (f[5] - f[8]) + (f[6] - f[7]);
+            acc[0] += rho; acc[1] += jx; acc[2] += jy;
+            acc[6] += bad ? 1.0 : 0.0;
+            const int t = tags[u];
+            if (t == TAG_BGK) {
+                acc[5] += (jx * jx + jy * jy) / (2.0 * rho);
+                acc[7] += rho;
+            } else if (t == TAG_BOUNCE && X >= 2 && X <= g.lx - 1 && Y >= 2 && Y <= g.ly - 1) {
+#pragma unroll
+                for (int i = 1; i < 9; ++i) {
+                    if (tag[g.idx(X - cx(i), Y - cy(i))] != TAG_BOUNCE) {
+                        acc[3] += 2.0 * cx(i) * f[i];
+                        acc[4] += 2.0 * cy(i) * f[i];
+                    }
                 }
             }
         }
@@ -1174,9 +1188,11 @@ __global__ void __launch_bounds__(BX) k_accumulate_velocity(Geo g, int view, con
     const int X = blockIdx.x * BX + threadIdx.x + 1;
     const int Y = blockIdx.y + 1;
     if (X > g.lx) return;
+    typename Codec<S>::R w[9];
+    load_state(g, view, cur, other, side, X, Y, inv, w);
     double f[9];
 #pragma unroll
-    for (int i = 0; i < 9; ++i) f[i] = (double)logical(g, view, cur, other, side, X, Y, i, inv);
+    for (int i = 0; i < 9; ++i) f[i] = (double)w[i];
     const double rho = ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7])) + f[8];
     const double jx = (f[1] - f[3]) + (f[5] - f[6]) + (f[8] - f[7]);
     const double jy = (f[2] - f[4]) + (f[5] - f[8]) + (f[6] - f[7]);
@@ -1200,9 +1216,11 @@ __global__ void __launch_bounds__(BX) k_velocity_change(Geo g, int view, const S
     const int Y = blockIdx.y + 1;
     float d = 0.0f;
     if (X <= g.lx) {
+        typename Codec<S>::R w[9];
+        load_state(g, view, cur, other, side, X, Y, inv, w);
         double f[9];
 #pragma unroll
-        for (int i = 0; i < 9; ++i) f[i] = (double)logical(g, view, cur, other, side, X, Y, i, inv);
+        for (int i = 0; i < 9; ++i) f[i] = (double)w[i];
         const double rho = ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7])) + f[8];
         const float ux = (float)(((f[1] - f[3]) + (f[5] - f[6]) + (f[8] - f[7])) / rho);
         const float uy = (float)(((f[2] - f[4]) + (f[5] - f[8]) + (f[6] - f[7])) / rho);

@@ -237,6 +237,35 @@ __device__ __forceinline__ S enc_row(const Geo &g, typename Codec<S>::R f, int i
     return Codec<S>::enc(f, i, sc);
 }
 
+// The post-stream state of interior node (X, Y) under a view, decoded: logical() for each slot, but off the
+// perimeter, where every slot has an interior source, nine loads without its tests (one after
+// another with their tests they kept one load in flight a node).
+template <class S>
+__device__ __forceinline__ void load_state(const Geo &g, int view, const S *__restrict__ cur, const S *__restrict__ other,
+                                           const S *__restrict__ side, int X, int Y, float inv,
+                                           typename Codec<S>::R f[9])
+{
+    if (g.perimeter(X, Y)) {
+#pragma unroll
+        for (int i = 0; i < 9; ++i) f[i] = logical(g, view, cur, other, side, X, Y, i, inv);
+        return;
+    }
+    const long long o = g.idx(X, Y);
+    S v[9];
+    if (view == VIEW_PULL_PENDING) {
+#pragma unroll
+        for (int i = 0; i < 9; ++i) v[i] = plane(cur, g, i)[o - cx(i) - (long long)cy(i) * g.pitch];
+    } else if (view == VIEW_AA_SWAPPED) {
+#pragma unroll
+        for (int i = 0; i < 9; ++i) v[i] = plane(cur, g, opp(i))[o - cx(i) - (long long)cy(i) * g.pitch];
+    } else {
+#pragma unroll
+        for (int i = 0; i < 9; ++i) v[i] = plane(cur, g, i)[o];
+    }
+#pragma unroll
+    for (int i = 0; i < 9; ++i) f[i] = dec_row<S>(g, v[i], i, inv, Y);
+}
+
 // A post-collision value of direction i at row Y, as stored in a population plane: with a row
 // shift it is relative to the row that consumes it after streaming, Y + c_iy (stale-slot copies
 // in the side store are consumed by the node itself and stay relative to row Y).
