@@ -399,7 +399,7 @@ __device__ __forceinline__ void regularize_exact(double f[9], int side, double r
 // Any non-BGK rule; (p0, p1) are the node's table entry: (ux, uy) or (rho, uPar).
 // Boundary rules chain to bulk BGK like every function of boundaries.c:171-414.
 template <class T>
-static __device__ __noinline__ void collide_boundary(int t, T f[9], T omega, T p0, T p1)
+__device__ __forceinline__ void boundary_rule(int t, T f[9], T omega, T p0, T p1)
 {
     if (t == TAG_BOUNCE) { bounce(f); return; }
     if (t < TAG_ZOUHE_FIRST || t >= TAG_COUNT) return;
@@ -420,6 +420,12 @@ static __device__ __noinline__ void collide_boundary(int t, T f[9], T omega, T p
     else regularize(f, side, rho, ux, uy);
     if constexpr (sizeof(T) == 8) bgk_exact(f, omega);
     else bgk(f, omega);
+}
+
+template <class T>
+static __device__ __noinline__ void collide_boundary(int t, T f[9], T omega, T p0, T p1)
+{
+    boundary_rule<T>(t, f, omega, p0, p1);
 }
 
 // The boundary rules run out of line on a private copy, so the bulk path's populations stay
