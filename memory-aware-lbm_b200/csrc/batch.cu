@@ -94,6 +94,10 @@ BatchInst describe(const Lattice &L)
     b.buf[0] = L.d.buf[0];
     b.buf[1] = L.d.buf[1];
     b.side = L.d.side;
+    for (int p = 0; p < 2; ++p) {
+        const int slot = L.d.side_slot[p];
+        b.side_of[p] = slot == 3 ? L.d.side_extra : static_cast<char *>(L.d.side) + (size_t)slot * 9 * (size_t)L.d.g.nper * L.elem;
+    }
     b.side_slot[0] = L.d.side_slot[0];
     b.side_slot[1] = L.d.side_slot[1];
     b.tag = L.d.tag;

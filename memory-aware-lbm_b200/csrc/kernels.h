@@ -12,6 +12,7 @@ struct DevLattice {
     int precision;       // LBGPU_F64 / F32 / F16 / BF16: element type of buf and side
     void *buf[2];        // population buffers (buf[1] unused by the AA scheme)
     void *side;          // stale-slot store: slots of [9][nper], two (AA) or three (pull)
+    void *side_extra;    // a fourth slot, of pull lattices with row-shifted offsets
     int side_slot[2];    // the slot of each collision parity
     int ghost_flip;      // 1: the ring that belongs to the second buffer is in the current one (launch_tile)
     int rules_inside;    // some node off the perimeter has a boundary rule
@@ -24,6 +25,14 @@ struct DevLattice {
     double omega;
     float scale, inv_scale;  // FP16/BF16 offset storage: stored = (f - w) * scale
 };
+
+// The k-th slot (0, 1) that holds neither parity's stale slots; slot 3 counts where there is one.
+inline int side_free(const DevLattice &d, int k)
+{
+    for (int s = 0; s < 4; ++s)
+        if (s != d.side_slot[0] && s != d.side_slot[1] && (s < 3 || d.side_extra) && k-- == 0) return s;
+    return -1;
+}
 
 // How the post-stream state is read from a buffer:
 //   VIEW_DIRECT        the buffer holds it (pull form L, or a collided state read as is)
@@ -100,6 +109,7 @@ struct BatchInst {
     Geo g;
     void *buf[2];
     void *side;
+    void *side_of[2];                 // of each collision parity
     int side_slot[2];
     const uint8_t *tag;
     const double *bc;

@@ -334,8 +334,9 @@ int Lattice::step(int nsteps)
 
 void Lattice::after_tile(int T)
 {
-    const int a = (int)((n + 1) & 1);
-    d.side_slot[a] = 3 - d.side_slot[0] - d.side_slot[1];
+    const int a = (int)((n + 1) & 1), prev = side_free(d, 0), last = side_free(d, 1);
+    d.side_slot[a] = prev;
+    if (d.g.shift_u) d.side_slot[1 - a] = last;
     d.ghost_flip ^= 1;
     cur = 1 - cur;
     n += T;

@@ -370,13 +370,12 @@ template <class S> S *OTHER(const DevLattice &d, int cur)
 {
     return d.buf[1] ? static_cast<S *>(d.buf[(1 - cur) ^ d.ghost_flip]) : static_cast<S *>(d.ghost2);
 }
-// The side store of a parity, and (pull lattices) the third slot, which holds neither.
+// The side store's slots: two or three in it, the fourth of row-shifted pull lattices beside it; a parity's.
 template <class S> S *SIDE_SLOT(const DevLattice &d, int slot)
 {
-    return static_cast<S *>(d.side) + (size_t)slot * 9 * (size_t)d.g.nper;
+    return slot == 3 ? static_cast<S *>(d.side_extra) : static_cast<S *>(d.side) + (size_t)slot * 9 * (size_t)d.g.nper;
 }
 template <class S> S *SIDE(const DevLattice &d, int p) { return SIDE_SLOT<S>(d, d.side_slot[p & 1]); }
-template <class S> S *SIDE_FREE(const DevLattice &d) { return SIDE_SLOT<S>(d, 3 - d.side_slot[0] - d.side_slot[1]); }
 
 }  // namespace
 

@@ -21,7 +21,9 @@ namespace {
 //     several blocks a SM: 8192 x 2048 FP64 233 (two blocks of 64 x 16; 236 with four of 32 x 16; single 355), FP32
 //     109 (five of 64 x 12; 111 with six of 64 x 8; single 187), FP16 93 (97 with prefetch; single 109);
 //     16384 x 4096 FP16 342 (single 388), with stochastic rounding 398 (single 398: its hash and
-//     multiplies bind), so those keep k_pull4h from 24M nodes on; 4096 x 1024 31 and 38.
+//     multiplies bind), so those keep k_pull4h from 24M nodes on; 4096 x 1024 31 and 38.  Row-shifted FP16 110 (single
+//     117) at 8192 x 2048, 420 (408) at 16384 x 4096: from 24M nodes too; both together 34.9 (39.4) at 4096 x 1024,
+//     126 (117) at 8192 x 2048: from 8M.
 // Large lattices prefetch the tile 100 (FP64) or 200 (FP32) blocks ahead into L2: 253 -> 233 and 120 -> 109 us;
 // 0.3 of that distance does half as much, 4 times it costs 15-30 % (evicted before it is read).
 using F64Small = TileShape<double, 16, 8, 8, 704, 1>;
@@ -54,7 +56,7 @@ int tile_shape(const DevLattice &d)
     return n < k[0] ? TILE_SMALL : (n < k[1] ? TILE_MID : (n < k[2] ? TILE_WIDE : TILE_LARGE));
 }
 
-template <class SH, bool RS, bool EXTRAP>
+template <class SH, int M, bool EXTRAP>
 void launch_shape(const DevLattice &d, int src, int n_par, int pf, const unsigned *keys, cudaStream_t s)
 {
     using S = typename SH::S;
@@ -68,10 +70,12 @@ void launch_shape(const DevLattice &d, int src, int n_par, int pf, const unsigne
     a.omega = d.omega;
     a.omega_f = (float)d.omega;
     // step 1 reads the stale slots of C_{n-1}; the last step's replace those of C_n, which has them in
-    // its own slots, and the step's before it go to the free slot
+    // its own slots, and the step's before it go to the free slot.  Row-shifted offsets read C_n's from
+    // the side store too (its own slots are rebased), so both go to free slots, of four.
     a.stale1 = SIDE<S>(d, n_par + 1);
-    a.out_last = SIDE<S>(d, n_par);
-    a.out_prev = SIDE_FREE<S>(d);
+    a.stale2 = SIDE<S>(d, n_par);
+    a.out_last = (M & TILE_SHIFT) ? SIDE_SLOT<S>(d, side_free(d, 1)) : SIDE<S>(d, n_par);
+    a.out_prev = SIDE_SLOT<S>(d, side_free(d, 0));
     a.sc = d.scale;
     a.inv = d.inv_scale;
     // the outlet's extrapolation reads three columns back: its tile must not be narrower
@@ -84,22 +88,29 @@ void launch_shape(const DevLattice &d, int src, int n_par, int pf, const unsigne
     a.pf = a.x_first == 1 ? pf : 0;
     a.rules_inside = d.rules_inside;
     for (int k = 0; k < 8; ++k) a.keys[k] = keys[k];
-    cudaFuncSetAttribute(k_tile<SH, RS, EXTRAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SH::SMEM);
-    k_tile<SH, RS, EXTRAP><<<(unsigned)a.nx * (unsigned)a.ny, SH::NT, SH::SMEM, s>>>(a);
+    cudaFuncSetAttribute(k_tile<SH, M, EXTRAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SH::SMEM);
+    k_tile<SH, M, EXTRAP><<<(unsigned)a.nx * (unsigned)a.ny, SH::NT, SH::SMEM, s>>>(a);
 }
 
 template <class SH>
 void launch_one(const DevLattice &d, int src, int n_par, bool outlet, int pf, const unsigned *keys, cudaStream_t s)
 {
     if constexpr (sizeof(typename SH::S) == 2) {
+        if constexpr (SH::T < 8) {
+            if (d.g.shift_u) {
+                if (keys[0] != 0) launch_shape<SH, TILE_RS | TILE_SHIFT, false>(d, src, n_par, pf, keys, s);
+                else launch_shape<SH, TILE_SHIFT, false>(d, src, n_par, pf, keys, s);
+                return;
+            }
+        }
         if (keys[0] != 0) {
-            if (outlet) launch_shape<SH, true, true>(d, src, n_par, pf, keys, s);
-            else launch_shape<SH, true, false>(d, src, n_par, pf, keys, s);
+            if (outlet) launch_shape<SH, TILE_RS, true>(d, src, n_par, pf, keys, s);
+            else launch_shape<SH, TILE_RS, false>(d, src, n_par, pf, keys, s);
             return;
         }
     }
-    if (outlet) launch_shape<SH, false, true>(d, src, n_par, pf, keys, s);
-    else launch_shape<SH, false, false>(d, src, n_par, pf, keys, s);
+    if (outlet) launch_shape<SH, 0, true>(d, src, n_par, pf, keys, s);
+    else launch_shape<SH, 0, false>(d, src, n_par, pf, keys, s);
 }
 
 template <class S>
@@ -117,9 +128,10 @@ int tile_steps(const DevLattice &d, long long steps, bool outlet, bool rs)
     if (steps < 2 || (outlet && !d.outlet_tiles)) return 0;
     const int shape = tile_shape(d);
     if (d.precision == LBGPU_F16 || d.precision == LBGPU_BF16) {
-        if (d.g.shift_u) return 0;          // row-shifted offsets are rebased between rows
-        if (rs && (long long)d.g.lx * d.g.ly >= (24ll << 20)) return 0;
-        return shape == TILE_SMALL && steps >= 8 ? 8 : (steps >= 4 && shape != TILE_LARGE ? 4 : 2);
+        if (d.g.shift_u && (outlet || !d.side_extra)) return 0;
+        const long long nodes = (long long)d.g.lx * d.g.ly;
+        if (nodes >= ((rs && d.g.shift_u ? 8ll : 24ll) << 20) && (rs || d.g.shift_u)) return 0;
+        return shape == TILE_SMALL && steps >= 8 && !d.g.shift_u ? 8 : (steps >= 4 && shape != TILE_LARGE ? 4 : 2);
     }
     if (shape == TILE_SMALL && steps >= 8) return 8;
     if (steps >= 4 && (shape <= TILE_MID || (shape == TILE_WIDE && d.precision == LBGPU_F32))) return 4;

@@ -40,6 +40,9 @@ struct TileShape {
     static_assert(W % 2 == 0 && T % 2 == 0, "pairs of nodes");
 };
 
+// Modes of 16-bit storage (M): stochastic rounding, row-shifted offsets.
+enum { TILE_RS = 1, TILE_SHIFT = 2 };
+
 template <class S>
 struct TileArgs {
     Geo g;
@@ -50,6 +53,7 @@ struct TileArgs {
     const int *zgb;            // [nb] of the right pressure table: >= 0 where the outlet is extrapolated
     double omega;
     const S *stale1;           // stale slots of C_{n-1}, read by step 1
+    const S *stale2;           // and of C_n, by step 2 (row-shifted offsets: the planes' are rebased)
     S *out_last, *out_prev;    // where the stale slots of C_{n+T} and C_{n+T-1} go
     float sc, inv, omega_f;
     int x_first;               // column of the first tile (1, or less, see launch_tile)
@@ -101,16 +105,17 @@ __device__ __forceinline__ void stale_slots(const Geo &g, int X, int Y, FN fn)
 // node streams into hold the node's own value of two steps before): each lies in the ghost cell
 // that a gather reads for it, which no other node reads or writes, in the buffer that step s + 2
 // reads; after the last two steps they also go to the side store.
-template <class S, class SH, int s, bool EDGE, bool RS>
+template <class S, class SH, int s, bool EDGE, int M>
 __device__ __forceinline__ void tile_store(const TileArgs<S> &a, const typename Work<S>::W f[9], S *__restrict__ rd,
                                            S *__restrict__ wr, S *const gd[9], unsigned go, int X, int Y, int q, bool owned)
 {
     const Geo &g = a.g;
     constexpr int RW = SH::RW, PL = SH::PL;
+    constexpr bool RS = (M & TILE_RS) != 0, SHIFT = (M & TILE_SHIFT) != 0;
     const RsNode h = rs_node<S, RS>(g, a.keys[s - 1], X, Y);
     S v[9];
 #pragma unroll
-    for (int i = 0; i < 9; ++i) v[i] = put<S, RS>(f[i], i, a.sc, h);
+    for (int i = 0; i < 9; ++i) v[i] = put<S, RS>(stored_out<S, SHIFT ? 1 : 0>(g, Y, i, f[i], a.sc), i, a.sc, h);
     if (s == SH::T) {
 #pragma unroll
         for (int i = 0; i < 9; ++i) *reinterpret_cast<S *>(reinterpret_cast<char *>(gd[i]) + go) = v[i];
@@ -124,14 +129,15 @@ __device__ __forceinline__ void tile_store(const TileArgs<S> &a, const typename 
         stale_slots(g, X, Y, [&](int i) {
             const int dx = (i == 1 || i == 5 || i == 8) ? 1 : ((i == 3 || i == 6 || i == 7) ? -1 : 0);
             const int dy = (i == 2 || i == 5 || i == 6) ? 1 : ((i == 4 || i == 7 || i == 8) ? -1 : 0);
-            S w = v[0];
+            S w = v[0];                 // (relative to the node's own row: it is the one that reads it)
 #pragma unroll
-            for (int j = 1; j < 9; ++j) if (i == j) w = v[j];
+            for (int j = 1; j < 9; ++j) if (i == j) w = SHIFT ? put<S, RS>(f[j], j, a.sc, h) : v[j];
             const bool in = c - dx >= 0 && c - dx < RW && r - dy >= 0 && r - dy < SH::RH;
             // the ghost cell that feeds this slot at step s + 2
             if (s + 2 <= SH::T && in) rd[i * PL + q - dy * RW - dx] = w;
             // and at step 2, which reads C_n
-            if (s == 1 && in) wr[i * PL + q - dy * RW - dx] = a.src[(size_t)i * (size_t)g.plane + g.idx(X, Y)];
+            if (s == 1 && in) wr[i * PL + q - dy * RW - dx] =
+                SHIFT ? a.stale2[(size_t)i * g.nper + p] : a.src[(size_t)i * (size_t)g.plane + g.idx(X, Y)];
             if (s == SH::T) a.out_last[(size_t)i * g.nper + p] = w;
             if (s == SH::T - 1 && owned) a.out_prev[(size_t)i * g.nper + p] = w;
         });
@@ -155,7 +161,7 @@ __device__ __forceinline__ double tile_density(const TileArgs<S> &a, const S *__
 }
 
 // The boundary rules (tags of 3 and more) at one node.
-template <class S, class SH, int s, bool EXTRAP>
+template <class S, class SH, int s, int M, bool EXTRAP>
 __device__ __forceinline__ void tile_boundary(const TileArgs<S> &a, const S *__restrict__ rd, int t, int X, int Y, int q,
                                               typename Work<S>::W f[9])
 {
@@ -172,14 +178,18 @@ __device__ __forceinline__ void tile_boundary(const TileArgs<S> &a, const S *__r
         node_params(a.bc, g, t, X, Y, p0, p1);
         rules::boundary_rule<double>(t, f, a.omega, p0, p1);
     } else {
-        collide_w<S, 0>(a.bc, g, t, X, Y, f, a.omega, a.sc, a.inv);
+        collide_w<S, (M & TILE_SHIFT) ? 1 : 0>(a.bc, g, t, X, Y, f, a.omega, a.sc, a.inv);
     }
 }
 
 // Bulk, bounce-back and rule-less nodes.
-template <class S>
-__device__ __forceinline__ void tile_bulk(const TileArgs<S> &a, int t, typename Work<S>::W f[9])
+template <class S, int M>
+__device__ __forceinline__ void tile_bulk(const TileArgs<S> &a, int t, int X, int Y, typename Work<S>::W f[9])
 {
+    if constexpr ((M & TILE_SHIFT) != 0) {
+        collide_w<S, 1>(a.bc, a.g, t, X, Y, f, a.omega, a.sc, a.inv);
+        return;
+    }
     if constexpr (sizeof(S) == 2) {
         if (t == TAG_BGK) {
             bgk_offsets<false>(f, a.omega_f, a.sc, a.inv, 0.0f);
@@ -203,7 +213,7 @@ __device__ __forceinline__ void tile_bulk(const TileArgs<S> &a, int t, typename 
 // false and skip the tests of lattice bounds.  Nodes with boundary rules (250-500 operations, mostly one after
 // another) are listed at step 1 and run packed in warps of their own beside the others: left in
 // their places, one or two lanes of every row's warp would hold the whole warp that long.
-template <class S, class SH, int s, bool EDGE, bool RS, bool EXTRAP>
+template <class S, class SH, int s, bool EDGE, int M, bool EXTRAP>
 __device__ __forceinline__ void tile_step(const TileArgs<S> &a, S *__restrict__ sm, uint8_t *__restrict__ stag,
                                           unsigned short *__restrict__ list, int *__restrict__ nlist, int x0, int y0)
 {
@@ -261,8 +271,8 @@ __device__ __forceinline__ void tile_step(const TileArgs<S> &a, S *__restrict__ 
             for (int i = 0; i < 9; ++i) wr[i * PL + q] = Work<S>::store(f[i], i, a.sc);
             continue;
         }
-        tile_bulk<S>(a, t, f);
-        tile_store<S, SH, s, EDGE, RS>(a, f, rd, wr, gd, go, X, Y, q, c >= E && c < WS - E && r >= E && r < HS - E);
+        tile_bulk<S, M>(a, t, X, Y, f);
+        tile_store<S, SH, s, EDGE, M>(a, f, rd, wr, gd, go, X, Y, q, c >= E && c < WS - E && r >= E && r < HS - E);
     }
     if (EDGE) {
         if (s == 1) __syncthreads();
@@ -279,8 +289,8 @@ __device__ __forceinline__ void tile_step(const TileArgs<S> &a, S *__restrict__ 
 #pragma unroll
             for (int i = 0; i < 9; ++i)
                 f[i] = Work<S>::load(s == 1 ? wr[i * PL + q] : rd[i * PL + q - cy(i) * RW - cx(i)], i, a.inv);
-            tile_boundary<S, SH, s, EXTRAP>(a, rd, t, X, Y, q, f);
-            tile_store<S, SH, s, EDGE, RS>(a, f, rd, wr, gd, (unsigned)(r - O) * pitch + (unsigned)(c - O) * (unsigned)sizeof(S), X, Y, q,
+            tile_boundary<S, SH, s, M, EXTRAP>(a, rd, t, X, Y, q, f);
+            tile_store<S, SH, s, EDGE, M>(a, f, rd, wr, gd, (unsigned)(r - O) * pitch + (unsigned)(c - O) * (unsigned)sizeof(S), X, Y, q,
                                            c >= SH::T - 1 && c < RW - (SH::T - 1) && r >= SH::T - 1 && r < SH::RH - (SH::T - 1));
         }
     }
@@ -421,13 +431,48 @@ __device__ __forceinline__ void bgk_offsets_pair(float2 D[9], float omega, float
 #undef LBGPU_PAIR2
 }
 
+// bgk_offsets<true> on two nodes of a row.
+__device__ __forceinline__ void bgk_offsets_pair_shifted(float2 D[9], float omega, float sc, float inv, float us)
+{
+    const float2 sum = add2(add2(add2(add2(D[0], D[1]), add2(D[2], D[3])), add2(add2(D[4], D[5]), add2(D[6], D[7]))), D[8]);
+    const float2 d = mul2(c2(inv), sum);
+    const float2 Jx = add2(add2(sub2(D[1], D[3]), sub2(D[5], D[6])), sub2(D[8], D[7]));
+    const float2 Jy = add2(add2(sub2(D[2], D[4]), sub2(D[5], D[8])), sub2(D[6], D[7]));
+    const float2 ir = make_float2(__fdividef(1.0f, 1.0f + d.x), __fdividef(1.0f, 1.0f + d.y));
+    const float2 q = mul2(c2(inv), ir);
+    const float2 ux = fma2(Jx, q, mul2(c2(us), ir)), uy = mul2(Jy, q);
+    const float2 t = sub2(ux, c2(us));
+    const float2 A = fma2(c2(-1.5f * us), t, fma2(c2(-1.5f * inv), fma2(Jx, ux, mul2(Jy, uy)), d));
+    const float2 ux45 = mul2(c2(4.5f * inv), ux), uy45 = mul2(c2(4.5f * inv), uy);
+    const float hs = 4.5f * us;
+    const float2 A1 = fma2(c2(hs), t, A), ev = mul2(c2(hs), uy);
+    const float2 A5 = add2(A1, ev), A6 = sub2(A1, ev);
+    const float om1 = 1.0f - omega;
+    const float k0 = omega * sc * (4.f / 9.f), k1 = omega * sc * (1.f / 9.f), k2 = omega * sc * (1.f / 36.f);
+    const float b1 = (3.0f * inv) * k1, b2 = (3.0f * inv) * k2;
+    D[0] = fma2(c2(om1), D[0], mul2(c2(k0), A));
+#define LBGPU_PAIR2S(I, J, K, B, CU45, CJ, AP)                        \
+    {                                                                 \
+        const float2 cj = (CJ);                                       \
+        const float2 a = mul2(c2(K), fma2(CU45, cj, AP)), b = mul2(c2(B), cj); \
+        D[I] = fma2(c2(om1), D[I], add2(a, b));                       \
+        D[J] = fma2(c2(om1), D[J], sub2(a, b));                       \
+    }
+    LBGPU_PAIR2S(1, 3, k1, b1, ux45, Jx, A1)
+    LBGPU_PAIR2S(2, 4, k1, b1, uy45, Jy, A)
+    LBGPU_PAIR2S(5, 7, k2, b2, add2(ux45, uy45), add2(Jx, Jy), A5)
+    LBGPU_PAIR2S(6, 8, k2, b2, sub2(uy45, ux45), sub2(Jy, Jx), A6)
+#undef LBGPU_PAIR2S
+}
+
 // Step s of a tile that holds no perimeter node and no boundary rule, two nodes a thread (FP32 and 16-bit).
 // The pairs of step s start at column x0 - (T - s): a step later they start one column on, so the
 // two populations that a pair takes from x - 1 or x + 1 were stored (or, T being even, lie in the
 // planes) as one pair, and only those of the three directions along y are read one by one.
-template <class S, class SH, int s, bool RS>
+template <class S, class SH, int s, int M>
 __device__ __forceinline__ void tile_step_pairs(const TileArgs<S> &a, S *__restrict__ sm, uint8_t *__restrict__ stag, int x0, int y0)
 {
+    constexpr bool RS = (M & TILE_RS) != 0, SHIFT = (M & TILE_SHIFT) != 0;
     constexpr int E = SH::T - s, WP = (SH::W + 2 * E) / 2, HS = SH::H + 2 * E, O = s - 1, RW = SH::RW, PL = SH::PL;
     const Geo &g = a.g;
     const S *rd = sm + (size_t)(s & 1) * (SH::NBUF - 1) * SH::B1;
@@ -459,18 +504,25 @@ __device__ __forceinline__ void tile_step_pairs(const TileArgs<S> &a, S *__restr
                 f[i] = cx(i) != 0 ? pair_load(p + (i * PL - cy(i) * RW - cx(i))) : pair_gather(p + (i * PL - cy(i) * RW));
         }
         if (t == 0x0101u) {
-            if constexpr (sizeof(S) == 2) bgk_offsets_pair(f, a.omega_f, a.sc, a.inv);
+            if constexpr (SHIFT) bgk_offsets_pair_shifted(f, a.omega_f, a.sc, a.inv, g.shift_u[y0 - E + r]);
+            else if constexpr (sizeof(S) == 2) bgk_offsets_pair(f, a.omega_f, a.sc, a.inv);
             else bgk_pair(f, a.omega_f);
         } else {
             float h[9];
 #pragma unroll
             for (int i = 0; i < 9; ++i) h[i] = f[i].x;
-            tile_bulk<S>(a, (int)(t & 0xffu), h);
+            tile_bulk<S, M>(a, (int)(t & 0xffu), x0 - E + 2 * c, y0 - E + r, h);
 #pragma unroll
             for (int i = 0; i < 9; ++i) { f[i].x = h[i]; h[i] = f[i].y; }
-            tile_bulk<S>(a, (int)(t >> 8), h);
+            tile_bulk<S, M>(a, (int)(t >> 8), x0 - E + 2 * c + 1, y0 - E + r, h);
 #pragma unroll
             for (int i = 0; i < 9; ++i) f[i].y = h[i];
+        }
+        if (SHIFT && g.shift_rebased(y0 - E + r)) {
+            const float *rebase = g.shift_rebase(y0 - E + r);
+#pragma unroll
+            for (int i = 0; i < 9; ++i)
+                if (cy(i) != 0) f[i] = add2(f[i], mul2(c2(rebase[i]), c2(a.sc)));
         }
         constexpr bool SPLIT = (E & 1) != 0;              // x0 is odd: X = x0 - E + 2 c is even
         PairBits<SPLIT> b = {};
@@ -487,20 +539,20 @@ __device__ __forceinline__ void tile_step_pairs(const TileArgs<S> &a, S *__restr
     }
 }
 
-template <class S, class SH, int s, bool EDGE, bool RS, bool EXTRAP>
+template <class S, class SH, int s, bool EDGE, int M, bool EXTRAP>
 __device__ __forceinline__ void tile_steps(const TileArgs<S> &a, S *sm, uint8_t *stag, unsigned short *list, int *nlist,
                                            int x0, int y0)
 {
-    if constexpr (!EDGE && sizeof(S) <= 4) tile_step_pairs<S, SH, s, RS>(a, sm, stag, x0, y0);
-    else tile_step<S, SH, s, EDGE, RS, EXTRAP>(a, sm, stag, list, nlist, x0, y0);
+    if constexpr (!EDGE && sizeof(S) <= 4) tile_step_pairs<S, SH, s, M>(a, sm, stag, x0, y0);
+    else tile_step<S, SH, s, EDGE, M, EXTRAP>(a, sm, stag, list, nlist, x0, y0);
     if constexpr (s < SH::T) {
         __syncthreads();
-        tile_steps<S, SH, s + 1, EDGE, RS, EXTRAP>(a, sm, stag, list, nlist, x0, y0);
+        tile_steps<S, SH, s + 1, EDGE, M, EXTRAP>(a, sm, stag, list, nlist, x0, y0);
     }
 }
 
 // The T steps of the tile at (x0, y0) by one block.
-template <class SH, bool RS, bool EXTRAP>
+template <class SH, int M, bool EXTRAP>
 __device__ __forceinline__ void tile_block(const TileArgs<typename SH::S> &a, unsigned char *smem, int x0, int y0)
 {
     using S = typename SH::S;
@@ -511,15 +563,15 @@ __device__ __forceinline__ void tile_block(const TileArgs<typename SH::S> &a, un
     constexpr int E = SH::T - 1;
     const bool inside = !a.rules_inside && x0 - E >= 2 && x0 + SH::W - 1 + E <= a.g.lx - 1 && y0 - E >= 2 && y0 + SH::H - 1 + E <= a.g.ly - 1;
     if (inside) {
-        tile_steps<S, SH, 1, false, RS, EXTRAP>(a, sm, stag, list, nlist, x0, y0);
+        tile_steps<S, SH, 1, false, M, EXTRAP>(a, sm, stag, list, nlist, x0, y0);
     } else {
         if (threadIdx.x == 0) *nlist = 0;
         __syncthreads();
-        tile_steps<S, SH, 1, true, RS, EXTRAP>(a, sm, stag, list, nlist, x0, y0);
+        tile_steps<S, SH, 1, true, M, EXTRAP>(a, sm, stag, list, nlist, x0, y0);
     }
 }
 
-template <class SH, bool RS, bool EXTRAP>
+template <class SH, int M, bool EXTRAP>
 __global__ void __launch_bounds__(SH::NT, SH::MINB) k_tile(const __grid_constant__ TileArgs<typename SH::S> a)
 {
     extern __shared__ __align__(16) unsigned char tile_smem[];
@@ -533,7 +585,7 @@ __global__ void __launch_bounds__(SH::NT, SH::MINB) k_tile(const __grid_constant
     }
     int tx, ty;
     tile_place(blockIdx.x, a.nx, a.ny, a.ring_first, tx, ty);
-    tile_block<SH, RS, EXTRAP>(a, tile_smem, a.x_first + tx * SH::W, 1 + ty * SH::H);
+    tile_block<SH, M, EXTRAP>(a, tile_smem, a.x_first + tx * SH::W, 1 + ty * SH::H);
 }
 
 // T steps of every tile of a batch's work list (x0, y0: the tile's first node): launch `unit` of a
@@ -570,9 +622,9 @@ __global__ void __launch_bounds__(SH::NT, SH::MINB) k_batch_tile(const BatchInst
         if (d.rs) {
 #pragma unroll
             for (int k = 0; k < SH::T; ++k) a.keys[k] = rs_key(d.rs_seed, (unsigned long long)(d.tau0 + unit * SH::T + k));
-            tile_block<SH, true, false>(a, tile_smem, it.x0, it.y0);
+            tile_block<SH, 1, false>(a, tile_smem, it.x0, it.y0);
             return;
         }
     }
-    tile_block<SH, false, false>(a, tile_smem, it.x0, it.y0);
+    tile_block<SH, 0, false>(a, tile_smem, it.x0, it.y0);
 }

@@ -18,18 +18,20 @@ def make(size, precision, scheme):
     st = O.random_boundary_lattice(size[0], size[1], seed=size[0] + 3 * size[1])
     if size[0] > 20:
         st.tag[20, 5] = 14     # a boundary rule off the perimeter
-    base, _, rs = lbgpu.storage_form(precision)
+    base, shift, rs = lbgpu.storage_form(precision)
     lat = lbgpu.Lattice(st.lx, st.ly, base, scheme)
     if base == "f16":
         lat.set_offset_scale(10)
     if rs and size[0] != 65:       # and one member that rounds to nearest
         lat.set_stochastic_rounding(True, size[0])
+    if shift:
+        lat.set_offset_shift(lbgpu.shift_profile(shift, size[1], 0.03))
     lat.set_geometry(st.omega, st.tag, st.bc, st.zgb)
     lat.set_populations(st.lat, st.tmp)
     return lat
 
 
-@pytest.mark.parametrize("precision", ["f64", "f32", "f16", "f16r"])
+@pytest.mark.parametrize("precision", ["f64", "f32", "f16", "f16r", "f16sr"])
 @pytest.mark.parametrize("plan", PLANS)
 def test_members_equal_single_steps(precision, plan):
     kinds = [(s, "pull") for s in SIZES] + [((70, 20), "aa")]
