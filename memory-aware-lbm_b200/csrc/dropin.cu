@@ -56,6 +56,7 @@ struct DropIn {
     void *scratch_mem = nullptr;
     double *scratch = nullptr;
     bool ahead = false;
+    bool ahead_there = false;   // they are in the node array itself
     bool tmp_is_stream = false; // tmpLattice holds the stream of lattice (collide_with_stream)
     int sync_mode = LB_SYNC_OUTLET;
     bool pinned[3] = {false, false, false};         // host arrays, then the dynamics pointers
@@ -336,10 +337,9 @@ DropIn *prepare(Simulation *sim, const char *fn, bool tables = true, bool stream
     return c;
 }
 
-// The GPU's address of the pinned host array that sim->lattice points to, or null.
-double *mapped_lattice(Simulation *sim, DropIn *c)
+// The GPU's address of a host node array where it is pinned, or null.
+double *mapped_array(DropIn *c, Node *host)
 {
-    Node *host = chunk_of(sim->lattice);
     for (int k = 0; k < 2; ++k)
         if (c->pinned[k] && c->pinned_ptr[k] == host) {
             void *dev = nullptr;
@@ -371,9 +371,14 @@ void finish(Simulation *sim, DropIn *c, bool collided = false)
         L.readout_records(reinterpret_cast<double *>(host + (size_t)X0 * col), 10, c->dynp_dev, X0, X1);
         return;
     }
-    double *const dev = mapped_lattice(sim, c), *out = dev ? dev + (size_t)X0 * col * 10 : c->scratch;
+    double *const dev = mapped_array(c, host), *out = dev ? dev + (size_t)X0 * col * 10 : c->scratch;
+    c->ahead_there = false;
     if (collided && L.form == lbgpu::FORM_C && !L.pending) {
-        lbgpu::launch_readout_both(L.d, L.cur, (int)((L.n + 1) & 1), X0, X1, out, c->scratch + scratch_cols(sim), 10, c->dynp_dev, L.stream);
+        // those of the stream into the array that the stream's call will swap in, where that is pinned
+        double *const next = mapped_array(c, chunk_of(sim->tmpLattice));
+        c->ahead_there = next != nullptr;
+        lbgpu::launch_readout_both(L.d, L.cur, (int)((L.n + 1) & 1), X0, X1, out,
+                                   next ? next + (size_t)X0 * col * 10 : c->scratch + scratch_cols(sim), 10, c->dynp_dev, L.stream);
         L.d2h_bytes += (size_t)(X1 - X0) * col * sizeof(Node);
     } else {
         int v, par;
@@ -394,8 +399,9 @@ bool finish_ahead(Simulation *sim, DropIn *c)
     if (!c->ahead || c->sync_mode != LB_SYNC_OUTLET || c->dynp_dirty) return false;
     const size_t col = (size_t)(sim->ly + 2);
     const int X0 = sim->lx >= 2 ? sim->lx - 2 : 0;
-    std::memcpy(static_cast<void *>(chunk_of(sim->lattice) + (size_t)X0 * col), c->scratch + scratch_cols(sim),
-                (size_t)(sim->lx - X0) * col * sizeof(Node));
+    if (!c->ahead_there)
+        std::memcpy(static_cast<void *>(chunk_of(sim->lattice) + (size_t)X0 * col), c->scratch + scratch_cols(sim),
+                    (size_t)(sim->lx - X0) * col * sizeof(Node));
     c->ahead = false;
     return true;
 }
