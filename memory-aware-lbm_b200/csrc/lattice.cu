@@ -307,9 +307,13 @@ int Lattice::step(int nsteps)
 {
     if (nsteps < 0) return set_error(LB_ERR_ARG, "negative step count");
     launches = 0;
+    // While the caller captures the stream, steps stay single: an even number of them leaves the buffers where
+    // it found them, so the caller's graph can be replayed; a tile launch turns them over.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (nsteps > 1) LB_CUDA(cudaStreamIsCapturing(stream, &capture), "cudaStreamIsCapturing");
     for (int s = 0; s < nsteps; ++s) {
         // a run of pull steps: several a launch, the state as single steps leave it
-        if (scheme == LBGPU_PULL && !ghosts && form == FORM_C && pending) {
+        if (scheme == LBGPU_PULL && !ghosts && form == FORM_C && pending && capture == cudaStreamCaptureStatusNone) {
             if (const int T = tile_steps(d, nsteps - s, zgb_each_step, rs)) {
                 unsigned keys[8] = {0};
                 for (int k = 0; rs && k < T; ++k) keys[k] = rs_key(rs_seed, (unsigned long long)(n + 1 + k));

@@ -147,3 +147,27 @@ def test_row_shift_set_and_cleared_between_runs():
 
     for a, b in zip(go([[3], [9], [2]]), go([[1] * 3, [1] * 9, [1] * 2])):
         assert same(a, b)
+
+
+def test_steps_in_a_captured_graph_replay():
+    """A caller that captures an even number of steps on the lattice's stream can replay them."""
+    import torch
+
+    def channel():
+        lat = lbgpu.Lattice(150, 41, "f64", "pull")
+        lat.setup_cylinder(31, 21, 5, 0.03, 60.0, lbgpu.WALL_BOUNCEBACK, lbgpu.OUTLET_CONST)
+        lat.step(5)
+        lat.synchronize()
+        return lat
+
+    torch.zeros(1, device="cuda")
+    with channel() as lat, channel() as ref:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=torch.cuda.ExternalStream(lat.stream), capture_error_mode="thread_local"):
+            lat.step(4)
+        for _ in range(3):
+            graph.replay()
+        torch.cuda.synchronize()
+        ref.step(12)
+        assert same(lat.populations(), ref.populations())
+        del graph
