@@ -59,6 +59,7 @@ struct DropIn {
     bool ahead_there = false;   // they are in the node array itself
     bool tmp_is_stream = false; // tmpLattice holds the stream of lattice (collide_with_stream)
     int sync_mode = LB_SYNC_OUTLET;
+    bool pin_tried = false;
     bool pinned[3] = {false, false, false};         // host arrays, then the dynamics pointers
     void *pinned_ptr[3] = {nullptr, nullptr, nullptr};
     std::vector<uint64_t> dynp;          // host Dynamics* of every node, [X*(ly+2)+Y]
@@ -250,7 +251,8 @@ constexpr size_t kPinBytes = (size_t)64 << 20;
 
 void pin_host(Simulation *sim, DropIn *c)
 {
-    if (!pinning_allowed()) return;
+    if (c->pin_tried || !pinning_allowed()) return;
+    c->pin_tried = true;
     const size_t nodes = (size_t)(sim->lx + 2) * (sim->ly + 2);
     // the dynamics pointers too: the first read-out uploads them (the vector never reallocates)
     void *chunks[3] = {sim->memoryChunk, sim->tmpMemoryChunk, c->dynp.data()};

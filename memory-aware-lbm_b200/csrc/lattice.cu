@@ -88,8 +88,11 @@ void memory_drop()
 {
     std::lock_guard<std::mutex> lock(g_mem_mu);
     if (--g_lattices > 0) return;
-    for (cudaMemPool_t pool : g_pool)
-        if (pool) cudaMemPoolTrimTo(pool, 0);
+    for (cudaMemPool_t &pool : g_pool)     // (destroyed, not trimmed: a device reset in between is then harmless)
+        if (pool) {
+            cudaMemPoolDestroy(pool);
+            pool = nullptr;
+        }
     read_back_release();
 }
 

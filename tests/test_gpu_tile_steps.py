@@ -57,6 +57,16 @@ def test_every_boundary_rule_anywhere(precision, size):
         assert same(got, exp), describe_diff(got, exp)
 
 
+@pytest.mark.parametrize("precision", ["f64", "f32", "f16"])
+@pytest.mark.parametrize("size", [(1, 1), (1, 9), (9, 1), (2, 2), (2, 17), (3, 3), (18, 2)])
+def test_lattices_narrower_than_their_perimeter(precision, size):
+    """One or two rows or columns: nodes with several sides at once, no interior at all."""
+    st = O.random_boundary_lattice(size[0], size[1], seed=size[0] + 40 * size[1])
+    got = agree(st, precision, [1, 2, 11])
+    if precision == "f64":
+        assert same(got, O.run(st, 14).lat)
+
+
 # one and two columns past a multiple of every tile width, and a width below four columns
 @pytest.mark.parametrize("precision", ["f64", "f32", "f16", "bf16"])
 @pytest.mark.parametrize("size", [(17, 12), (34, 11), (65, 23), (130, 31), (67, 29)])
