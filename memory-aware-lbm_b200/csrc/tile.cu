@@ -12,7 +12,9 @@ namespace {
 // The shapes by storage type and node count, from a sweep of about ten shapes over channels of 250 x 51 to 8192 x
 // 2048 (us a step in a graph of launches; the next best shape or the single-step kernel in parentheses):
 //   small lattices: many steps a launch on small tiles, so that every SM has a tile and the launch is
-//     shared: FP64 250 x 51 2.4 (4 steps 2.8, single 3.5), FP32 1.5 (1.9, 3.3), FP16 1.9 (2.2, 6.7)
+//     shared: FP64 250 x 51 2.4 (4 steps 2.8, single 3.5), FP32 1.5 (1.9, 3.3), FP16 2.0 (2.2, 6.7)
+//     (to 19K nodes, a tile a SM; FP16 1.8 on 704 threads); 400 x 90: FP64 3.1 with 4 steps (4.0 with 8), FP32
+//     2.1 with two tiles a SM (2.5 with one), FP16 2.2 (2.6)
 //   511 x 127: FP64 3.8 (5.0 with 2 steps, single 4.0), FP32 2.5 (2.6 with 8 steps, single 3.5)
 //   700 x 200: FP64 5.4 (5.6 with 2 steps), FP32 2.9 (3.2 on 32 x 8 tiles, single 4.3), FP16 3.4 (3.5 on 416 threads, single 7.2)
 //   1024 x 256: FP64 7.4 (8.3 with 4 steps, single 7.0 in a graph and 9.0 launched), FP32 4.2 (5.2 with 2, 5.5)
@@ -31,6 +33,7 @@ using F64Mid = TileShape<double, 32, 8, 4, 288, 2>;
 using F64Wide = TileShape<double, 32, 8, 2, 352, 3>;
 using F64Large = TileShape<double, 64, 16, 2, 512, 2>;
 using F32Small = TileShape<float, 16, 8, 8, 768, 1>;
+using F32Small2 = TileShape<float, 16, 8, 8, 384, 2>;
 using F32Mid = TileShape<float, 32, 8, 4, 288, 3>;
 using F32Wide = TileShape<float, 32, 16, 4, 448, 2>;
 using F32Large = TileShape<float, 64, 12, 2, 224, 5>;
@@ -38,16 +41,19 @@ using F32Large = TileShape<float, 64, 12, 2, 224, 5>;
 // with FP64's in halves because members are small (71 against 72 GLUPS on one large lattice).
 using F64Batch = TileShape<double, 32, 16, 2, 256, 4>;
 using F32Batch = F32Large;
-template <class S> using HalfSmall = TileShape<S, 16, 8, 8, 384, 2>;
+template <class S> using HalfSmall = TileShape<S, 16, 8, 8, 704, 1>;
+template <class S> using HalfSmall2 = TileShape<S, 16, 8, 8, 384, 2>;
 template <class S> using HalfWide = TileShape<S, 32, 16, 4, 448, 3>;
 template <class S> using HalfLarge = TileShape<S, 64, 12, 2, 224, 5>;
 
 enum { TILE_SMALL = 0, TILE_MID = 1, TILE_WIDE = 2, TILE_LARGE = 3, TILE_NONE = 4 };
 
 // Node counts below which a shape is the fastest.
-constexpr long long kF64[3] = {40 << 10, 120 << 10, 3 << 20};
-constexpr long long kF32[3] = {40 << 10, 100 << 10, 700 << 10};
+constexpr long long kF64[3] = {19 << 10, 120 << 10, 3 << 20};
+constexpr long long kF32[3] = {52 << 10, 100 << 10, 700 << 10};
 constexpr long long kHalf[3] = {60 << 10, 60 << 10, 2 << 20};
+// Up to here the small tiles (128 nodes) are one a SM, and take all its threads; beyond, two share one.
+constexpr long long kOneASm = 148 * 128;
 
 int tile_shape(const DevLattice &d)
 {
@@ -116,7 +122,8 @@ void launch_one(const DevLattice &d, int src, int n_par, bool outlet, int pf, co
 template <class S>
 void launch_half(const DevLattice &d, int src, int n_par, int T, bool outlet, const unsigned *keys, cudaStream_t s)
 {
-    if (T == 8) launch_one<HalfSmall<S>>(d, src, n_par, outlet, 0, keys, s);
+    if (T == 8 && (long long)d.g.lx * d.g.ly <= kOneASm) launch_one<HalfSmall<S>>(d, src, n_par, outlet, 0, keys, s);
+    else if (T == 8) launch_one<HalfSmall2<S>>(d, src, n_par, outlet, 0, keys, s);
     else if (T == 4) launch_one<HalfWide<S>>(d, src, n_par, outlet, 0, keys, s);
     else launch_one<HalfLarge<S>>(d, src, n_par, outlet, 0, keys, s);
 }
@@ -149,7 +156,8 @@ void launch_tile(const DevLattice &d, int src, int n_par, int T, bool outlet, co
         else launch_one<F64Wide>(d, src, n_par, outlet, 0, keys, s);
         break;
     case LBGPU_F32:
-        if (T == 8) launch_one<F32Small>(d, src, n_par, outlet, 0, keys, s);
+        if (T == 8 && (long long)d.g.lx * d.g.ly <= kOneASm) launch_one<F32Small>(d, src, n_par, outlet, 0, keys, s);
+        else if (T == 8) launch_one<F32Small2>(d, src, n_par, outlet, 0, keys, s);
         else if (T == 4 && shape == TILE_WIDE) launch_one<F32Wide>(d, src, n_par, outlet, 0, keys, s);
         else if (T == 4) launch_one<F32Mid>(d, src, n_par, outlet, 0, keys, s);
         else launch_one<F32Large>(d, src, n_par, outlet, shape == TILE_LARGE ? 200 : 0, keys, s);

@@ -575,13 +575,15 @@ template <class SH, int M, bool EXTRAP>
 __global__ void __launch_bounds__(SH::NT, SH::MINB) k_tile(const __grid_constant__ TileArgs<typename SH::S> a)
 {
     extern __shared__ __align__(16) unsigned char tile_smem[];
-    if (a.pf > 0 && threadIdx.x < 9 * SH::H && blockIdx.x + (unsigned)a.pf < gridDim.x) {
-        int px, py;
-        tile_place(blockIdx.x + (unsigned)a.pf, a.nx, a.ny, a.ring_first, px, py);
-        const int Yp = 1 + py * SH::H + (int)threadIdx.x % SH::H, Xp = a.x_first + px * SH::W;
-        if (Yp <= a.g.ly && Xp >= 1 && Xp + SH::W - 1 <= a.g.lx)
-            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(plane(a.src, a.g, (int)threadIdx.x / SH::H) + a.g.idx(Xp, Yp)),
-                         "n"(SH::W * (int)sizeof(typename SH::S)) : "memory");
+    if constexpr (SH::W % 16 == 0) {         // (a prefetch is of whole 16-byte units)
+        if (a.pf > 0 && threadIdx.x < 9 * SH::H && blockIdx.x + (unsigned)a.pf < gridDim.x) {
+            int px, py;
+            tile_place(blockIdx.x + (unsigned)a.pf, a.nx, a.ny, a.ring_first, px, py);
+            const int Yp = 1 + py * SH::H + (int)threadIdx.x % SH::H, Xp = a.x_first + px * SH::W;
+            if (Yp <= a.g.ly && Xp >= 1 && Xp + SH::W - 1 <= a.g.lx)
+                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(plane(a.src, a.g, (int)threadIdx.x / SH::H) + a.g.idx(Xp, Yp)),
+                             "n"(SH::W * (int)sizeof(typename SH::S)) : "memory");
+        }
     }
     int tx, ty;
     tile_place(blockIdx.x, a.nx, a.ny, a.ring_first, tx, ty);

@@ -88,10 +88,10 @@ def test_extrapolated_outlet_of_a_custom_geometry():
 
 # either side of the node counts where the tile shape changes
 @pytest.mark.parametrize("precision,sizes", [
-    ("f64", [(257, 160), (401, 310), (2100, 1500)]),
-    ("f32", [(257, 160), (700, 200), (1030, 700)]),
-    ("f16", [(401, 160), (1030, 130), (2100, 1500)]),
-    ("bf16", [(401, 160), (1030, 130), (2100, 1500)]),
+    ("f64", [(230, 90), (257, 160), (401, 310), (2100, 1500)]),
+    ("f32", [(230, 90), (257, 240), (700, 200), (1030, 700)]),
+    ("f16", [(230, 90), (401, 160), (1030, 130), (2100, 1500)]),
+    ("bf16", [(230, 90), (401, 160), (1030, 130), (2100, 1500)]),
     ("f16r", [(401, 160), (1030, 130), (2100, 1500)]),
     ("bf16r", [(401, 160), (1030, 130)]),
     ("f16br", [(401, 160), (1030, 130), (2100, 1500)]),
