@@ -395,16 +395,18 @@ void finish(Simulation *sim, DropIn *c, bool collided = false)
     c->ahead = collided;
 }
 
-// After a stream whose outlet columns the collision before it brought along.
+// After a stream whose outlet columns the collision before it brought along: they are that stream's alone, handed
+// out or not.
 bool finish_ahead(Simulation *sim, DropIn *c)
 {
-    if (!c->ahead || c->sync_mode != LB_SYNC_OUTLET || c->dynp_dirty) return false;
+    const bool ahead = c->ahead;
+    c->ahead = false;
+    if (!ahead || c->sync_mode != LB_SYNC_OUTLET || c->dynp_dirty) return false;
     const size_t col = (size_t)(sim->ly + 2);
     const int X0 = sim->lx >= 2 ? sim->lx - 2 : 0;
     if (!c->ahead_there)
         std::memcpy(static_cast<void *>(chunk_of(sim->lattice) + (size_t)X0 * col), c->scratch + scratch_cols(sim),
                     (size_t)(sim->lx - X0) * col * sizeof(Node));
-    c->ahead = false;
     return true;
 }
 
