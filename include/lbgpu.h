@@ -165,7 +165,10 @@ double lbgpu_build_cylinder(int lx, int ly, int obst_x, int obst_y, int obst_r, 
  * two steps with the AA scheme. */
 int lbgpu_set_sweep_steps(lbgpu_lattice *lat, int steps);
 
-/* Advance `nsteps` time steps; asynchronous on the lattice's stream. */
+/* Advance `nsteps` time steps; asynchronous on the lattice's stream.  Steps (and velocity sums) on that stream
+ * can be captured in a CUDA graph by the caller; an even number of steps can be replayed wherever an even number
+ * of other steps lies between.  A lattice that has been captured takes its steps in somewhat more launches
+ * afterwards, so that its buffers stay where the graph has them. */
 int lbgpu_step(lbgpu_lattice *lat, int nsteps);
 
 /* Advance `nsteps` steps and report their device time in milliseconds (CUDA events on the

@@ -502,6 +502,20 @@ int lbgpu_batch_step(lbgpu_batch *b, int nsteps)
     if (!b || nsteps < 0) return set_error(LB_ERR_ARG, "lbgpu_batch_step: bad arguments");
     b->launches = 0;
     if (nsteps == 0 || lbgpu_batch_size(b) == 0) return LB_OK;
+    // A member whose stream was captured keeps its buffers in place over an even number of steps (Lattice::step); a
+    // capture of a member's stream takes the batch's stream in.
+    bool capturing = false, keep = false;
+    for (lbgpu_lattice *m : b->members) {
+        bool c = false;
+        if (m)
+            if (int rc = m->L.see_capture(c)) return rc;
+        capturing = capturing || c;
+    }
+    for (lbgpu_lattice *m : b->members)
+        if (m) {
+            m->L.keep_roles = m->L.keep_roles || capturing;
+            keep = keep || m->L.keep_roles;
+        }
     bool any_rs = false;
     for (lbgpu_lattice *m : b->members)
         if (m && m->L.rs) any_rs = true;
@@ -510,6 +524,15 @@ int lbgpu_batch_step(lbgpu_batch *b, int nsteps)
     bool own = false;
     for (lbgpu_lattice *m : b->members)
         if (m && needs_own_step(m->L)) own = true;
+    if (capturing) {
+        // nothing that waits or copies from the host's memory can be captured
+        bool ready = !own && !any_rs && !(nsteps & 1) && !b->dirty;
+        for (size_t i = 0; i < b->members.size() && ready; ++i)
+            if (b->members[i]) ready = i < b->h_inst.size() && describes(b->h_inst[i], b->members[i]->L);
+        if (!ready)
+            return set_error(LB_ERR_STATE, "lbgpu_batch_step: a captured call takes an even number of steps, of members "
+                             "without stochastic rounding that have stepped in the batch since they last changed");
+    }
     if (own) {
         for (lbgpu_lattice *m : b->members) {
             if (!m) continue;
@@ -539,7 +562,7 @@ int lbgpu_batch_step(lbgpu_batch *b, int nsteps)
         if (int rc = refresh_collision_numbers(b, 0)) return rc;
     }
     int done = 0;
-    while (nsteps - done >= kChunk) {
+    while (nsteps - done >= kChunk && !capturing) {
         if (any_rs && done)
             if (int rc = refresh_collision_numbers(b, done)) return rc;
         if (!b->graph[b->aa_phase])
@@ -551,12 +574,20 @@ int lbgpu_batch_step(lbgpu_batch *b, int nsteps)
     const int rem = nsteps - done;
     if (any_rs && done && rem)
         if (int rc = refresh_collision_numbers(b, done)) return rc;
-    for (int u = 0; u < rem / 2; ++u) launch_unit(b, u);
+    // an odd number of two-step launches would turn buffers and side store over: the last two steps stay single
+    // where they have to be kept
+    const bool tiled = b->nwork[kTiles] > 0;
+    const int last = keep && tiled && (rem & 2) ? 2 : 0;
+    for (int u = 0; u < (rem - last) / 2; ++u) launch_unit(b, u);
+    for (int k = rem - last; k < rem; ++k) launch_step(b, k, false);
     if (int rc = lbgpu::cuda_error(cudaGetLastError(), "batch step")) return rc;
     for (lbgpu_lattice *m : b->members)
-        if (m) advance(m->L, nsteps, b->nwork[kTiles] > 0);
+        if (m) {
+            advance(m->L, nsteps - last, tiled);
+            advance(m->L, last, false);
+        }
     if (int rc = order_after(b)) return rc;
-    if ((rem & 3) || any_rs) {
+    if ((tiled && ((rem - last) & 2)) || any_rs) {
         // two-step launches in an odd number turned buffers and side store over (or stochastically
         // rounded members count collisions): new descriptors before the next call, whose graphs read
         // them

@@ -34,6 +34,16 @@ inline int side_free(const DevLattice &d, int k)
     return -1;
 }
 
+// The slots a tile launch writes beside those in use: `prev` for the parity of the last collision but one, a (the
+// parity whose stale slots step 1 reads), and with row-shifted offsets `last` for the other parity.  The order of
+// the two parities' slots is kept, so that a second launch from the same parity takes back the slots of the first.
+inline int side_prev(const DevLattice &d, int a)
+{
+    const int other = side_free(d, 1);
+    return other < 0 || d.side_slot[a] < d.side_slot[1 - a] ? side_free(d, 0) : other;
+}
+inline int side_last(const DevLattice &d, int a) { return side_free(d, d.side_slot[a] < d.side_slot[1 - a] ? 1 : 0); }
+
 // How the post-stream state is read from a buffer:
 //   VIEW_DIRECT        the buffer holds it (pull form L, or a collided state read as is)
 //   VIEW_PULL_PENDING  the buffer holds C_n; the state is C_n streamed (side store: C_{n-1})

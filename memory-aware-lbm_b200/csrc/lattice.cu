@@ -169,16 +169,37 @@ int Lattice::create(int lx_, int ly_, int precision_, int scheme_)
     reset_roles();
     bc_host.assign(16 * (size_t)d.g.nb, 0.0);
     zgb_src_host.assign(4 * (size_t)d.g.nb, -1);
-    cur = 0; form = FORM_L; pending = 0; n = 0;
     return check("lattice create");
 }
 
-// The state is written afresh: each parity's stale slots in its own slot, each ring in its buffer.
+// The state is written afresh, into buffer `cur`: each parity's stale slots in its own slot, each ring in its
+// buffer; or where a captured graph expects it, whose steps then start from the same buffers and slots
+// again after as many steps as before its capture.
 void Lattice::reset_roles()
 {
-    d.side_slot[0] = 0;
-    d.side_slot[1] = 1;
+    cur = keep_roles ? cur ^ (int)(n & 1) : 0;
+    if (!keep_roles) {
+        d.side_slot[0] = 0;
+        d.side_slot[1] = 1;
+    }
     d.ghost_flip = 0;
+    form = FORM_L; pending = 0; n = 0;
+}
+
+void *Lattice::side_ptr(int p) const
+{
+    const int slot = d.side_slot[p];
+    return slot == 3 ? d.side_extra : static_cast<char *>(d.side) + (size_t)slot * 9 * (size_t)d.g.nper * elem;
+}
+
+// Whether the caller captures the stream; remembered, because its graph holds the buffers and slots of now.
+int Lattice::see_capture(bool &capturing)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    LB_CUDA(cudaStreamIsCapturing(stream, &status), "cudaStreamIsCapturing");
+    capturing = status != cudaStreamCaptureStatusNone;
+    keep_roles = keep_roles || capturing;
+    return LB_OK;
 }
 
 void Lattice::destroy()
@@ -310,14 +331,19 @@ int Lattice::step(int nsteps)
 {
     if (nsteps < 0) return set_error(LB_ERR_ARG, "negative step count");
     launches = 0;
-    // While the caller captures the stream, steps stay single: an even number of them leaves the buffers where
-    // it found them, so the caller's graph can be replayed; a tile launch turns them over.
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (nsteps > 1) LB_CUDA(cudaStreamIsCapturing(stream, &capture), "cudaStreamIsCapturing");
+    // A single step turns the buffers over, so an even number of them leaves them in place, and a caller's graph
+    // of them can be replayed; a tile launch turns them over too, whatever its steps.  So steps stay single
+    // while the caller captures the stream, and from then on tiles go in pairs of equal launches, which
+    // leave the buffers and the side store's slots where they were.
+    bool capturing = false;
+    if (nsteps > 0) LB_TRY(see_capture(capturing));
+    int second = 0;       // steps of a pair's second launch
     for (int s = 0; s < nsteps; ++s) {
         // a run of pull steps: several a launch, the state as single steps leave it
-        if (scheme == LBGPU_PULL && !ghosts && form == FORM_C && pending && capture == cudaStreamCaptureStatusNone) {
-            if (const int T = tile_steps(d, nsteps - s, zgb_each_step, rs)) {
+        if (scheme == LBGPU_PULL && !ghosts && form == FORM_C && pending && !capturing) {
+            const int rest = nsteps - s;
+            if (const int T = second ? second : tile_steps(d, keep_roles ? rest / 2 : rest, zgb_each_step, rs)) {
+                second = keep_roles && !second ? T : 0;
                 unsigned keys[8] = {0};
                 for (int k = 0; rs && k < T; ++k) keys[k] = rs_key(rs_seed, (unsigned long long)(n + 1 + k));
                 launch_tile(d, cur, (int)(n & 1), T, zgb_each_step, keys, stream);
@@ -341,7 +367,7 @@ int Lattice::step(int nsteps)
 
 void Lattice::after_tile(int T)
 {
-    const int a = (int)((n + 1) & 1), prev = side_free(d, 0), last = side_free(d, 1);
+    const int a = (int)((n + 1) & 1), prev = side_prev(d, a), last = side_last(d, a);
     d.side_slot[a] = prev;
     if (d.g.shift_u) d.side_slot[1 - a] = last;
     d.ghost_flip ^= 1;
@@ -476,7 +502,7 @@ int Lattice::init_side_from(int b, int par)
 
 int Lattice::init_cylinder(double umax)
 {
-    launch_init_cylinder(d, 0, umax, stream);
+    launch_init_cylinder(d, cur, umax, stream);
     ++launches;
     return check("init cylinder");
 }
@@ -547,6 +573,8 @@ int Lattice::velocity_accumulate()
         LB_CUDA(cudaMemsetAsync(vel_acc, 0, bytes, stream), "clear velocity sums");
         vel_samples = 0;
     }
+    bool capturing;
+    LB_TRY(see_capture(capturing));
     int v, par;
     view(v, par);
     launch_accumulate_velocity(d, v, cur, par, vel_acc, stream);

@@ -52,6 +52,7 @@ struct Lattice {
     void *memory = nullptr;        // the one allocation that d's pointers lead into
     size_t memory_bytes = 0;
     bool held = false;             // counted by memory_hold
+    bool keep_roles = false;       // a caller captured the stream: an even number of steps leaves buffers and slots in place
     int launches = 0;    // kernels launched by the last public call
     unsigned long long h2d_bytes = 0, d2h_bytes = 0;  // bytes copied host<->device so far
     int device = 0;      // CUDA device the lattice lives on
@@ -64,6 +65,8 @@ struct Lattice {
     int create(int lx, int ly, int precision, int scheme);
     void destroy();
     void reset_roles();
+    void *side_ptr(int p) const;          // the side store's slot of collision parity p
+    int see_capture(bool &capturing);
 
     // per-step operations (asynchronous on `stream`)
     int op_collide();        // collide the current state in place or through the pull kernel
@@ -93,7 +96,7 @@ struct Lattice {
     int readout_records(double *host, int rs, const uint64_t *dynp_dev, int X0, int X1);
     int readout_populations(double *host);       // [lx+2][ly+2][9] into a pageable array
     int init_side_from(int b, int par);
-    int init_cylinder(double umax);  // equilibrium Poiseuille populations into buffer 0
+    int init_cylinder(double umax);  // equilibrium Poiseuille populations into the current buffer
     int get_macros(double *rho, double *ux, double *uy);  // host [ly][lx] arrays
     int moments(double out[8]);                           // FP64 sums (kernels.h)
     int velocity_accumulate();

@@ -227,18 +227,18 @@ int lbgpu_set_populations(lbgpu_lattice *h, const double *f, const double *tmp)
         if (int rc = L.upload_records(0, f, 9, 0, L.lx + 2)) return rc;
         if (int rc = L.init_side_from(0, 0)) return rc;
     } else {
-        if (int rc = L.upload_records(0, f, 9, 0, L.lx + 2)) return rc;
+        const int other = 1 - L.cur;
+        if (int rc = L.upload_records(L.cur, f, 9, 0, L.lx + 2)) return rc;
         if (tmp) {
-            if (int rc = L.upload_records(1, tmp, 9, 0, L.lx + 2)) return rc;
+            if (int rc = L.upload_records(other, tmp, 9, 0, L.lx + 2)) return rc;
         } else {
-            if (int rc = lbgpu::cuda_error(cudaMemsetAsync(L.d.buf[1], 0, 9 * (size_t)L.d.g.plane * L.elem,
+            if (int rc = lbgpu::cuda_error(cudaMemsetAsync(L.d.buf[other], 0, 9 * (size_t)L.d.g.plane * L.elem,
                                                            L.stream), "clear second buffer"))
                 return rc;
         }
         // the first stream leaves the second buffer's content in the stale slots: side parity 1
-        if (int rc = L.init_side_from(1, 1)) return rc;
+        if (int rc = L.init_side_from(other, 1)) return rc;
     }
-    L.cur = 0; L.form = lbgpu::FORM_L; L.pending = 0; L.n = 0;
     return lbgpu::cuda_error(cudaStreamSynchronize(L.stream), "lbgpu_set_populations");
 }
 
@@ -269,9 +269,10 @@ int lbgpu_setup_cylinder(lbgpu_lattice *h, int obst_x, int obst_y, int obst_r, d
             if (int rc = lbgpu::cuda_error(cudaMemsetAsync(L.d.buf[b], 0, 9 * (size_t)L.d.g.plane * L.elem,
                                                            L.stream), "clear populations"))
                 return rc;
-    if (int rc = lbgpu::cuda_error(cudaMemsetAsync(L.d.side, 0, 2 * 9 * (size_t)L.d.g.nper * L.elem,
-                                                   L.stream), "clear side store"))
-        return rc;
+    for (int p = 0; p < 2; ++p)
+        if (int rc = lbgpu::cuda_error(cudaMemsetAsync(L.side_ptr(p), 0, 9 * (size_t)L.d.g.nper * L.elem, L.stream),
+                                       "clear side store"))
+            return rc;
     if (int rc = L.init_cylinder(umax)) return rc;
     // second buffer zero (reference calloc, lb.c:91-92): side parity 1 stays zero; the AA scheme
     // reads the initial state's own stale slots from parity 0
@@ -281,7 +282,6 @@ int lbgpu_setup_cylinder(lbgpu_lattice *h, int obst_x, int obst_y, int obst_r, d
                                                        L.stream), "clear ghost ring"))
             return rc;
     }
-    L.cur = 0; L.form = lbgpu::FORM_L; L.pending = 0; L.n = 0;
     return lbgpu::cuda_error(cudaStreamSynchronize(L.stream), "lbgpu_setup_cylinder");
 }
 

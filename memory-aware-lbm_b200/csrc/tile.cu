@@ -80,8 +80,9 @@ void launch_shape(const DevLattice &d, int src, int n_par, int pf, const unsigne
     // the side store too (its own slots are rebased), so both go to free slots, of four.
     a.stale1 = SIDE<S>(d, n_par + 1);
     a.stale2 = SIDE<S>(d, n_par);
-    a.out_last = (M & TILE_SHIFT) ? SIDE_SLOT<S>(d, side_free(d, 1)) : SIDE<S>(d, n_par);
-    a.out_prev = SIDE_SLOT<S>(d, side_free(d, 0));
+    const int ap = (n_par + 1) & 1;
+    a.out_last = (M & TILE_SHIFT) ? SIDE_SLOT<S>(d, side_last(d, ap)) : SIDE<S>(d, n_par);
+    a.out_prev = SIDE_SLOT<S>(d, side_prev(d, ap));
     a.sc = d.scale;
     a.inv = d.inv_scale;
     // the outlet's extrapolation reads three columns back: its tile must not be narrower
