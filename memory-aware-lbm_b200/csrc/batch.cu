@@ -121,13 +121,13 @@ BatchInst describe(const Lattice &L)
     return b;
 }
 
-// Whether a descriptor still holds for a member (its collision number apart, of which kernels without
-// stochastic rounding use the parity only).
+// Whether a descriptor still holds for a member.  Of its collision number kernels without stochastic rounding use
+// the parity only.
 bool describes(const BatchInst &b, const Lattice &L)
 {
     const BatchInst now = describe(L);
     return b.rs == now.rs && b.rs_seed == now.rs_seed && b.g.shift_u == now.g.shift_u && b.cur0 == now.cur0 &&
-           b.phase0 == now.phase0 && ((b.tau0 ^ now.tau0) & 1) == 0 && b.side_slot[0] == now.side_slot[0] &&
+           b.phase0 == now.phase0 && (now.rs ? b.tau0 == now.tau0 : ((b.tau0 ^ now.tau0) & 1) == 0) && b.side_slot[0] == now.side_slot[0] &&
            b.side_slot[1] == now.side_slot[1] && b.omega == now.omega && b.scale == now.scale &&
            b.rules_inside == now.rules_inside;
 }

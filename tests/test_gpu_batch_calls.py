@@ -1,0 +1,41 @@
+"""Calls of lbgpu_batch_step between other calls: that they return before their work ends, and that members' own
+steps between them are seen."""
+import pytest
+
+import lbgpu
+from helpers import same
+
+pytestmark = pytest.mark.gpu
+
+
+def singles(lat, n):
+    for _ in range(n):
+        lat.step(1)
+
+
+@pytest.mark.parametrize("precision", ["f16r", "bf16r"])
+def test_rounding_keys_follow_members_that_step_alone(precision):
+    """A stochastically rounded member counts its collisions wherever it steps, also where its own steps leave
+    its buffers in place, or its state is set again."""
+    def run(batched):
+        lat = lbgpu.Lattice(33, 40, lbgpu.storage_form(precision)[0], "pull")
+        lbgpu.configure_storage(lat, precision, 0.03, 7)
+        lat.setup_cylinder(8, 20, 4, 0.03, 30.0, lbgpu.WALL_REGULARIZED, lbgpu.OUTLET_CONST)
+        with lbgpu.Batch(lbgpu.storage_form(precision)[0]) as b:
+            b.add(lat)
+            go = b.step if batched else (lambda n: singles(lat, n))
+            go(7)
+            lat.step(16)
+            go(46)
+            b.synchronize()
+            first = lat.populations()
+            go(1)
+            lat.set_populations(first, first)
+            go(22)
+            b.synchronize()
+            out = (first, lat.populations())
+        lat.close()
+        return out
+
+    for got, exp in zip(run(True), run(False)):
+        assert same(got, exp)
