@@ -146,6 +146,29 @@ int refresh_collision_numbers(lbgpu_batch *b, int done)
                                        cudaMemcpyHostToDevice, b->stream), "update batch collision numbers");
 }
 
+// The descriptors after an odd number of two-step launches, on the device: what describe() gives then, but for the
+// collision number, whose parity stays.  A new copy from the host's memory would make the call wait.
+__global__ void k_batch_turn(BatchInst *insts, int n, int elem)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n || insts[i].scheme != LBGPU_PULL) return;
+    BatchInst &d = insts[i];
+    const int a = d.tau0 & 1, spare = 3 - d.side_slot[0] - d.side_slot[1];
+    d.side_slot[a] = spare;
+    d.side_of[a] = static_cast<char *>(d.side) + (size_t)spare * 9 * (size_t)d.g.nper * elem;
+    d.cur0 ^= 1;
+}
+
+int turn_descriptors(lbgpu_batch *b)
+{
+    const int n = (int)b->members.size();
+    const int elem = b->precision == LBGPU_F64 ? 8 : (b->precision == LBGPU_F32 ? 4 : 2);
+    k_batch_turn<<<(n + 127) / 128, 128, 0, b->stream>>>(b->d_inst, n, elem);
+    for (int i = 0; i < n; ++i)
+        if (b->members[i]) b->h_inst[i] = describe(b->members[i]->L);
+    return batch_error(cudaGetLastError(), "batch descriptors");
+}
+
 // Pull members can take two steps a launch, but for row-shifted offsets (rebased between rows).
 bool takes_tiles(const Lattice &L) { return L.scheme == LBGPU_PULL && !L.d.g.shift_u; }
 
@@ -586,11 +609,12 @@ int lbgpu_batch_step(lbgpu_batch *b, int nsteps)
             advance(m->L, nsteps - last, tiled);
             advance(m->L, last, false);
         }
+    if (tiled && ((rem - last) & 2) && !any_rs)
+        if (int rc = turn_descriptors(b)) return rc;
     if (int rc = order_after(b)) return rc;
-    if ((tiled && ((rem - last) & 2)) || any_rs) {
-        // two-step launches in an odd number turned buffers and side store over (or stochastically
-        // rounded members count collisions): new descriptors before the next call, whose graphs read
-        // them
+    if (any_rs) {
+        // stochastically rounded members count collisions: new descriptors before the next call, whose
+        // graphs read them
         if (int rc = refresh_collision_numbers(b, 0)) return rc;
         if (int rc = batch_error(cudaStreamSynchronize(b->stream), "update batch members")) return rc;
     }

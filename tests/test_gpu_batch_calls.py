@@ -39,3 +39,28 @@ def test_rounding_keys_follow_members_that_step_alone(precision):
 
     for got, exp in zip(run(True), run(False)):
         assert same(got, exp)
+@pytest.mark.parametrize("storage,scheme", [("f32", "pull"), ("f32", "aa"), ("f16b", "pull")])
+def test_batch_steps_do_not_wait(storage, scheme):
+    """Even counts return while the GPU still works, whatever their remainder."""
+    import torch
+
+    base = lbgpu.storage_form(storage)[0]
+    lats = []
+    for _ in range(8):
+        lat = lbgpu.Lattice(2048, 1024, base, scheme)
+        lbgpu.configure_storage(lat, storage, 0.03)
+        lat.setup_cylinder(400, 500, 100, 0.03, 60.0, lbgpu.WALL_BOUNCEBACK, lbgpu.OUTLET_CONST)
+        lats.append(lat)
+    with lbgpu.Batch(base) as b:
+        for lat in lats:
+            b.add(lat)
+        b.step(41)
+        stream = torch.cuda.ExternalStream(lats[0].stream)
+        for n in (10, 14, 12):
+            b.synchronize()
+            stream.synchronize()
+            b.step(n)
+            assert not stream.query(), n
+        b.synchronize()
+    for lat in lats:
+        lat.close()
