@@ -214,8 +214,8 @@ int lbgpu_synchronize(lbgpu_lattice *lat);
  * No counterpart in the reference (one lattice per process).  Members are lattices of the
  * batch's precision, pull or AA, with constant-density outlets (an extrapolated outlet is
  * stepped on its own).  lbgpu_batch_step advances every member by nsteps: one launch per two steps
- * for the pull members (per step where one stores row-shifted offsets) and one per step for each phase of the AA members walks a
- * work list of tiles; chunks of 20 steps are replayed as a CUDA graph.  Each member's result is bit-identical to stepping it alone.  The batch does not
+ * for the pull members (per step where one stores row-shifted offsets, and for the odd step of a
+ * call) and one per step for each phase of the AA members walks a work list of tiles; chunks of 20 steps are replayed as a CUDA graph.  Each member's result is bit-identical to stepping it alone.  The batch does not
  * own its members; remove a member before destroying it.  Steps are asynchronous on the batch's
  * stream and ordered with the members' own streams. */
 typedef struct lbgpu_batch lbgpu_batch;
@@ -254,7 +254,10 @@ int lbgpu_batch_get_threads(lbgpu_batch *b);
  * launch-form pair, then, for each size class present, with each tile shape (three widths, and
  * four nodes per thread for 16-bit storage), keeping the fastest at each stage (the members
  * really advance 6 x (steps + 1) plus 3 or 4 x (steps + 1) per class present); best_ms[6]
- * receives each class's best time (0 for classes not present) when not NULL. */
+ * receives each class's best time (0 for classes not present) when not NULL.
+ * These settings shape single steps: those of AA members, of pull members in a batch with row-shifted
+ * offsets, and the odd step of a call.  With an even `steps` a class of other pull members, which take
+ * two steps a launch, is not tuned: the batch is timed once, as it is set, for its best_ms. */
 int lbgpu_batch_autotune(lbgpu_batch *b, int steps, float *best_ms);
 
 /* Device bytes a lattice of this size, precision and scheme allocates. */

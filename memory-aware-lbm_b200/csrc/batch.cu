@@ -172,6 +172,14 @@ int turn_descriptors(lbgpu_batch *b)
 // Pull members can take two steps a launch, but for row-shifted offsets (rebased between rows).
 bool takes_tiles(const Lattice &L) { return L.scheme == LBGPU_PULL && !L.d.g.shift_u; }
 
+// All pull members do, or none: their single-step lists are shared.
+bool all_tiled(const lbgpu_batch *b)
+{
+    for (const lbgpu_lattice *m : b->members)
+        if (m && m->L.scheme == LBGPU_PULL && !takes_tiles(m->L)) return false;
+    return true;
+}
+
 // A member's host-side state after `m` batch steps (no launches); tiles: pull members took two a launch.
 void advance(Lattice &L, int m, bool tiles)
 {
@@ -231,9 +239,7 @@ int rebuild(lbgpu_batch *b)
     std::vector<BatchWork> work[kLists], inner;
     int w, h;
     lbgpu::batch_tile(b->precision, &w, &h);
-    bool tiled = true;      // all pull members, or none: their single-step lists are shared
-    for (const lbgpu_lattice *m : b->members)
-        if (m && m->L.scheme == LBGPU_PULL && !takes_tiles(m->L)) tiled = false;
+    const bool tiled = all_tiled(b);
     b->h_inst.assign(b->members.size(), BatchInst{});
     for (size_t i = 0; i < b->members.size(); ++i) {
         lbgpu_lattice *m = b->members[i];
@@ -659,13 +665,24 @@ static int time_setting(lbgpu_batch *b, int steps, float *ms)
 // class present the three tile widths (and for 16-bit storage the four-nodes-a-thread pull),
 // each timed over `steps` batch steps after one untimed step; the fastest is kept at each
 // stage.  The members really step (6 x (steps + 1), then 3 or 4 x (steps + 1) per class).
+// The settings shape the single-step launches.  Pull members that take two steps a launch make one only where
+// `steps` is odd: a class of nothing else keeps its settings, and the batch is timed once for it.
 int lbgpu_batch_autotune(lbgpu_batch *b, int steps, float *best_ms_out)
 {
     if (!b || steps < 1) return set_error(LB_ERR_ARG, "lbgpu_batch_autotune: bad arguments");
-    bool present[kClasses] = {false};
+    const bool tiled = all_tiled(b) && !(steps & 1);
+    bool present[kClasses] = {false}, shaped[kClasses] = {false}, any = false, other = false;
     for (lbgpu_lattice *m : b->members)
-        if (m) present[size_class((long long)m->L.lx * m->L.ly)] = true;
-    {
+        if (m) {
+            const int c = size_class((long long)m->L.lx * m->L.ly);
+            present[c] = true;
+            shaped[c] = shaped[c] || !tiled || m->L.scheme == LBGPU_AA;
+        }
+    for (int c = 0; c < kClasses; ++c) {
+        any = any || shaped[c];
+        other = other || (present[c] && !shaped[c]);
+    }
+    if (any) {
         float best = 1e30f;
         int best_t = b->threads, best_p = b->persistent ? 1 : 0;
         for (int t = 128; t <= 512; t *= 2)
@@ -681,7 +698,7 @@ int lbgpu_batch_autotune(lbgpu_batch *b, int steps, float *best_ms_out)
     }
     for (int c = 0; c < kClasses; ++c) {
         if (best_ms_out) best_ms_out[c] = 0.f;
-        if (!present[c]) continue;
+        if (!shaped[c]) continue;
         float best = 1e30f;
         int best_shape = b->shape[c];
         const int nshapes = (b->precision == LBGPU_F16 || b->precision == LBGPU_BF16) ? 4 : 3;
@@ -709,6 +726,12 @@ int lbgpu_batch_autotune(lbgpu_batch *b, int steps, float *best_ms_out)
         b->passes[c] = best_np;
         b->dirty = true;
         if (best_ms_out) best_ms_out[c] = best;
+    }
+    if (other && best_ms_out) {
+        float ms = 0.f;
+        if (int rc = time_setting(b, steps, &ms)) return rc;
+        for (int c = 0; c < kClasses; ++c)
+            if (present[c] && !shaped[c]) best_ms_out[c] = ms;
     }
     return LB_OK;
 }

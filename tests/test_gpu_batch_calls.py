@@ -55,12 +55,42 @@ def test_batch_steps_do_not_wait(storage, scheme):
         for lat in lats:
             b.add(lat)
         b.step(41)
+        b.step(2)
         stream = torch.cuda.ExternalStream(lats[0].stream)
-        for n in (10, 14, 12):
+        for n in (110, 114, 112):
             b.synchronize()
             stream.synchronize()
             b.step(n)
             assert not stream.query(), n
         b.synchronize()
+    for lat in lats:
+        lat.close()
+
+
+def test_the_tuner_leaves_alone_what_its_settings_do_not_reach():
+    """Pull members that take two steps a launch: one timing, no setting changed; the class of an AA member beside
+    them, and odd counts, are tuned."""
+    lats = [lbgpu.Lattice(40, 30, "f32", "pull"), lbgpu.Lattice(300, 90, "f32", "pull"), lbgpu.Lattice(300, 90, "f32", "aa")]
+    for lat in lats:
+        lat.setup_cylinder(9, 12, 3, 0.03, 30.0, lbgpu.WALL_BOUNCEBACK, lbgpu.OUTLET_CONST)
+    small, large = lbgpu.size_class(40 * 30), lbgpu.size_class(300 * 90)
+    with lbgpu.Batch("f32") as b:
+        b.add(lats[0])
+        slot = b.add(lats[1])
+        b.set_shape(small, 32)
+        b.threads = 256
+        best = b.autotune(4)
+        assert lats[0].steps_done == lats[1].steps_done == 5
+        assert (b.shape(small), b.threads) == ((32, 1), 256)
+        assert [k for k, ms in enumerate(best) if ms > 0] == sorted({small, large})
+        b.remove(slot)
+        b.add(lats[2])
+        best = b.autotune(4)
+        # the launch forms, three widths and four or five strip lengths of the large class, and one for the other class
+        done = lats[0].steps_done
+        assert done - 5 in (5 * (6 + 3 + 4 + 1), 5 * (6 + 3 + 5 + 1)) and b.shape(small) == (32, 1)
+        assert best[small] > 0 and best[large] > 0
+        b.autotune(3)
+        assert lats[0].steps_done >= done + 4 * (6 + 2 * (3 + 4))
     for lat in lats:
         lat.close()
