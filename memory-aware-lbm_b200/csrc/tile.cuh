@@ -469,8 +469,10 @@ __device__ __forceinline__ void bgk_offsets_pair_shifted(float2 D[9], float omeg
 // The pairs of step s start at column x0 - (T - s): a step later they start one column on, so the
 // two populations that a pair takes from x - 1 or x + 1 were stored (or, T being even, lie in the
 // planes) as one pair, and only those of the three directions along y are read one by one.
+// Step 1 sets *met where it meets a node with a boundary rule, which it does not apply.
 template <class S, class SH, int s, int M>
-__device__ __forceinline__ void tile_step_pairs(const TileArgs<S> &a, S *__restrict__ sm, uint8_t *__restrict__ stag, int x0, int y0)
+__device__ __forceinline__ void tile_step_pairs(const TileArgs<S> &a, S *__restrict__ sm, uint8_t *__restrict__ stag,
+                                                int *__restrict__ met, int x0, int y0)
 {
     constexpr bool RS = (M & TILE_RS) != 0, SHIFT = (M & TILE_SHIFT) != 0;
     constexpr int E = SH::T - s, WP = (SH::W + 2 * E) / 2, HS = SH::H + 2 * E, O = s - 1, RW = SH::RW, PL = SH::PL;
@@ -508,6 +510,7 @@ __device__ __forceinline__ void tile_step_pairs(const TileArgs<S> &a, S *__restr
             else if constexpr (sizeof(S) == 2) bgk_offsets_pair(f, a.omega_f, a.sc, a.inv);
             else bgk_pair(f, a.omega_f);
         } else {
+            if (s == 1 && ((t & 0xffu) >= TAG_ZOUHE_FIRST || (t >> 8) >= TAG_ZOUHE_FIRST)) *met = 1;
             float h[9];
 #pragma unroll
             for (int i = 0; i < 9; ++i) h[i] = f[i].x;
@@ -539,16 +542,20 @@ __device__ __forceinline__ void tile_step_pairs(const TileArgs<S> &a, S *__restr
     }
 }
 
+// Steps s to T; false where step 1 of a tile off the perimeter met a boundary rule: nothing is written to the planes
+// yet, and the tile takes its steps afresh as one with rules.
 template <class S, class SH, int s, bool EDGE, int M, bool EXTRAP>
-__device__ __forceinline__ void tile_steps(const TileArgs<S> &a, S *sm, uint8_t *stag, unsigned short *list, int *nlist,
+__device__ __forceinline__ bool tile_steps(const TileArgs<S> &a, S *sm, uint8_t *stag, unsigned short *list, int *nlist,
                                            int x0, int y0)
 {
-    if constexpr (!EDGE && sizeof(S) <= 4) tile_step_pairs<S, SH, s, M>(a, sm, stag, x0, y0);
+    if constexpr (!EDGE && sizeof(S) <= 4) tile_step_pairs<S, SH, s, M>(a, sm, stag, nlist, x0, y0);
     else tile_step<S, SH, s, EDGE, M, EXTRAP>(a, sm, stag, list, nlist, x0, y0);
     if constexpr (s < SH::T) {
         __syncthreads();
-        tile_steps<S, SH, s + 1, EDGE, M, EXTRAP>(a, sm, stag, list, nlist, x0, y0);
+        if (s == 1 && !EDGE && sizeof(S) <= 4 && a.rules_inside && *nlist != 0) return false;
+        return tile_steps<S, SH, s + 1, EDGE, M, EXTRAP>(a, sm, stag, list, nlist, x0, y0);
     }
+    return true;
 }
 
 // The T steps of the tile at (x0, y0) by one block.
@@ -561,14 +568,21 @@ __device__ __forceinline__ void tile_block(const TileArgs<typename SH::S> &a, un
     unsigned short *list = reinterpret_cast<unsigned short *>(stag + SH::TAGS);
     int *nlist = reinterpret_cast<int *>(smem + SH::SMEM - 16);
     constexpr int E = SH::T - 1;
-    const bool inside = !a.rules_inside && x0 - E >= 2 && x0 + SH::W - 1 + E <= a.g.lx - 1 && y0 - E >= 2 && y0 + SH::H - 1 + E <= a.g.ly - 1;
+    // Where some node off the perimeter has a boundary rule, pairs (FP32 and 16-bit) find out in step 1 whether it is one
+    // of this tile's; FP64, whose two forms run alike, does not try.
+    const bool inside = (sizeof(S) <= 4 || !a.rules_inside) &&
+                        x0 - E >= 2 && x0 + SH::W - 1 + E <= a.g.lx - 1 && y0 - E >= 2 && y0 + SH::H - 1 + E <= a.g.ly - 1;
     if (inside) {
-        tile_steps<S, SH, 1, false, M, EXTRAP>(a, sm, stag, list, nlist, x0, y0);
-    } else {
-        if (threadIdx.x == 0) *nlist = 0;
-        __syncthreads();
-        tile_steps<S, SH, 1, true, M, EXTRAP>(a, sm, stag, list, nlist, x0, y0);
+        if (a.rules_inside) {
+            if (threadIdx.x == 0) *nlist = 0;
+            __syncthreads();
+        }
+        if (tile_steps<S, SH, 1, false, M, EXTRAP>(a, sm, stag, list, nlist, x0, y0)) return;
+        __syncthreads();           // every thread has read what it met
     }
+    if (threadIdx.x == 0) *nlist = 0;
+    __syncthreads();
+    tile_steps<S, SH, 1, true, M, EXTRAP>(a, sm, stag, list, nlist, x0, y0);
 }
 
 template <class SH, int M, bool EXTRAP>
