@@ -398,7 +398,8 @@ __device__ __forceinline__ void regularize_exact(double f[9], int side, double r
 
 // Any non-BGK rule; (p0, p1) are the node's table entry: (ux, uy) or (rho, uPar).
 // Boundary rules chain to bulk BGK like every function of boundaries.c:171-414.
-template <class T>
+// EXACT: the FP64 forms with fewer operations, for the tile kernel.
+template <class T, bool EXACT = false>
 __device__ __forceinline__ void boundary_rule(int t, T f[9], T omega, T p0, T p1)
 {
     if (t == TAG_BOUNCE) { bounce(f); return; }
@@ -416,34 +417,39 @@ __device__ __forceinline__ void boundary_rule(int t, T f[9], T omega, T p0, T p1
         uy = tb ? u : p1;
     }
     if (t < TAG_REG_FIRST) zouhe_complete(f, side, ux, uy, rho);
-    else if constexpr (sizeof(T) == 8) regularize_exact(f, side, rho, ux, uy);
+    else if constexpr (EXACT) regularize_exact(f, side, rho, ux, uy);
     else regularize(f, side, rho, ux, uy);
-    if constexpr (sizeof(T) == 8) bgk_exact(f, omega);
+    if constexpr (EXACT) bgk_exact(f, omega);
     else bgk(f, omega);
 }
 
-template <class T>
+template <class T, bool EXACT = false>
 static __device__ __noinline__ void collide_boundary(int t, T f[9], T omega, T p0, T p1)
 {
-    boundary_rule<T>(t, f, omega, p0, p1);
+    boundary_rule<T, EXACT>(t, f, omega, p0, p1);
 }
 
 // The boundary rules run out of line on a private copy, so the bulk path's populations stay
 // in registers (a warp whose lanes are all bulk nodes never enters the call).
+template <class T, bool EXACT>
+__device__ __forceinline__ void collide_called(int t, T f[9], T omega, T p0, T p1)
+{
+    T g[9];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) g[i] = f[i];
+    collide_boundary<T, EXACT>(t, g, omega, p0, p1);
+#pragma unroll
+    for (int i = 0; i < 9; ++i) f[i] = g[i];
+}
+
+// The single-step kernels: FP64 in its general forms too.  Those kernels stream, and the forms with fewer operations
+// cost them resident warps, also in the rules out of line (a kernel has the registers of what it calls):
+// k_pull<double> 56 -> 72 registers, 2047 x 511 28.7 -> 30.1 us a step on one B200, 700 x 200 7.0 -> 8.0.
 template <class T>
 __device__ __forceinline__ void collide(int t, T f[9], T omega, T p0, T p1)
 {
-    if (t == TAG_BGK) {
-        if constexpr (sizeof(T) == 8) bgk_exact(f, omega);
-        else bgk(f, omega);
-    } else {
-        T g[9];
-#pragma unroll
-        for (int i = 0; i < 9; ++i) g[i] = f[i];
-        collide_boundary<T>(t, g, omega, p0, p1);
-#pragma unroll
-        for (int i = 0; i < 9; ++i) f[i] = g[i];
-    }
+    if (t == TAG_BGK) bgk(f, omega);
+    else collide_called<T, false>(t, f, omega, p0, p1);
 }
 
 // equilibrium at (rho, ux, uy) for initialisation (lb.c:71-78)

@@ -169,14 +169,17 @@ __device__ __forceinline__ void tile_boundary(const TileArgs<S> &a, const S *__r
     if (EXTRAP && (t == LBGPU_TAG_RIGHT_PRESSURE_ZOUHE || t == LBGPU_TAG_RIGHT_PRESSURE_REGULARIZED) && a.zgb[Y] >= 0) {
         using D = Ar<double>;
         const double r1 = tile_density<S, SH, s>(a, rd, X, Y, q, 0), r2 = tile_density<S, SH, s>(a, rd, X, Y, q, 1);
-        collide_given<S>(g, t, f, a.omega, a.sc, a.inv, D::S(D::M(4. / 3., r1), D::M(1. / 3., r2)), 0.0);
-    } else if constexpr (sizeof(S) == 8 && SH::T == 4) {
-        // in line: the call's way through local memory is part of a step's longest chain.  FP64 511 x 127 3.8 -> 3.4
-        // us a step; eight steps' copies of it leave the instruction cache (250 x 51 2.4 -> 2.9), and FP32 gains
-        // nothing.
+        const double rho = D::S(D::M(4. / 3., r1), D::M(1. / 3., r2));
+        if constexpr (sizeof(S) == 8) rules::collide_called<double, true>(t, f, a.omega, rho, 0.0);
+        else collide_given<S>(g, t, f, a.omega, a.sc, a.inv, rho, 0.0);
+    } else if constexpr (sizeof(S) == 8) {
+        // in line where a launch takes four steps: the call's way through local memory is part of a step's longest chain.
+        // 511 x 127 3.8 -> 3.4 us a step; eight steps' copies of it leave the instruction cache (250 x 51 2.4 -> 2.9),
+        // and FP32 gains nothing.
         double p0, p1;
         node_params(a.bc, g, t, X, Y, p0, p1);
-        rules::boundary_rule<double>(t, f, a.omega, p0, p1);
+        if constexpr (SH::T == 4) rules::boundary_rule<double, true>(t, f, a.omega, p0, p1);
+        else rules::collide_called<double, true>(t, f, a.omega, p0, p1);
     } else {
         collide_w<S, (M & TILE_SHIFT) ? 1 : 0>(a.bc, g, t, X, Y, f, a.omega, a.sc, a.inv);
     }
