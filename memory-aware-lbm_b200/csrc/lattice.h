@@ -19,11 +19,11 @@ void clear_error();
 // 256 MiB of what was given back (a cudaMalloc takes 0.1 ms and more, a cudaFree waits for the whole
 // device: a 1024 x 256 FP32 lattice is made in 0.07 ms instead of 0.74 and closed in 0.07 instead of 0.6, a
 // served stream of 24 requests takes 52 ms instead of 65); what it keeps goes back with the last lattice.  Larger
-// parts are cudaMalloc's (150 MB 0.4 ms, 2.4 GB 0.9, against 13.5 from a pool that has to grow).  Usable on other streams once `s` has
-// reached the allocation; give it back, with its size, when nothing uses it any more.
+// parts are cudaMalloc's (150 MB 0.4 ms, 2.4 GB 0.9, against 13.5 from a pool that has to grow).  Usable on
+// any stream at once; given back, with its size, after what `s` still does with it.
 constexpr size_t kPoolBytes = (size_t)64 << 20;
-cudaError_t device_alloc(void **p, size_t bytes, int device, cudaStream_t s);
-cudaError_t device_free(void *p, size_t bytes, cudaStream_t s);
+cudaError_t device_alloc(void **p, size_t bytes, int device);
+cudaError_t device_free(void *p, size_t bytes, int device, cudaStream_t s);
 // Lattices alive (each calls hold once and drop once): the last one returns what is kept between them, the
 // pools' memory and the pinned buffer of read_back.
 void memory_hold();

@@ -111,7 +111,7 @@ int start(lbgpu_server *s, Req &q, int id)
     if (int rc = lbgpu_setup_cylinder(q.lat, r.obst_x, r.obst_y, r.obst_r, r.umax, r.re,
                                       LBGPU_WALL_BOUNCEBACK, LBGPU_OUTLET_CONST, nullptr))
         return rc;
-    if (int rc = serr(lbgpu::device_alloc(&q.prev, 8 * (size_t)r.lx * r.ly, q.lat->L.device, q.lat->L.stream),
+    if (int rc = serr(lbgpu::device_alloc(&q.prev, 8 * (size_t)r.lx * r.ly, q.lat->L.device),
                       "device memory (velocity snapshot)"))
         return rc;
     // the snapshot starts as the initial velocity (the first check compares against it)
@@ -127,7 +127,7 @@ int start(lbgpu_server *s, Req &q, int id)
 
 void release(Req &q)
 {
-    if (q.prev) lbgpu::device_free(q.prev, 8 * (size_t)q.spec.lx * q.spec.ly, q.lat->L.stream);
+    if (q.prev) lbgpu::device_free(q.prev, 8 * (size_t)q.spec.lx * q.spec.ly, q.lat->L.device, q.lat->L.stream);
     q.prev = nullptr;
     if (q.lat) lbgpu_destroy(q.lat);
     q.lat = nullptr;
