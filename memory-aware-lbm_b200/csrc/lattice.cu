@@ -171,9 +171,9 @@ int Lattice::create(int lx_, int ly_, int precision_, int scheme_)
                             16 * (size_t)d.g.nb * sizeof(double), 2 * (size_t)(ly + 2) * sizeof(double),
                             4 * (size_t)d.g.nb * sizeof(int)};
     size_t at[9] = {0};
+    for (int k = 0; k < 8; ++k) {
         const size_t page = (size_t)2 << 20;
         if (part[k] >= page) at[k] = (at[k] + page - 1) / page * page;
-    for (int k = 0; k < 8; ++k) {
         at[k + 1] = at[k] + (part[k] + 255) / 256 * 256;
         bytes += part[k];
     }
