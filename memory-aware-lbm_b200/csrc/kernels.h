@@ -16,6 +16,7 @@ struct DevLattice {
     int side_slot[2];    // the slot of each collision parity
     int ghost_flip;      // 1: the ring that belongs to the second buffer is in the current one (launch_tile)
     int rules_inside;    // some node off the perimeter has a boundary rule
+    int row_rules;       // more than half of the first and last rows' nodes have boundary rules
     int outlet_tiles;    // the extrapolated outlet's nodes lie where the tile kernel extrapolates them
     void *ghost2;        // AA only: the second buffer's ghost ring [9][nghost] (see logical())
     const uint8_t *tag;  // tag plane

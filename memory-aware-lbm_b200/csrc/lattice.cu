@@ -674,6 +674,7 @@ int Lattice::upload_tag_plane(const uint8_t *plane)
 int Lattice::upload_tags(const uint8_t *tag_xy, const uint8_t *zgb_row)
 {
     int inside = 0, outlet = lx >= 4;
+    long long rows = 0;
     for (int X = 0; X < lx + 2; ++X)
         for (int Y = 0; Y < ly + 2; ++Y) {
             const int t = tag_xy[(size_t)X * (ly + 2) + Y];
@@ -682,12 +683,14 @@ int Lattice::upload_tags(const uint8_t *tag_xy, const uint8_t *zgb_row)
             if (d.g.interior(X, Y) && t == LBGPU_TAG_NONE)
                 return set_error(LB_ERR_DYNAMICS, "interior node (%d,%d) has no dynamics", X, Y);
             if (t >= LBGPU_TAG_UPPER_ZOUHE && X > 1 && X < lx && Y > 1 && Y < ly) inside = 1;
+            if (t >= LBGPU_TAG_UPPER_ZOUHE && (Y == 1 || Y == ly)) ++rows;
             // an extrapolated row's pressure nodes anywhere but at its end, or the rows at the walls
             const bool right = t == LBGPU_TAG_RIGHT_PRESSURE_ZOUHE || t == LBGPU_TAG_RIGHT_PRESSURE_REGULARIZED;
             if (zgb_row && zgb_row[Y] && right && (X != lx || Y < 2 || Y > ly - 1)) outlet = 0;
         }
     LB_TRY(upload_tags_xy(tag_xy));
     d.rules_inside = inside;
+    d.row_rules = rows > lx;
     d.outlet_tiles = outlet;
     return LB_OK;
 }

@@ -261,6 +261,7 @@ int lbgpu_setup_cylinder(lbgpu_lattice *h, int obst_x, int obst_y, int obst_r, d
     if (int rc = lbgpu::cuda_error(cudaGetLastError(), "cylinder tags")) return rc;
     if (int rc = set_tables(L, omega, bc.data(), zgb.data())) return rc;
     L.d.rules_inside = 0;
+    L.d.row_rules = wall_kind == LBGPU_WALL_REGULARIZED;
     L.d.outlet_tiles = L.lx >= 4;
     L.reset_roles();
     L.launches = 0;

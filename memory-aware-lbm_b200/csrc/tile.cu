@@ -25,7 +25,7 @@ namespace {
 //     16384 x 4096 FP16 342 (single 388), with stochastic rounding 398 (single 398: its hash and
 //     multiplies bind), so those keep k_pull4h from 24M nodes on; 4096 x 1024 31 and 38.  Row-shifted FP16 110 (single
 //     117) at 8192 x 2048, 420 (408) at 16384 x 4096: from 24M nodes too; both together 34.9 (39.4) at 4096 x 1024,
-//     126 (117) at 8192 x 2048: from 8M.
+//     126 (117) at 8192 x 2048, 65.6 (62.4) at 6926 x 1153, 43.3 (41.5) at 7745 x 645, 40.8 (42.8) at 5438 x 906: from 4.7M.
 // Large lattices prefetch the tile 100 (FP64) or 200 (FP32) blocks ahead into L2: 253 -> 233 and 120 -> 109 us;
 // 0.3 of that distance does half as much, 4 times it costs 15-30 % (evicted before it is read).
 using F64Small = TileShape<double, 16, 8, 8, 704, 1>;
@@ -52,14 +52,83 @@ enum { TILE_SMALL = 0, TILE_MID = 1, TILE_WIDE = 2, TILE_LARGE = 3, TILE_NONE = 
 constexpr long long kF64[3] = {19 << 10, 120 << 10, 3 << 20};
 constexpr long long kF32[3] = {52 << 10, 100 << 10, 700 << 10};
 constexpr long long kHalf[3] = {60 << 10, 60 << 10, 2 << 20};
+bool elem16(const DevLattice &d) { return d.precision == LBGPU_F16 || d.precision == LBGPU_BF16; }
+
 // Up to here the small tiles (128 nodes) are one a SM, and take all its threads; beyond, two share one.
 constexpr long long kOneASm = 148 * 128;
 
-int tile_shape(const DevLattice &d)
+// Lattices that are only some tiles high or wide are nearly all halo and edge (us a step, single steps in parentheses):
+//   FP64 large tiles, 64 x 16: 250000 x 20 130 (122), 66 x 65000 211 (197), against 120 and 201 on 32 x 8 tiles, which
+//     are ahead up to 256 rows or columns, but for 12 to 16 rows; 33 to 64 columns are one tile of 64 x 16, ahead from
+//     600K nodes on: 33 x 20000 44 and 53 (51).
+//   16-bit tiles of 32 x 16, four steps, up to 35 rows (none of them off the perimeter): 250000 x 5 29 (27), 60000 x 32 22.3
+//     (19.6), against 22.6 and 18.0 on 64 x 12; the line lies where both run alike.
+//   Row-shifted offsets, whose four steps spill registers: 64 x 12 tiles are ahead from 600K nodes (1937 x 968 22.0 and
+//     15.4, single 21.3).
+int tile_shape(const DevLattice &d, bool rs)
+{
+    const int lx = d.g.lx, ly = d.g.ly;
+    const long long n = (long long)lx * ly;
+    const long long *k = d.precision == LBGPU_F64 ? kF64 : (d.precision == LBGPU_F32 ? kF32 : kHalf);
+    const int shape = n < k[0] ? TILE_SMALL : (n < k[1] ? TILE_MID : (n < k[2] ? TILE_WIDE : TILE_LARGE));
+    if (d.precision == LBGPU_F64 && shape >= TILE_WIDE) {
+        if (lx > 32 && lx <= 64) return n >= (600ll << 10) ? TILE_LARGE : TILE_WIDE;
+        if ((ly < 256 && (ly < 12 || ly > 16)) || lx < 256) return TILE_WIDE;
+    }
+    if (shape == TILE_WIDE && elem16(d) &&
+        n >= (d.g.shift_u ? 600ll << 10 : (ly <= 35 ? (rs ? 700ll << 10 : 1ll << 20) : kHalf[2])))
+        return TILE_LARGE;
+    return shape;
+}
+
+// Lattices whose single steps are the faster way for their shape (the same sweeps): a few long rows, whose nodes are
+// nearly all computed in tiles of edges, while a single step streams them well.  `rules`: where the first and
+// last row are boundary rules, which every tile then lists.
+struct Flat {
+    int rows, to;              // rows of the lattice
+    long long nodes, below;    // its nodes
+    int ratio;                 // nodes a row for each row, at least
+    bool rules;
+};
+constexpr long long kK = 1 << 10, kM = 1 << 20, kAny = 1ll << 62;
+// FP64 60000 x 10 22.3 (16.4), 1000000 x 3 142 (97); 12 to 14 rows fill a tile of 64 x 16: 1000000 x 12 278 (291).  Rules: 250000 x
+// 20 189 (136), 8000 x 16 9.3 (6.5).
+constexpr Flat kFlat64[] = {{1, 11, 170 * kK, kAny, 0, false}, {12, 14, 170 * kK, 3 * kM, 0, false}, {15, 16, 900 * kK, kAny, 0, false},
+                            {1, 48, 170 * kK, kAny, 0, true}, {1, 48, 100 * kK, kAny, 300, true}};
+// FP32 60000 x 3 8.7 (6.2), 1000000 x 5 90 (76).  Rules: 60000 x 10 15.4 (10.5), 20000 x 32 12.3 (10.3), 1000000 x 16 263 (241).
+constexpr Flat kFlat32[] = {{1, 8, 170 * kK, kAny, 0, false}, {1, 32, 150 * kK, 1300 * kK, 500, true},
+                            {1, 20, 1300 * kK, 2 * kM, 500, true}, {1, 16, 2 * kM, kAny, 500, true}};
+// 16-bit: two rows of tiles of 64 x 12, none off the perimeter: 1000000 x 16 184 (152).  Rules: 250000 x 3 43.5 (28.7), 1000000 x
+// 32 320 (282).
+constexpr Flat kFlat16[] = {{13, 25, 1 * kM, kAny, 0, false}, {1, 12, 500 * kK, kAny, 0, true}, {26, 35, 4 * kM, kAny, 0, true}};
+// with stochastic rounding 60000 x 24 23 (16.7), 1000000 x 8 118 (108).  Rules: 60000 x 5 13.9 (12.3), 250000 x 48 124 (112).
+constexpr Flat kFlat16R[] = {{13, 35, 700 * kK, kAny, 0, false}, {1, 12, 6 * kM, kAny, 0, false}, {1, 12, 290 * kK, kAny, 0, true},
+                             {1, 56, 6 * kM, kAny, 0, true}};
+// with a row shift 60000 x 24 30.6 (14.9), 20000 x 20 11.2 (8.2); from 64 rows on both run alike.  Rules: 60000 x 64 37.9 (34.9).
+constexpr Flat kFlat16B[] = {{1, 63, 250 * kK, kAny, 64, false}, {1, 63, 58 * kK, kAny, 256, false}, {64, 100, 3 * kM, kAny, 64, true}};
+// with both 60000 x 96 54 (47), 20000 x 32 15.4 (10.2).
+constexpr Flat kFlat16BR[] = {{1, 1 << 30, 250 * kK, kAny, 64, false}, {1, 1 << 30, 58 * kK, kAny, 128, false}};
+
+template <size_t N>
+bool on_lines(const Flat (&lines)[N], const DevLattice &d, bool outlet)
 {
     const long long n = (long long)d.g.lx * d.g.ly;
-    const long long *k = d.precision == LBGPU_F64 ? kF64 : (d.precision == LBGPU_F32 ? kF32 : kHalf);
-    return n < k[0] ? TILE_SMALL : (n < k[1] ? TILE_MID : (n < k[2] ? TILE_WIDE : TILE_LARGE));
+    for (const Flat &f : lines)
+        if (d.g.ly >= f.rows && d.g.ly <= f.to && n >= f.nodes && n < f.below && d.g.lx >= (long long)f.ratio * d.g.ly &&
+            (d.row_rules || !f.rules) &&
+            // the pass of an extrapolated outlet makes a single step longer, but for FP64's rules
+            (!outlet || n >= kM || (f.rules && d.precision == LBGPU_F64)))
+            return true;
+    return false;
+}
+
+bool too_flat(const DevLattice &d, bool outlet, bool rs)
+{
+    if (d.precision == LBGPU_F64)      // and narrow ones: 66 x 65000 201 (197)
+        return on_lines(kFlat64, d, outlet) || (d.g.lx > 64 && d.g.lx <= 100 && (long long)d.g.lx * d.g.ly >= 4 * kM);
+    if (d.precision == LBGPU_F32) return on_lines(kFlat32, d, outlet);
+    if (d.g.shift_u) return rs ? on_lines(kFlat16BR, d, outlet) : on_lines(kFlat16B, d, outlet);
+    return rs ? on_lines(kFlat16R, d, outlet) : on_lines(kFlat16, d, outlet);
 }
 
 template <class SH, int M, bool EXTRAP>
@@ -133,12 +202,12 @@ void launch_half(const DevLattice &d, int src, int n_par, int T, bool outlet, co
 
 int tile_steps(const DevLattice &d, long long steps, bool outlet, bool rs)
 {
-    if (steps < 2 || (outlet && !d.outlet_tiles)) return 0;
-    const int shape = tile_shape(d);
-    if (d.precision == LBGPU_F16 || d.precision == LBGPU_BF16) {
-        if (d.g.shift_u && (outlet || !d.side_extra)) return 0;
+    if (steps < 2 || (outlet && !d.outlet_tiles) || too_flat(d, outlet, rs)) return 0;
+    const int shape = tile_shape(d, rs);
+    if (elem16(d)) {
+        if (d.g.shift_u && outlet) return 0;
         const long long nodes = (long long)d.g.lx * d.g.ly;
-        if (nodes >= ((rs && d.g.shift_u ? 8ll : 24ll) << 20) && (rs || d.g.shift_u)) return 0;
+        if (nodes >= (rs && d.g.shift_u ? 9ll << 19 : 24ll << 20) && (rs || d.g.shift_u)) return 0;
         return shape == TILE_SMALL && steps >= 8 && !d.g.shift_u ? 8 : (steps >= 4 && shape != TILE_LARGE ? 4 : 2);
     }
     if (shape == TILE_SMALL && steps >= 8) return 8;
@@ -148,7 +217,7 @@ int tile_steps(const DevLattice &d, long long steps, bool outlet, bool rs)
 
 void launch_tile(const DevLattice &d, int src, int n_par, int T, bool outlet, const unsigned *keys, cudaStream_t s)
 {
-    const int shape = tile_shape(d);
+    const int shape = tile_shape(d, keys[0] != 0);
     switch (d.precision) {
     case LBGPU_F64:
         if (T == 8) launch_one<F64Small>(d, src, n_par, outlet, 0, keys, s);
