@@ -86,6 +86,15 @@ namespace {
 
 int batch_error(cudaError_t e, const char *what) { return lbgpu::cuda_error(e, what); }
 
+// Where a member's next step starts from.
+void start_of(const Lattice &L, int &cur0, int &phase0, int &tau0)
+{
+    const bool pull = L.scheme == LBGPU_PULL, natural = L.form == lbgpu::FORM_L;
+    cur0 = pull ? L.cur : 0;
+    phase0 = pull || natural ? 0 : 1;
+    tau0 = (int)(pull || !natural ? L.n + 1 : L.n);
+}
+
 // Descriptor of a member from its lattice state (see kernels.h BatchInst).
 BatchInst describe(const Lattice &L)
 {
@@ -94,27 +103,14 @@ BatchInst describe(const Lattice &L)
     b.buf[0] = L.d.buf[0];
     b.buf[1] = L.d.buf[1];
     b.side = L.d.side;
-    for (int p = 0; p < 2; ++p) {
-        const int slot = L.d.side_slot[p];
-        b.side_of[p] = slot == 3 ? L.d.side_extra : static_cast<char *>(L.d.side) + (size_t)slot * 9 * (size_t)L.d.g.nper * L.elem;
-    }
-    b.side_slot[0] = L.d.side_slot[0];
-    b.side_slot[1] = L.d.side_slot[1];
+    b.side_slot = lbgpu::batch_side_slots(L.d.side_slot[0], L.d.side_slot[1]);
     b.tag = L.d.tag;
     b.bc = L.d.bc;
     b.omega = L.d.omega;
     b.scale = L.d.scale;
     b.inv_scale = L.d.inv_scale;
     b.scheme = L.scheme;
-    if (L.scheme == LBGPU_PULL) {
-        b.cur0 = L.cur;
-        b.phase0 = 0;
-        b.tau0 = (int)(L.n + 1);
-    } else {
-        b.cur0 = 0;
-        b.phase0 = (L.form == lbgpu::FORM_L) ? 0 : 1;
-        b.tau0 = (int)((L.form == lbgpu::FORM_L) ? L.n : L.n + 1);
-    }
+    start_of(L, b.cur0, b.phase0, b.tau0);
     b.rs = L.rs ? 1 : 0;
     b.rs_seed = L.rs_seed;
     b.rules_inside = L.d.rules_inside;
@@ -125,11 +121,12 @@ BatchInst describe(const Lattice &L)
 // the parity only.
 bool describes(const BatchInst &b, const Lattice &L)
 {
-    const BatchInst now = describe(L);
-    return b.rs == now.rs && b.rs_seed == now.rs_seed && b.g.shift_u == now.g.shift_u && b.cur0 == now.cur0 &&
-           b.phase0 == now.phase0 && (now.rs ? b.tau0 == now.tau0 : ((b.tau0 ^ now.tau0) & 1) == 0) && b.side_slot[0] == now.side_slot[0] &&
-           b.side_slot[1] == now.side_slot[1] && b.omega == now.omega && b.scale == now.scale &&
-           b.rules_inside == now.rules_inside;
+    int cur0, phase0, tau0;
+    start_of(L, cur0, phase0, tau0);
+    return b.rs == (L.rs ? 1 : 0) && b.rs_seed == L.rs_seed && b.g.shift_u == L.d.g.shift_u && b.cur0 == cur0 &&
+           b.phase0 == phase0 && (L.rs ? b.tau0 == tau0 : ((b.tau0 ^ tau0) & 1) == 0) &&
+           b.side_slot == lbgpu::batch_side_slots(L.d.side_slot[0], L.d.side_slot[1]) && b.omega == L.d.omega &&
+           b.scale == L.d.scale && b.rules_inside == L.d.rules_inside;
 }
 
 // Stochastically rounded members key their collisions by number (tau0 + k), which a replayed
@@ -148,22 +145,21 @@ int refresh_collision_numbers(lbgpu_batch *b, int done)
 
 // The descriptors after an odd number of two-step launches, on the device: what describe() gives then, but for the
 // collision number, whose parity stays.  A new copy from the host's memory would make the call wait.
-__global__ void k_batch_turn(BatchInst *insts, int n, int elem)
+__global__ void k_batch_turn(BatchInst *insts, int n, bool half)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n || insts[i].scheme != LBGPU_PULL) return;
     BatchInst &d = insts[i];
-    const int a = d.tau0 & 1, spare = 3 - d.side_slot[0] - d.side_slot[1];
-    d.side_slot[a] = spare;
-    d.side_of[a] = static_cast<char *>(d.side) + (size_t)spare * 9 * (size_t)d.g.nper * elem;
+    const int a = d.tau0 & 1, now = lbgpu::batch_side_slot(d.side_slot, a), last = lbgpu::batch_side_slot(d.side_slot, 1 - a);
+    const int spare = half ? now ^ 2 : 3 - now - last;      // side_other
+    d.side_slot = a ? lbgpu::batch_side_slots(last, spare) : lbgpu::batch_side_slots(spare, last);
     d.cur0 ^= 1;
 }
 
 int turn_descriptors(lbgpu_batch *b)
 {
     const int n = (int)b->members.size();
-    const int elem = b->precision == LBGPU_F64 ? 8 : (b->precision == LBGPU_F32 ? 4 : 2);
-    k_batch_turn<<<(n + 127) / 128, 128, 0, b->stream>>>(b->d_inst, n, elem);
+    k_batch_turn<<<(n + 127) / 128, 128, 0, b->stream>>>(b->d_inst, n, b->precision == LBGPU_F16 || b->precision == LBGPU_BF16);
     for (int i = 0; i < n; ++i)
         if (b->members[i]) b->h_inst[i] = describe(b->members[i]->L);
     return batch_error(cudaGetLastError(), "batch descriptors");

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include "layout.cuh"
+#include "lbgpu.h"
 
 namespace lbgpu {
 
@@ -11,8 +12,7 @@ struct DevLattice {
     Geo g;
     int precision;       // LBGPU_F64 / F32 / F16 / BF16: element type of buf and side
     void *buf[2];        // population buffers (buf[1] unused by the AA scheme)
-    void *side;          // stale-slot store: slots of [9][nper], two (AA) or three (pull)
-    void *side_extra;    // a fourth slot, of pull lattices with row-shifted offsets
+    void *side;          // stale-slot store: side_slots() slots of [9][nper]
     int side_slot[2];    // the slot of each collision parity
     int ghost_flip;      // 1: the ring that belongs to the second buffer is in the current one (launch_tile)
     int rules_inside;    // some node off the perimeter has a boundary rule
@@ -27,23 +27,18 @@ struct DevLattice {
     float scale, inv_scale;  // FP16/BF16 offset storage: stored = (f - w) * scale
 };
 
-// The k-th slot (0, 1) that holds neither parity's stale slots; slot 3 counts where there is one.
-inline int side_free(const DevLattice &d, int k)
+// The side store's slots: AA two; pull three (FP64, FP32), or four for 16-bit storage, whose row-shifted tiles write both
+// parities' slots beside those they read.
+inline int side_slots(int precision, int scheme)
 {
-    for (int s = 0; s < 4; ++s)
-        if (s != d.side_slot[0] && s != d.side_slot[1] && (s < 3 || d.side_extra) && k-- == 0) return s;
-    return -1;
+    return scheme == LBGPU_AA ? 2 : (precision == LBGPU_F64 || precision == LBGPU_F32 ? 3 : 4);
 }
-
-// The slots a tile launch writes beside those in use: `prev` for the parity of the last collision but one, a (the
-// parity whose stale slots step 1 reads), and with row-shifted offsets `last` for the other parity.  The order of
-// the two parities' slots is kept, so that a second launch from the same parity takes back the slots of the first.
-inline int side_prev(const DevLattice &d, int a)
+// The slot that a tile launch writes for parity p beside the one in use; the next launch from the same parity takes
+// that one back, so that two launches leave the slots where they were.
+inline int side_other(const DevLattice &d, int p)
 {
-    const int other = side_free(d, 1);
-    return other < 0 || d.side_slot[a] < d.side_slot[1 - a] ? side_free(d, 0) : other;
+    return d.precision == LBGPU_F64 || d.precision == LBGPU_F32 ? 3 - d.side_slot[0] - d.side_slot[1] : d.side_slot[p] ^ 2;
 }
-inline int side_last(const DevLattice &d, int a) { return side_free(d, d.side_slot[a] < d.side_slot[1 - a] ? 1 : 0); }
 
 // How the post-stream state is read from a buffer:
 //   VIEW_DIRECT        the buffer holds it (pull form L, or a collided state read as is)
@@ -116,21 +111,31 @@ constexpr int BATCH_KINDS = 5;
 // One lattice of a batch, with its state at the start of the current chunk of steps:
 // pull scheme: the buffer holding C_n is buf[cur0]; AA: phase0 0 = natural form, 1 = swapped;
 // tau0 = the time step the chunk's first launch executes (its side parity is tau0 & 1).
-struct BatchInst {
+// What every block reads lies in one 128-byte line (a second line: AA members of 1500 x 400 in FP32 124.7 us a step, 119.9
+// without it).
+struct alignas(128) BatchInst {
     Geo g;
     void *buf[2];
     void *side;
-    void *side_of[2];                 // of each collision parity
-    int side_slot[2];
     const uint8_t *tag;
     const double *bc;
     double omega;
     float scale, inv_scale;
+    int tau0;                         // tau0 + k: the collision number of step k of a chunk
+    int cur0;
+    int side_slot;                    // of each collision parity (batch_side_slot)
     int rules_inside;
-    int scheme, cur0, phase0, tau0;   // tau0 + k: the collision number of step k of a chunk
+    int scheme, phase0;
     unsigned rs_seed;                 // 16-bit members: stochastic rounding seed (rs != 0)
     int rs;
 };
+static_assert(sizeof(Geo) == 56 && sizeof(BatchInst) == 256, "the first line holds all up to rules_inside");
+
+// One word for both parities' slots: with a pointer for each the kernels keep what they can otherwise compute again, and
+// spill (FP16 pull, 32 registers: 104 bytes instead of 8; 64 channels of 100 x 60 with row-shifted offsets 25.9
+// us a step on one B200 instead of 22.9, AA ones in FP32 16.8 and 15.7).
+__host__ __device__ inline int batch_side_slot(int slots, int parity) { return (slots >> (8 * parity)) & 0xff; }
+__host__ __device__ inline int batch_side_slots(int even, int odd) { return even | (odd << 8); }
 
 // A strip of `passes` tiles of a lattice stacked in y, stepped by one block from the top down.
 // A tile: nodes x0 .. x0 + (32 << shape) - 1 and threads / (32 << shape) rows (BATCH_PULL4:

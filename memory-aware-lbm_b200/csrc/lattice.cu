@@ -164,8 +164,7 @@ int Lattice::create(int lx_, int ly_, int precision_, int scheme_)
     // extrapolated row.
     const size_t nbuf = (scheme == LBGPU_AA) ? 1 : 2;
     const size_t pbytes = 9 * (size_t)d.g.plane * elem;
-    // two parities, and for the pull scheme the slot the tile kernel writes beside them
-    const size_t sbytes = (scheme == LBGPU_PULL ? 3 : 2) * 9 * (size_t)d.g.nper * elem;
+    const size_t sbytes = (size_t)side_slots(precision, scheme) * 9 * (size_t)d.g.nper * elem;
     const size_t gbytes = scheme == LBGPU_AA ? 9 * (size_t)d.g.nghost() * elem : 0;
     const size_t part[8] = {pbytes, nbuf == 2 ? pbytes : 0, gbytes, sbytes, (size_t)d.g.plane,
                             16 * (size_t)d.g.nb * sizeof(double), 2 * (size_t)(ly + 2) * sizeof(double),
@@ -214,8 +213,7 @@ void Lattice::reset_roles()
 
 void *Lattice::side_ptr(int p) const
 {
-    const int slot = d.side_slot[p];
-    return slot == 3 ? d.side_extra : static_cast<char *>(d.side) + (size_t)slot * 9 * (size_t)d.g.nper * elem;
+    return static_cast<char *>(d.side) + (size_t)d.side_slot[p] * 9 * (size_t)d.g.nper * elem;
 }
 
 // Whether the caller captures the stream; remembered, because its graph holds the buffers and slots of now.
@@ -390,9 +388,9 @@ int Lattice::step(int nsteps)
 
 void Lattice::after_tile(int T)
 {
-    const int a = (int)((n + 1) & 1), prev = side_prev(d, a), last = side_last(d, a);
-    d.side_slot[a] = prev;
-    if (d.g.shift_u) d.side_slot[1 - a] = last;
+    const int a = (int)((n + 1) & 1);
+    d.side_slot[a] = side_other(d, a);
+    if (d.g.shift_u) d.side_slot[1 - a] = side_other(d, 1 - a);
     d.ghost_flip ^= 1;
     cur = 1 - cur;
     n += T;

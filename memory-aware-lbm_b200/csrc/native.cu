@@ -132,21 +132,9 @@ int lbgpu_set_offset_shift(lbgpu_lattice *h, const double *u_row)
         return set_error(LB_ERR_STATE, "lbgpu_set_offset_shift: FP16/BF16 storage only");
     if (!u_row) {
         if (L.shift) {
-            // the fourth slot goes with the table: what it holds moves to a free one of the three
-            for (int p = 0; p < 2; ++p)
-                if (L.d.side_slot[p] == 3) {
-                    const int to = lbgpu::side_free(L.d, 0);
-                    const size_t bytes = 9 * (size_t)L.d.g.nper * L.elem;
-                    if (int rc = lbgpu::cuda_error(cudaMemcpyAsync(static_cast<char *>(L.d.side) + (size_t)to * bytes,
-                                                                   L.d.side_extra, bytes, cudaMemcpyDeviceToDevice, L.stream),
-                                                   "lbgpu_set_offset_shift"))
-                        return rc;
-                    L.d.side_slot[p] = to;
-                }
             if (int rc = lbgpu::cuda_error(cudaStreamSynchronize(L.stream), "lbgpu_set_offset_shift")) return rc;
             cudaFree(L.shift);
         }
-        L.d.side_extra = nullptr;
         L.shift = nullptr;
         L.d.g.shift_u = nullptr;
         return LB_OK;
@@ -173,12 +161,8 @@ int lbgpu_set_offset_shift(lbgpu_lattice *h, const double *u_row)
         }
     if (!L.shift) {
         void *p = nullptr;
-        // the table, and for the pull scheme a fourth slot of the side store (launch_tile)
-        const size_t table = (u.size() * sizeof(float) + 255) / 256 * 256;
-        const size_t slot = L.scheme == LBGPU_PULL ? 9 * (size_t)L.d.g.nper * L.elem : 0;
-        if (int rc = lbgpu::cuda_error(cudaMalloc(&p, table + slot), "cudaMalloc(offset shift)")) return rc;
+        if (int rc = lbgpu::cuda_error(cudaMalloc(&p, u.size() * sizeof(float)), "cudaMalloc(offset shift)")) return rc;
         L.shift = static_cast<float *>(p);
-        L.d.side_extra = slot ? static_cast<char *>(p) + table : nullptr;
     }
     if (int rc = lbgpu::cuda_error(cudaMemcpyAsync(L.shift, u.data(), u.size() * sizeof(float),
                                                    cudaMemcpyHostToDevice, L.stream), "upload offset shift"))

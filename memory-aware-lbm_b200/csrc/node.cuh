@@ -370,10 +370,10 @@ template <class S> S *OTHER(const DevLattice &d, int cur)
 {
     return d.buf[1] ? static_cast<S *>(d.buf[(1 - cur) ^ d.ghost_flip]) : static_cast<S *>(d.ghost2);
 }
-// The side store's slots: two or three in it, the fourth of row-shifted pull lattices beside it; a parity's.
+// A slot of the side store; a parity's.
 template <class S> S *SIDE_SLOT(const DevLattice &d, int slot)
 {
-    return slot == 3 ? static_cast<S *>(d.side_extra) : static_cast<S *>(d.side) + (size_t)slot * 9 * (size_t)d.g.nper;
+    return static_cast<S *>(d.side) + (size_t)slot * 9 * (size_t)d.g.nper;
 }
 template <class S> S *SIDE(const DevLattice &d, int p) { return SIDE_SLOT<S>(d, d.side_slot[p & 1]); }
 

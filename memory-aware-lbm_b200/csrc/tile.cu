@@ -145,13 +145,12 @@ void launch_shape(const DevLattice &d, int src, int n_par, int pf, const unsigne
     a.omega = d.omega;
     a.omega_f = (float)d.omega;
     // step 1 reads the stale slots of C_{n-1}; the last step's replace those of C_n, which has them in
-    // its own slots, and the step's before it go to the free slot.  Row-shifted offsets read C_n's from
+    // its own slots, and the step's before it go to a free slot.  Row-shifted offsets read C_n's from
     // the side store too (its own slots are rebased), so both go to free slots, of four.
     a.stale1 = SIDE<S>(d, n_par + 1);
     a.stale2 = SIDE<S>(d, n_par);
-    const int ap = (n_par + 1) & 1;
-    a.out_last = (M & TILE_SHIFT) ? SIDE_SLOT<S>(d, side_last(d, ap)) : SIDE<S>(d, n_par);
-    a.out_prev = SIDE_SLOT<S>(d, side_prev(d, ap));
+    a.out_last = (M & TILE_SHIFT) ? SIDE_SLOT<S>(d, side_other(d, n_par)) : SIDE<S>(d, n_par);
+    a.out_prev = SIDE_SLOT<S>(d, side_other(d, 1 - n_par));
     a.sc = d.scale;
     a.inv = d.inv_scale;
     // the outlet's extrapolation reads three columns back: its tile must not be narrower

@@ -628,11 +628,12 @@ __global__ void __launch_bounds__(SH::NT, SH::MINB) k_batch_tile(const BatchInst
     a.omega = d.omega;
     a.omega_f = (float)d.omega;
     const size_t slot = 9 * (size_t)d.g.nper;
-    const int now = d.side_slot[pa], spare = 3 - d.side_slot[0] - d.side_slot[1];
+    const int now = batch_side_slot(d.side_slot, pa), last = batch_side_slot(d.side_slot, pa ^ 1);
+    const int spare = sizeof(S) == 2 ? now ^ 2 : 3 - now - last;              // side_other
     S *side = static_cast<S *>(d.side);
     a.stale1 = side + slot * ((unit & 1) ? spare : now);
     a.out_prev = side + slot * ((unit & 1) ? now : spare);
-    a.out_last = side + slot * d.side_slot[pa ^ 1];
+    a.out_last = side + slot * last;
     a.sc = d.scale;
     a.inv = d.inv_scale;
     a.x_first = 1;
