@@ -446,6 +446,12 @@ int lbgpu_batch_remove(lbgpu_batch *b, int slot)
     return LB_OK;
 }
 
+static int not_captured()
+{
+    return set_error(LB_ERR_STATE, "lbgpu_batch_step: a captured call takes an even number of steps, of members without "
+                     "stochastic rounding that have stepped in the batch since they last changed");
+}
+
 int lbgpu_batch_size(lbgpu_batch *b)
 {
     if (!b) return 0;
@@ -527,37 +533,28 @@ int lbgpu_batch_step(lbgpu_batch *b, int nsteps)
     if (!b || nsteps < 0) return set_error(LB_ERR_ARG, "lbgpu_batch_step: bad arguments");
     b->launches = 0;
     if (nsteps == 0 || lbgpu_batch_size(b) == 0) return LB_OK;
-    // A member whose stream was captured keeps its buffers in place over an even number of steps (Lattice::step); a
-    // capture of a member's stream takes the batch's stream in.
-    bool capturing = false, keep = false;
-    for (lbgpu_lattice *m : b->members) {
-        bool c = false;
-        if (m)
-            if (int rc = m->L.see_capture(c)) return rc;
-        capturing = capturing || c;
-    }
-    for (lbgpu_lattice *m : b->members)
-        if (m) {
-            m->L.keep_roles = m->L.keep_roles || capturing;
-            keep = keep || m->L.keep_roles;
-        }
-    bool any_rs = false;
-    for (lbgpu_lattice *m : b->members)
-        if (m && m->L.rs) any_rs = true;
     // A member that needs its first step on its own (see needs_own_step) makes every member
     // take that step on its own path (the same per-node arithmetic as the batch kernel).
-    bool own = false;
+    bool any_rs = false, own = false, keep = false;
     for (lbgpu_lattice *m : b->members)
-        if (m && needs_own_step(m->L)) own = true;
-    if (capturing) {
-        // nothing that waits or copies from the host's memory can be captured
-        bool ready = !own && !any_rs && !(nsteps & 1) && !b->dirty;
-        for (size_t i = 0; i < b->members.size() && ready; ++i)
-            if (b->members[i]) ready = i < b->h_inst.size() && describes(b->h_inst[i], b->members[i]->L);
-        if (!ready)
-            return set_error(LB_ERR_STATE, "lbgpu_batch_step: a captured call takes an even number of steps, of members "
-                             "without stochastic rounding that have stepped in the batch since they last changed");
-    }
+        if (m) {
+            any_rs = any_rs || m->L.rs;
+            own = own || needs_own_step(m->L);
+            keep = keep || m->L.keep_roles;
+        }
+    // what a member's descriptor says no longer holds: rounding switched (or reseeded), a row shift set or
+    // cleared, another geometry, or the member stepped on its own since
+    for (size_t i = 0; i < b->members.size() && !b->dirty; ++i)
+        if (b->members[i] && (i >= b->h_inst.size() || !describes(b->h_inst[i], b->members[i]->L))) b->dirty = true;
+    // Nothing that waits or copies from the host's memory can be captured.  (Elsewhere the batch's own stream is asked,
+    // once: it is part of a capture when it waits for a member's.)
+    if (own || b->dirty)
+        for (lbgpu_lattice *m : b->members) {
+            bool capturing = false;
+            if (m)
+                if (int rc = m->L.see_capture(capturing)) return rc;
+            if (capturing) return not_captured();
+        }
     if (own) {
         for (lbgpu_lattice *m : b->members) {
             if (!m) continue;
@@ -570,13 +567,22 @@ int lbgpu_batch_step(lbgpu_batch *b, int nsteps)
         --nsteps;
         b->dirty = true;
     }
-    // what a member's descriptor says no longer holds: rounding switched (or reseeded), a row shift set or
-    // cleared, another geometry, or the member stepped on its own since
-    for (size_t i = 0; i < b->members.size() && !b->dirty; ++i)
-        if (b->members[i] && (i >= b->h_inst.size() || !describes(b->h_inst[i], b->members[i]->L))) b->dirty = true;
     if (b->dirty)
         if (int rc = rebuild(b)) return rc;
     if (int rc = order_before(b)) return rc;
+    // A member whose stream is or was captured keeps its buffers in place over an even number of steps (Lattice::step).
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (int rc = batch_error(cudaStreamIsCapturing(b->stream, &status), "cudaStreamIsCapturing")) return rc;
+    const bool capturing = status != cudaStreamCaptureStatusNone;
+    if (capturing) {
+        if (any_rs || (nsteps & 1)) {
+            order_after(b);
+            return not_captured();
+        }
+        for (lbgpu_lattice *m : b->members)
+            if (m) m->L.keep_roles = true;
+        keep = true;
+    }
     // An odd count takes its single step first: what follows runs in pairs of steps.
     if (nsteps & 1) {
         launch_step(b, 0, false);
