@@ -3,7 +3,7 @@
 // State convention shared by every kernel here (n = index of the last collision):
 //   pull form L : buffer `cur` holds the post-stream populations L_m, stale slots included.
 //   pull form C : buffer `cur` holds the post-collision populations C_n; the post-stream state
-//                 L_{n+1} is "C_n streamed", read through logical().
+//                 L_{n+1} is "C_n streamed", read through logical_at().
 //   AA natural  : the AA buffer holds L_m in each node's own slots (stale slots in the side store).
 //   AA swapped  : the AA buffer holds C_n of direction i in slot opp(i) of each node.
 //   side store parity p = k & 1 holds the post-collision values C_k of the perimeter nodes'
@@ -882,8 +882,10 @@ __device__ __forceinline__ void readout_block(const Geo &g, int view, const S *_
     {
         const int c = threadIdx.x & 31, r = threadIdx.x >> 5, X = Xb + c, Y = Yb + r;
         if (X < X1 && Y <= g.ly + 1) {
+            typename Codec<S>::R f[9];
+            logical_node(g, view, cur, other, side, X, Y, inv, f);
 #pragma unroll
-            for (int i = 0; i < 9; ++i) rec[c][r * rs + i] = (double)logical(g, view, cur, other, side, X, Y, i, inv);
+            for (int i = 0; i < 9; ++i) rec[c][r * rs + i] = (double)f[i];
             if (rs > 9) rec[c][r * rs + 9] = dynp ? __longlong_as_double((long long)dynp[(size_t)X * (g.ly + 2) + Y]) : 0.0;
         }
     }
@@ -943,8 +945,7 @@ __device__ __forceinline__ double state_density(const Geo &g, int view, const S 
                                                 const S *__restrict__ side, int X, int Y, float inv)
 {
     typename Codec<S>::R f[9];
-#pragma unroll
-    for (int i = 0; i < 9; ++i) f[i] = logical(g, view, cur, other, side, X, Y, i, inv);
+    logical_node(g, view, cur, other, side, X, Y, inv, f);
     return (double)rules::density(f);
 }
 
@@ -1110,7 +1111,8 @@ __global__ void __launch_bounds__(RED_THREADS) k_moments_rows(Geo g, int view, c
         int tags[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const int X = min(Xu + u * RED_THREADS, g.lx);
+            const int X = Xu + u * RED_THREADS;
+            if (X > g.lx) break;
             load_state(g, view, cur, other, side, X, Y, inv, w[u]);
             tags[u] = tag[g.idx(X, Y)];
         }

@@ -18,7 +18,7 @@ struct DevLattice {
     int rules_inside;    // some node off the perimeter has a boundary rule
     int row_rules;       // more than half of the first and last rows' nodes have boundary rules
     int outlet_tiles;    // the extrapolated outlet's nodes lie where the tile kernel extrapolates them
-    void *ghost2;        // AA only: the second buffer's ghost ring [9][nghost] (see logical())
+    void *ghost2;        // AA only: the second buffer's ghost ring [9][nghost] (see logical_at())
     const uint8_t *tag;  // tag plane
     double *bc;          // boundary tables [8][2][nb]
     const int *zgb_src;  // [4][nb]: pressure-table slot -> source row of its ZGB density, or -1

@@ -211,11 +211,6 @@ void Lattice::reset_roles()
     form = FORM_L; pending = 0; n = 0;
 }
 
-void *Lattice::side_ptr(int p) const
-{
-    return static_cast<char *>(d.side) + (size_t)d.side_slot[p] * 9 * (size_t)d.g.nper * elem;
-}
-
 // Whether the caller captures the stream; remembered, because its graph holds the buffers and slots of now.
 int Lattice::see_capture(bool &capturing)
 {
@@ -402,8 +397,11 @@ long long Lattice::steps_done() const
     return n;
 }
 
-// Results up to this size are copied from a device buffer; larger ones go through read_back.
-static constexpr size_t kStagedBytes = (size_t)1 << 20;
+// Results up to this size are copied from a device buffer; larger ones go through read_back.  us a call on one B200, buffer
+// and read_back: fields 400 x 90 (0.9 MB) 109 and -, 400 x 120 (1.2 MB) 129 and 103; velocity averages 250 x 51 48 and
+// 102; populations, whose chunks of columns are transposed, 600 x 150 (6.7 MB) 365 and 461, 700 x 200 (10 MB) 537
+// and 424.
+static constexpr size_t kStagedBytes = (size_t)1 << 20, kStagedPops = (size_t)8 << 20;
 
 // ---- data movement --------------------------------------------------------------------
 int Lattice::ensure_stage(size_t need)
@@ -498,7 +496,7 @@ int Lattice::readout_records(double *host, int rs, const uint64_t *dynp_dev, int
 int Lattice::readout_populations(double *host)
 {
     // small ones through the device staging: pinned memory that nobody holds yet takes 1.7 ms to get
-    if ((size_t)(lx + 2) * (ly + 2) * 72 <= kStagedBytes) return readout_records(host, 9, nullptr, 0, lx + 2);
+    if ((size_t)(lx + 2) * (ly + 2) * 72 <= kStagedPops) return readout_records(host, 9, nullptr, 0, lx + 2);
     int v, par;
     view(v, par);
     const size_t col = (size_t)(ly + 2) * 9;
@@ -610,6 +608,27 @@ int Lattice::velocity_average(double *ux, double *uy, long long *samples)
     if (!vel_acc || vel_samples == 0) return set_error(LB_ERR_STATE, "no velocity samples accumulated");
     const double k = 1.0 / (double)vel_samples;
     double *const to[2] = {ux, uy};
+    if (2 * nn * sizeof(double) <= kStagedBytes) {
+        // small: copied from a device buffer, or the smallest as they are and scaled here (20 x 16 27 us instead of 32)
+        const bool here = nn <= 4096;
+        const double *from = vel_acc;
+        if (!here) {
+            LB_TRY(ensure_stage(2 * nn * sizeof(double)));
+            launch_scaled(vel_acc, k, stage, 2 * (long long)nn, stream);
+            LB_TRY(check("velocity average"));
+            from = stage;
+        }
+        for (int j = 0; j < 2; ++j)
+            if (to[j]) {
+                LB_CUDA(cudaMemcpyAsync(to[j], from + j * nn, nn * sizeof(double), cudaMemcpyDeviceToHost, stream), "velocity average");
+                d2h_bytes += nn * sizeof(double);
+            }
+        LB_CUDA(cudaStreamSynchronize(stream), "velocity average");
+        if (here)
+            for (double *p : to)
+                for (size_t x = 0; p && x < nn; ++x) p[x] *= k;
+        return LB_OK;
+    }
     for (int j = 0; j < 2; ++j) {
         if (!to[j]) continue;
         const cudaError_t e = read_back(

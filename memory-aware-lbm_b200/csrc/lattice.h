@@ -65,7 +65,6 @@ struct Lattice {
     int create(int lx, int ly, int precision, int scheme);
     void destroy();
     void reset_roles();
-    void *side_ptr(int p) const;          // the side store's slot of collision parity p
     int see_capture(bool &capturing);
 
     // per-step operations (asynchronous on `stream`)

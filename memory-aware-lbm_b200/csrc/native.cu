@@ -254,10 +254,9 @@ int lbgpu_setup_cylinder(lbgpu_lattice *h, int obst_x, int obst_y, int obst_r, d
             if (int rc = lbgpu::cuda_error(cudaMemsetAsync(L.d.buf[b], 0, 9 * (size_t)L.d.g.plane * L.elem,
                                                            L.stream), "clear populations"))
                 return rc;
-    for (int p = 0; p < 2; ++p)
-        if (int rc = lbgpu::cuda_error(cudaMemsetAsync(L.side_ptr(p), 0, 9 * (size_t)L.d.g.nper * L.elem, L.stream),
-                                       "clear side store"))
-            return rc;
+    if (int rc = lbgpu::cuda_error(cudaMemsetAsync(L.d.side, 0, lbgpu::side_slots(L.precision, L.scheme) * 9 *
+                                                   (size_t)L.d.g.nper * L.elem, L.stream), "clear side store"))
+        return rc;
     if (int rc = L.init_cylinder(umax)) return rc;
     // second buffer zero (reference calloc, lb.c:91-92): side parity 1 stays zero; the AA scheme
     // reads the initial state's own stale slots from parity 0

@@ -54,36 +54,41 @@ __device__ __forceinline__ void collide_node(const double *__restrict__ bc, cons
 template <class S>
 __device__ __forceinline__ typename Codec<S>::R dec_row(const Geo &g, S v, int i, float inv, int Y);
 
-// Post-stream value of slot i at node (X, Y), any node of the lattice including the ghost
+// Where the post-stream value of slot i at node (X, Y) lies, any node of the lattice including the ghost
 // ring, under each view (kernels.h).  Ghost slots that no interior node streams into keep the
 // content of the buffer the state lives in, as in the reference: for the pull scheme `other`
 // is the second buffer; for the AA scheme's swapped view (an odd step count, which the
 // reference leaves in its second buffer) `other` is that buffer's saved ghost ring
 // [9][nghost].
 template <class S>
-__device__ __forceinline__ typename Codec<S>::R logical(const Geo &g, int view, const S *__restrict__ cur,
-                                                        const S *__restrict__ other,
-                                                        const S *__restrict__ side, int X, int Y,
-                                                        int i, float inv)
+__device__ __forceinline__ const S *logical_at(const Geo &g, int view, const S *__restrict__ cur, const S *__restrict__ other,
+                                               const S *__restrict__ side, int X, int Y, int i)
 {
-    using C = Codec<S>;
     const int sx = X - cx(i), sy = Y - cy(i);
+    const bool streamed = g.interior(sx, sy), inside = g.interior(X, Y);
+    const S *stale = side + ((size_t)i * g.nper + g.pidx(X, Y));
     switch (view) {
-    case VIEW_PULL_PENDING:
-        if (g.interior(sx, sy)) return dec_row<S>(g, plane(cur, g, i)[g.idx(sx, sy)], i, inv, Y);
-        if (g.interior(X, Y)) return dec_row<S>(g, side[(size_t)i * g.nper + g.pidx(X, Y)], i, inv, Y);
-        return dec_row<S>(g, plane(other, g, i)[g.idx(X, Y)], i, inv, Y);
-    case VIEW_AA_NATURAL:
-        if (g.interior(X, Y) && !g.interior(sx, sy))
-            return dec_row<S>(g, side[(size_t)i * g.nper + g.pidx(X, Y)], i, inv, Y);
-        return dec_row<S>(g, plane(cur, g, i)[g.idx(X, Y)], i, inv, Y);
+    case VIEW_PULL_PENDING: return streamed ? plane(cur, g, i) + g.idx(sx, sy) : (inside ? stale : plane(other, g, i) + g.idx(X, Y));
+    case VIEW_AA_NATURAL: return inside && !streamed ? stale : plane(cur, g, i) + g.idx(X, Y);
     case VIEW_AA_SWAPPED:
-        if (g.interior(sx, sy)) return dec_row<S>(g, plane(cur, g, opp(i))[g.idx(sx, sy)], i, inv, Y);
-        if (g.interior(X, Y)) return dec_row<S>(g, side[(size_t)i * g.nper + g.pidx(X, Y)], i, inv, Y);
-        return dec_row<S>(g, other[(size_t)i * g.nghost() + g.gidx(X, Y)], i, inv, Y);
-    default:
-        return dec_row<S>(g, plane(cur, g, i)[g.idx(X, Y)], i, inv, Y);
+        return streamed ? plane(cur, g, opp(i)) + g.idx(sx, sy) : (inside ? stale : other + ((size_t)i * g.nghost() + g.gidx(X, Y)));
+    default: return plane(cur, g, i) + g.idx(X, Y);
     }
+}
+
+// The nine slots of a node: their addresses first, so that all nine loads are in flight.
+template <class S>
+__device__ __forceinline__ void logical_node(const Geo &g, int view, const S *__restrict__ cur, const S *__restrict__ other,
+                                             const S *__restrict__ side, int X, int Y, float inv, typename Codec<S>::R f[9])
+{
+    const S *at[9];
+    S v[9];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) at[i] = logical_at(g, view, cur, other, side, X, Y, i);
+#pragma unroll
+    for (int i = 0; i < 9; ++i) v[i] = *at[i];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) f[i] = dec_row<S>(g, v[i], i, inv, Y);
 }
 
 // ---- 16-bit storage, four nodes per thread ------------------------------------------------
@@ -237,17 +242,15 @@ __device__ __forceinline__ S enc_row(const Geo &g, typename Codec<S>::R f, int i
     return Codec<S>::enc(f, i, sc);
 }
 
-// The post-stream state of interior node (X, Y) under a view, decoded: logical() for each slot, but off the
-// perimeter, where every slot has an interior source, nine loads without its tests (one after
-// another with their tests they kept one load in flight a node).
+// The post-stream state of interior node (X, Y) under a view, decoded: logical_node(), but off the perimeter, where
+// every slot has an interior source, without its tests.
 template <class S>
 __device__ __forceinline__ void load_state(const Geo &g, int view, const S *__restrict__ cur, const S *__restrict__ other,
                                            const S *__restrict__ side, int X, int Y, float inv,
                                            typename Codec<S>::R f[9])
 {
     if (g.perimeter(X, Y)) {
-#pragma unroll
-        for (int i = 0; i < 9; ++i) f[i] = logical(g, view, cur, other, side, X, Y, i, inv);
+        logical_node(g, view, cur, other, side, X, Y, inv, f);
         return;
     }
     const long long o = g.idx(X, Y);
@@ -365,7 +368,7 @@ __device__ __forceinline__ void collide_given(const Geo &g, int t, typename Work
 inline unsigned cdiv(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
 
 template <class S> S *B(const DevLattice &d, int b) { return static_cast<S *>(d.buf[b]); }
-// The `other` argument of logical(): the pull scheme's second buffer, or the AA ring copy.
+// The `other` argument of logical_at(): the pull scheme's second buffer, or the AA ring copy.
 template <class S> S *OTHER(const DevLattice &d, int cur)
 {
     return d.buf[1] ? static_cast<S *>(d.buf[(1 - cur) ^ d.ghost_flip]) : static_cast<S *>(d.ghost2);
