@@ -279,7 +279,7 @@ int create_device(Simulation *sim, DropIn *c)
     }
     L.ghosts = true;
     c->created = true;
-    if ((size_t)(sim->lx + 2) * (sim->ly + 2) * sizeof(Node) >= kPinBytes) pin_host(sim, c);
+    if (c->sync_mode == LB_SYNC_FULL || (size_t)(sim->lx + 2) * (sim->ly + 2) * sizeof(Node) >= kPinBytes) pin_host(sim, c);
     // (registered: 0.7 ms, where cudaHostAlloc takes 1.7)
     const size_t bytes = (scratch_doubles(sim) * sizeof(double) + 4095) / 4096 * 4096;
     if (pinning_allowed() && !c->scratch_mem) c->scratch_mem = aligned_alloc(4096, bytes);
@@ -735,6 +735,8 @@ void lbSetSyncMode(Simulation *sim, int mode)
     if (!c) { set_error(LB_ERR_STATE, "lbSetSyncMode: simulation not constructed"); return; }
     if (mode < LB_SYNC_NONE || mode > LB_SYNC_FULL) { set_error(LB_ERR_ARG, "lbSetSyncMode: mode %d", mode); return; }
     c->sync_mode = mode;
+    // whole copies after every call: pinned now, before the driver fills the arrays and times its loop
+    if (mode == LB_SYNC_FULL && c->created) pin_host(sim, c);
 }
 
 void saveVel(Simulation *sim, char fName[])
