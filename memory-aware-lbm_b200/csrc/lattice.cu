@@ -95,7 +95,9 @@ cudaError_t device_free(void *p, size_t bytes, int device, cudaStream_t s)
     if (cudaError_t e = pool_of(device, pool)) return e;
     const cudaError_t e = cudaStreamSynchronize(s);
     const cudaError_t f = cudaFreeAsync(p, pool.stream);
-    return e ? e : f;
+    // (the wait is where the pool gives back what it keeps too much of, and where cudaMalloc can have the rest)
+    const cudaError_t g = cudaStreamSynchronize(pool.stream);
+    return e ? e : (f ? f : g);
 }
 
 void memory_hold()
