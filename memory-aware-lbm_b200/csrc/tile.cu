@@ -203,9 +203,12 @@ int tile_steps(const DevLattice &d, long long steps, bool outlet, bool rs)
 {
     if (steps < 2 || (outlet && !d.outlet_tiles) || too_flat(d, outlet, rs)) return 0;
     const int shape = tile_shape(d, rs);
+    const long long nodes = (long long)d.g.lx * d.g.ly;
+    // A rest of two or three steps on a small lattice, whose tiles of two steps are too few and too large for the GPU: a
+    // launch of two and two single steps, FP32 250 x 51 11.4 and 10.3 us, row-shifted 400 x 90 15.8 and 12.4.
+    if (steps < 4 && !outlet && ((d.precision == LBGPU_F32 && nodes < (30ll << 10)) || (d.g.shift_u && nodes < (100ll << 10)))) return 0;
     if (elem16(d)) {
         if (d.g.shift_u && outlet) return 0;
-        const long long nodes = (long long)d.g.lx * d.g.ly;
         if (nodes >= (rs && d.g.shift_u ? 9ll << 19 : 24ll << 20) && (rs || d.g.shift_u)) return 0;
         return shape == TILE_SMALL && steps >= 8 && !d.g.shift_u ? 8 : (steps >= 4 && shape != TILE_LARGE ? 4 : 2);
     }
