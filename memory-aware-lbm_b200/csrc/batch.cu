@@ -168,12 +168,22 @@ int turn_descriptors(lbgpu_batch *b)
 // Pull members can take two steps a launch, but for row-shifted offsets (rebased between rows).
 bool takes_tiles(const Lattice &L) { return L.scheme == LBGPU_PULL && !L.d.g.shift_u; }
 
-// All pull members do, or none: their single-step lists are shared.
+// All pull members do, or none: their single-step lists are shared.  None where most nodes lie in members of so few
+// rows that a tile holds little else than its halo (us a step on one B200, tiles and single steps): FP64 64 of 2048 x
+// 4 24.7 and 22.0, 16 of 60000 x 3 144 and 99, but 24 of 16384 x 6 70 and 79; FP32 16 of 60000 x 3 62 and 54, 64 of
+// 2048 x 4 13.1 and 13.9; 16-bit members gain at any size.
 bool all_tiled(const lbgpu_batch *b)
 {
-    for (const lbgpu_lattice *m : b->members)
-        if (m && m->L.scheme == LBGPU_PULL && !takes_tiles(m->L)) return false;
-    return true;
+    const int few = b->precision == LBGPU_F64 ? 4 : (b->precision == LBGPU_F32 ? 3 : 0);
+    long long flat = 0, nodes = 0;
+    for (const lbgpu_lattice *m : b->members) {
+        if (!m || m->L.scheme != LBGPU_PULL) continue;
+        if (!takes_tiles(m->L)) return false;
+        const long long n = (long long)m->L.lx * m->L.ly;
+        nodes += n;
+        if (m->L.ly <= few) flat += n;
+    }
+    return flat <= nodes / 2;
 }
 
 // A member's host-side state after `m` batch steps (no launches); tiles: pull members took two a launch.

@@ -94,3 +94,26 @@ def test_the_tuner_leaves_alone_what_its_settings_do_not_reach():
         assert lats[0].steps_done >= done + 4 * (6 + 2 * (3 + 4))
     for lat in lats:
         lat.close()
+
+
+@pytest.mark.parametrize("precision,ly,launches", [("f64", 4, 10), ("f64", 5, 5), ("f32", 3, 10), ("f32", 4, 5), ("f16", 3, 5)])
+def test_batches_of_members_of_few_rows(precision, ly, launches):
+    """They step one at a time where tiles hold little but halo, and as alone either way."""
+    def make():
+        lat = lbgpu.Lattice(700, ly, precision, "pull")
+        lat.setup_cylinder(300, 90, 1, 0.03, 0.6, lbgpu.WALL_BOUNCEBACK, lbgpu.OUTLET_CONST)
+        return lat
+
+    lats, ref = [make(), make()], make()
+    with lbgpu.Batch(precision) as b:
+        for lat in lats:
+            b.add(lat)
+        b.step(3)
+        b.step(10)
+        assert b.last_launches == launches
+        b.synchronize()
+        singles(ref, 13)
+        for lat in lats:
+            assert same(lat.populations(), ref.populations())
+    for one in lats + [ref]:
+        one.close()
