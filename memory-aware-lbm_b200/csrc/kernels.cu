@@ -721,7 +721,8 @@ __device__ __forceinline__ void batch_strip(const BatchInst *__restrict__ insts,
     const BatchInst &d = insts[it.inst];
     const Geo g = d.g;
     const int passes = batch_passes(it.sp);
-    S *side = static_cast<S *>(d.side) + (size_t)batch_side_slot(d.side_slot, (d.tau0 + k) & 1) * 9 * (size_t)d.g.nper;
+    // (in 32 bits: at most 3 slots of 9 x 2.3M entries)
+    S *side = static_cast<S *>(d.side) + batch_side_slot(d.side_slot, (d.tau0 + k) & 1) * 9 * d.g.nper;
     const double omega = d.omega;
     const float sc = d.scale, inv = d.inv_scale;
     if constexpr (KIND == BATCH_PULL4) {
