@@ -445,11 +445,20 @@ __device__ __forceinline__ void collide_called(int t, T f[9], T omega, T p0, T p
 // The single-step kernels: FP64 in its general forms too.  Those kernels stream, and the forms with fewer operations
 // cost them resident warps, also in the rules out of line (a kernel has the registers of what it calls):
 // k_pull<double> 56 -> 72 registers, 2047 x 511 28.7 -> 30.1 us a step on one B200, 700 x 200 7.0 -> 8.0.
-template <class T>
+template <class T, bool EXACT = false>
 __device__ __forceinline__ void collide(int t, T f[9], T omega, T p0, T p1)
 {
-    if (t == TAG_BGK) bgk(f, omega);
-    else collide_called<T, false>(t, f, omega, p0, p1);
+    if (t == TAG_BGK) {
+        if constexpr (EXACT) bgk_exact(f, omega);
+        else bgk(f, omega);
+    } else {
+        T g[9];
+#pragma unroll
+        for (int i = 0; i < 9; ++i) g[i] = f[i];
+        collide_boundary<T, EXACT>(t, g, omega, p0, p1);
+#pragma unroll
+        for (int i = 0; i < 9; ++i) f[i] = g[i];
+    }
 }
 
 // equilibrium at (rho, ux, uy) for initialisation (lb.c:71-78)

@@ -41,14 +41,14 @@ __device__ __forceinline__ void node_params(const double *__restrict__ bc, const
     node_params(bc, g.nb, t, X, Y, p0, p1);
 }
 
-template <class S>
+template <class S, bool EXACT = false>
 __device__ __forceinline__ void collide_node(const double *__restrict__ bc, const Geo &g, int t,
                                              int X, int Y, typename Codec<S>::R f[9], double omega)
 {
     using R = typename Codec<S>::R;
     double p0, p1;
     node_params(bc, g, t, X, Y, p0, p1);
-    rules::collide<R>(t, f, (R)omega, (R)p0, (R)p1);
+    rules::collide<R, EXACT>(t, f, (R)omega, (R)p0, (R)p1);
 }
 
 template <class S>

@@ -160,6 +160,16 @@ __device__ __forceinline__ double tile_density(const TileArgs<S> &a, const S *__
     return (double)rules::density(h);
 }
 
+// A boundary rule in exact FP64, out of line.  Tiles of 64 columns go through the general dispatch, whose BGK no rule takes:
+// with it the compiler spills less around the call (64 x 16, 8192 x 2048 with the extrapolated outlet 254 us a step on
+// one B200 and 276 without it, 16384 x 4096 982 and 1004); smaller ones are faster without (250 x 51 2.65 and 2.78).
+template <class SH>
+__device__ __forceinline__ void tile_rule(int t, double f[9], double omega, double p0, double p1)
+{
+    if constexpr (SH::W >= 64) rules::collide<double, true>(t, f, omega, p0, p1);
+    else rules::collide_called<double, true>(t, f, omega, p0, p1);
+}
+
 // The boundary rules (tags of 3 and more) at one node.
 template <class S, class SH, int s, int M, bool EXTRAP>
 __device__ __forceinline__ void tile_boundary(const TileArgs<S> &a, const S *__restrict__ rd, int t, int X, int Y, int q,
@@ -170,16 +180,21 @@ __device__ __forceinline__ void tile_boundary(const TileArgs<S> &a, const S *__r
         using D = Ar<double>;
         const double r1 = tile_density<S, SH, s>(a, rd, X, Y, q, 0), r2 = tile_density<S, SH, s>(a, rd, X, Y, q, 1);
         const double rho = D::S(D::M(4. / 3., r1), D::M(1. / 3., r2));
-        if constexpr (sizeof(S) == 8) rules::collide_called<double, true>(t, f, a.omega, rho, 0.0);
+        if constexpr (sizeof(S) == 8) tile_rule<SH>(t, f, a.omega, rho, 0.0);
         else collide_given<S>(g, t, f, a.omega, a.sc, a.inv, rho, 0.0);
-    } else if constexpr (sizeof(S) == 8) {
-        // in line where a launch takes four steps: the call's way through local memory is part of a step's longest chain.
-        // 511 x 127 3.8 -> 3.4 us a step; eight steps' copies of it leave the instruction cache (250 x 51 2.4 -> 2.9),
-        // and FP32 gains nothing.
+    } else if constexpr (sizeof(S) == 8 && SH::T == 4) {
+        // in line: the call's way through local memory is part of a step's longest chain.  FP64 511 x 127 3.8 -> 3.4
+        // us a step; eight steps' copies of it leave the instruction cache (250 x 51 2.4 -> 2.9), and FP32 gains
+        // nothing.
         double p0, p1;
         node_params(a.bc, g, t, X, Y, p0, p1);
-        if constexpr (SH::T == 4) rules::boundary_rule<double, true>(t, f, a.omega, p0, p1);
-        else rules::collide_called<double, true>(t, f, a.omega, p0, p1);
+        rules::boundary_rule<double, true>(t, f, a.omega, p0, p1);
+    } else if constexpr (sizeof(S) == 8 && SH::W >= 64) {
+        collide_node<S, true>(a.bc, g, t, X, Y, f, a.omega);
+    } else if constexpr (sizeof(S) == 8) {
+        double p0, p1;
+        node_params(a.bc, g, t, X, Y, p0, p1);
+        rules::collide_called<double, true>(t, f, a.omega, p0, p1);
     } else {
         collide_w<S, (M & TILE_SHIFT) ? 1 : 0>(a.bc, g, t, X, Y, f, a.omega, a.sc, a.inv);
     }
