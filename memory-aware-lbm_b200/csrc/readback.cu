@@ -8,8 +8,9 @@
 #include <algorithm>
 #include <atomic>
 #include <mutex>
-#include <exception>
+#include <system_error>
 #include <thread>
+#include <vector>
 #include "readback.h"
 
 namespace lbgpu {
@@ -70,8 +71,9 @@ void read_back_release()
     if (p) cudaFreeHost(p);
 }
 
-cudaError_t read_back(int device, cudaStream_t stream, long long items, size_t item_bytes, RangeFn<double> fill,
-                      RangeFn<const double> take)
+cudaError_t read_back(int device, cudaStream_t stream, long long items, size_t item_bytes,
+                      const std::function<void(long long, long long, double *)> &fill,
+                      const std::function<void(long long, long long, const double *)> &take)
 {
     if (items <= 0 || item_bytes == 0) return cudaStreamSynchronize(stream);
     int before = device;
@@ -88,7 +90,7 @@ cudaError_t read_back(int device, cudaStream_t stream, long long items, size_t i
     if (cudaError_t e = take_pinned(2 * slot * (size_t)want, &mem, &bytes)) return e;
     std::atomic<long long> next(0);
     std::atomic<int> failed(0);
-    cudaError_t errors[kThreads] = {};
+    std::vector<cudaError_t> errors((size_t)want, cudaSuccess);
     auto work = [&](int t) {
         double *buf[2];
         cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -121,19 +123,18 @@ cudaError_t read_back(int device, cudaStream_t stream, long long items, size_t i
         for (int b = 0; b < 2; ++b)
             if (ev[b]) cudaEventDestroy(ev[b]);
         if (e != cudaSuccess) failed.store(1);
-        errors[t] = e;
+        errors[(size_t)t] = e;
     };
-    std::thread team[kThreads];
+    std::vector<std::thread> team;
     for (int t = 1; t < want; ++t) {
         try {
-            team[t] = std::thread(work, t);
-        } catch (const std::exception &) {
+            team.emplace_back(work, t);
+        } catch (const std::system_error &) {
             break;                       // fewer threads: the others take their chunks
         }
     }
     work(0);
-    for (std::thread &t : team)
-        if (t.joinable()) t.join();
+    for (std::thread &t : team) t.join();
     cudaError_t first = cudaSuccess;
     for (cudaError_t e : errors)
         if (first == cudaSuccess) first = e;
