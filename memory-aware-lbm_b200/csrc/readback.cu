@@ -8,9 +8,8 @@
 #include <algorithm>
 #include <atomic>
 #include <mutex>
-#include <system_error>
+#include <exception>
 #include <thread>
-#include <vector>
 #include "readback.h"
 
 namespace lbgpu {
@@ -71,9 +70,8 @@ void read_back_release()
     if (p) cudaFreeHost(p);
 }
 
-cudaError_t read_back(int device, cudaStream_t stream, long long items, size_t item_bytes,
-                      const std::function<void(long long, long long, double *)> &fill,
-                      const std::function<void(long long, long long, const double *)> &take)
+cudaError_t read_back(int device, cudaStream_t stream, long long items, size_t item_bytes, RangeFn<double> fill,
+                      RangeFn<const double> take)
 {
     if (items <= 0 || item_bytes == 0) return cudaStreamSynchronize(stream);
     int before = device;
@@ -90,7 +88,7 @@ cudaError_t read_back(int device, cudaStream_t stream, long long items, size_t i
     if (cudaError_t e = take_pinned(2 * slot * (size_t)want, &mem, &bytes)) return e;
     std::atomic<long long> next(0);
     std::atomic<int> failed(0);
-    std::vector<cudaError_t> errors((size_t)want, cudaSuccess);
+    cudaError_t errors[kThreads] = {};
     auto work = [&](int t) {
         double *buf[2];
         cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -123,18 +121,19 @@ cudaError_t read_back(int device, cudaStream_t stream, long long items, size_t i
         for (int b = 0; b < 2; ++b)
             if (ev[b]) cudaEventDestroy(ev[b]);
         if (e != cudaSuccess) failed.store(1);
-        errors[(size_t)t] = e;
+        errors[t] = e;
     };
-    std::vector<std::thread> team;
+    std::thread team[kThreads];
     for (int t = 1; t < want; ++t) {
         try {
-            team.emplace_back(work, t);
-        } catch (const std::system_error &) {
+            team[t] = std::thread(work, t);
+        } catch (const std::exception &) {
             break;                       // fewer threads: the others take their chunks
         }
     }
     work(0);
-    for (std::thread &t : team) t.join();
+    for (std::thread &t : team)
+        if (t.joinable()) t.join();
     cudaError_t first = cudaSuccess;
     for (cudaError_t e : errors)
         if (first == cudaSuccess) first = e;

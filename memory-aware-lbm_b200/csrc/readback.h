@@ -2,7 +2,6 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stddef.h>
-#include <functional>
 
 namespace lbgpu {
 
@@ -11,9 +10,21 @@ namespace lbgpu {
 // them from there into the caller's arrays.  Both are called from several threads at once for large
 // results, for ranges that do not overlap.  Returns when everything has arrived, or the first CUDA
 // error (nothing is in flight then either).
-cudaError_t read_back(int device, cudaStream_t stream, long long items, size_t item_bytes,
-                      const std::function<void(long long, long long, double *)> &fill,
-                      const std::function<void(long long, long long, const double *)> &take);
+// fill and take are functions or lambdas that outlive the call; nothing here allocates memory of the host's heap but
+// for threads, without which it goes on.
+template <class P>
+struct RangeFn {
+    const void *object;
+    void (*call)(const void *, long long, long long, P *);
+    template <class F>
+    RangeFn(const F &f)
+        : object(&f), call([](const void *o, long long a, long long b, P *p) { (*static_cast<const F *>(o))(a, b, p); })
+    {
+    }
+    void operator()(long long a, long long b, P *p) const { call(object, a, b, p); }
+};
+cudaError_t read_back(int device, cudaStream_t stream, long long items, size_t item_bytes, RangeFn<double> fill,
+                      RangeFn<const double> take);
 
 // Gives back the pinned memory that is kept between calls (the last lattice went).
 void read_back_release();
