@@ -214,10 +214,12 @@ int lbgpu_synchronize(lbgpu_lattice *lat);
  * No counterpart in the reference (one lattice per process).  Members are lattices of the
  * batch's precision, pull or AA, with constant-density outlets (an extrapolated outlet is
  * stepped on its own).  lbgpu_batch_step advances every member by nsteps: one launch per two steps
- * for the pull members (per step where one stores row-shifted offsets, and for the odd step of a
- * call) and one per step for each phase of the AA members walks a work list of tiles; chunks of 20 steps are replayed as a CUDA graph.  Each member's result is bit-identical to stepping it alone.  The batch does not
- * own its members; remove a member before destroying it.  Steps are asynchronous on the batch's
- * stream and ordered with the members' own streams. */
+ * for the pull members (per step where one stores row-shifted offsets or most have three or four rows, and
+ * for the odd step of a call) and one per step for each phase of the AA members walks a work list
+ * of tiles; chunks of 20 steps are replayed as a CUDA graph.  Each member's result is bit-identical
+ * to stepping it alone.  The batch does not own its members; remove a member before destroying it.
+ * Steps are asynchronous on the batch's stream and ordered with the members' own streams; an even
+ * number of them can be captured through a member's stream once the batch has stepped. */
 typedef struct lbgpu_batch lbgpu_batch;
 int lbgpu_batch_create(int precision, lbgpu_batch **out);
 int lbgpu_batch_destroy(lbgpu_batch *b);

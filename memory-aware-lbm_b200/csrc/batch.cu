@@ -1,23 +1,22 @@
 // batch.cu -- many independent lattices advanced together (lbgpu_batch_* of include/lbgpu.h).
 //
-// Every step of every member runs in at most four launches, one per kind of step: the pull step
-// of the two-buffer members (one node per thread, or for 16-bit storage optionally four nodes
-// per thread), and the even and the odd AA step of the in-place members (AA members are kept in
-// two lists by the parity of their phase, so each list runs one kind at a time).  A launch
+// Pull members take two steps a launch on tiles in shared memory (tile.cuh), one work list of tiles for
+// all of them: 24 uneven channels of 8.6M nodes in FP32 119 -> 75 us a step, 24 of 5.7M nodes in FP64 162 -> 108,
+// 24 small ones (0.7M nodes) in FP32 20.7 -> 8.3, 48 of 13.4M nodes in FP16 153 -> 101 (packed pairs of nodes).
+// Single steps (the odd one of a call, and all of a batch with row-shifted offsets or of members of a few rows) and AA
+// members run from lists of their own, one launch a list: the pull step one node per thread, or for
+// 16-bit storage optionally four with the members' perimeters apart, and the even and the odd AA step (AA
+// members are kept in two lists by the parity of their phase, so each list runs one kind at a time).  Such a launch
 // walks a work list of tiles (member, x0, y0, shape) of 128, 256 or 512 nodes, one per thread
 // (or four per thread): either one block per tile, or a persistent grid of (blocks per SM x
 // SMs) blocks strides through it.  Steps are grouped in chunks of 20 captured
 // once as a CUDA graph: the kernels read each member's buffers and parities from a device
 // descriptor array, so the same graph replays chunk after chunk; it is re-captured when the
-// membership or the launch form changes.
-// Pull members take two steps a launch on tiles in shared memory (tile.cuh), one work list of tiles for
-// all of them: 24 uneven channels of 8.6M nodes in FP32 119 -> 75 us a step, 24 of 5.7M nodes in FP64 162 -> 108,
-// 24 small ones (0.7M nodes) in FP32 20.7 -> 8.3, 48 of 13.4M nodes in FP16 153 -> 101 (packed pairs of nodes).
-// A work item is a strip of tiles of one member stacked in y: its block reads the member's
+// membership or the launch form changes.  Of the single-step lists a work item is a strip of tiles of one member stacked in y: its block reads the member's
 // descriptor once and steps the tiles one after another down the lattice, so the descriptor's
 // dependent loads are spread over the strip.  Tile widths and strip lengths are chosen per size
 // class of member (node count), the threads per tile and the launch form per batch, by hand or by
-// lbgpu_batch_autotune.
+// lbgpu_batch_autotune; none of it shapes the tiles of two steps.
 #include <algorithm>
 #include <cstring>
 #include <vector>

@@ -681,15 +681,6 @@ int Lattice::upload_zgb_src(const int *src)
     return LB_OK;
 }
 
-int Lattice::upload_tag_plane(const uint8_t *plane)
-{
-    LB_CUDA(cudaMemcpyAsync(const_cast<uint8_t *>(d.tag), plane, (size_t)d.g.plane,
-                            cudaMemcpyHostToDevice, stream), "upload tags");
-    h2d_bytes += (size_t)d.g.plane;
-    LB_CUDA(cudaStreamSynchronize(stream), "upload tags");
-    return LB_OK;
-}
-
 int Lattice::upload_tags(const uint8_t *tag_xy, const uint8_t *zgb_row)
 {
     int inside = 0, outlet = lx >= 4;

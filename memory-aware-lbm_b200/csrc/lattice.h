@@ -17,9 +17,10 @@ void clear_error();
 
 // Device memory of lattices and requests.  Up to kPoolBytes it comes from a pool per device that keeps up to
 // 256 MiB of what was given back (a cudaMalloc takes 0.1 ms and more, a cudaFree waits for the whole
-// device: a 1024 x 256 FP32 lattice is made in 0.07 ms instead of 0.74 and closed in 0.07 instead of 0.6, a
-// served stream of 24 requests takes 52 ms instead of 65); what it keeps goes back with the last lattice.  Larger
-// parts are cudaMalloc's (150 MB 0.4 ms, 2.4 GB 0.9, against 13.5 from a pool that has to grow).  Usable on
+// device: beside others a 1024 x 256 FP32 lattice is made and set up in 0.15 ms instead of 0.87 and closed in 0.06
+// instead of 0.6; alone 0.5 and 1.2); what it keeps goes back with the last lattice.  Larger
+// parts are cudaMalloc's, one a lattice (made and set up in ms, parts apart before: FP32 8192 x 2048 1.15 and 2.3, FP64
+// 16384 x 4096 5.7 and 6.3; a pool that has to grow by 2.4 GB takes 13.5).  Usable on
 // any stream at once; given back, with its size, after what `s` still does with it.
 constexpr size_t kPoolBytes = (size_t)64 << 20;
 cudaError_t device_alloc(void **p, size_t bytes, int device);
@@ -83,7 +84,6 @@ struct Lattice {
     int upload_zgb_src(const int *src);   // host [4*nb]
     // host tag[X*(ly+2)+Y], validated here; zgb_row: rows of the extrapolated outlet, or null
     int upload_tags(const uint8_t *tag_xy, const uint8_t *zgb_row);
-    int upload_tag_plane(const uint8_t *plane);  // host plane in device layout
     int upload_records(int b, const double *host, int rs, int X0, int X1);
     // rows Y0..Y0+H-1 of columns X0..X1-1 from host records laid out like upload_records' (host
     // points at column X0, row 0)

@@ -9,8 +9,8 @@
 //
 // Slots of boundary nodes whose source lies outside the lattice ("stale" slots: the
 // reference never streams into them, lb.c:258-267, so they keep the second buffer's old
-// content) are kept in a side store: two parities x nine directions x `nper` perimeter
-// nodes.  pidx() numbers the perimeter: row Y=1, row Y=ly, then column X=1 and column X=lx
+// content) are kept in a side store: slots of nine directions x `nper` perimeter nodes, one for each
+// parity of the collisions, and for the pull scheme spare ones (side_slots).  pidx() numbers the perimeter: row Y=1, row Y=ly, then column X=1 and column X=lx
 // without their corners.
 #pragma once
 #include <cuda_runtime.h>

@@ -6,8 +6,8 @@
 // streams cannot afford them (cudaMalloc and cudaFree synchronize with the device and stall
 // every stream), and a host application whose device memory is reserved up front by another
 // allocator (a framework's caching allocator, a fixed per-process budget) may have none left
-// to hand out.  lbgpu_get_macros allocates a lattice-sized device buffer on every call; this
-// variant uses a fixed device array instead.
+// to hand out.  lbgpu_get_macros takes device memory for results up to 1 MiB when a lattice is
+// first read, and pinned host memory for larger ones; this variant uses a fixed device array instead.
 //
 // The scratch: a file-scope __device__ array of 3 x 262,144 doubles (6 MiB).  Every GPU that
 // loads the library holds it until the process exits.  Lattices with more than 262,144

@@ -445,7 +445,7 @@ def declared_functions():
 
 
 class Batch:
-    """lbgpu_batch: many lattices of one precision stepped together (one launch per step)."""
+    """lbgpu_batch: many lattices of one precision stepped together (pull members two steps a launch)."""
 
     def __init__(self, precision="f32"):
         self.precision = precision

@@ -4,9 +4,9 @@ Every number comes from the library's kernels through lbgpu.py; the inputs are s
 cylinder channels (bounce-back walls, Poiseuille inlet, constant-density outlet).
 
 batching   independent channels of uneven size, Reynolds number and obstacle placement stepped
-           together (one launch per work list and step, persistent or one block per strip as
-           the autotuner picks, CUDA-graph chunks of 50 steps, tile shapes and pull/AA chosen per
-           size class by the autotuners) against a sequential loop that steps each channel
+           together (pull members two steps a launch on tiles, AA members one launch a step, in
+           strips whose shape the autotuner picks; CUDA-graph chunks of 20 steps; pull or AA per
+           size class) against a sequential loop that steps each channel
            alone with its own launches.
 shapes     the batch's speed against its members' size and shape at a constant node count:
            one large channel stepped alone, then batches of equal members, from one member of
@@ -86,7 +86,7 @@ def batching_study(precisions=("f32", "f16"), n=512, steps=2000, seed=20260101, 
     """tune=0 keeps the defaults (pull members, default tile shapes and launch form)."""
     insts = batching_instances(n, seed)
     nodes = sum(q["lx"] * q["ly"] for q in insts)
-    res = {"instances": n, "seed": seed, "nodes": nodes, "steps": steps, "chunk": 50,
+    res = {"instances": n, "seed": seed, "nodes": nodes, "steps": steps, "chunk": 20,
            "precisions": {}}
     for prec in precisions:
         if tune:
